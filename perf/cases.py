@@ -115,10 +115,10 @@ def _randn(gen, shape, std, dtype):
     return t.mul_(std).to(dtype)
 
 
-def prepare(case, seed):
-    tmb.register_mojo_devices()
+def _inputs(case, seed):
+    """q, k, v as (B, H, S, D) views, and the upstream gradient of a training case."""
     B, Hq, Hkv, Sq, Sk, D = (case[n] for n in ("B", "Hq", "Hkv", "Sq", "Sk", "D"))
-    dtype, std, kind = _DTYPES[case["dtype"]], case["std"], case["kind"]
+    dtype, std = _DTYPES[case["dtype"]], case["std"]
     gen = torch.Generator(device="cuda").manual_seed(seed)
     if case["fused"]:
         proj = _randn(gen, (B, Sq, (Hq + 2 * Hkv) * D), std, dtype)
@@ -126,16 +126,25 @@ def prepare(case, seed):
     else:
         q = _randn(gen, (B, Hq, Sq, D), std, dtype)
         k, v = (_randn(gen, (B, Hkv, Sk, D), std, dtype) for _ in range(2))
-    state = {"kind": kind, "q": q, "k": k, "v": v, "causal": case["mask"] == "causal", "scale": D ** -0.5,
-             "dropout": case["dropout"], "gqa": Hq != Hkv}
+    grad = None
+    if case["kind"] == "train":
+        # the gradient arrives in the layout the output is handed on in: (B, S, H, D) behind a fused projection
+        grad = (_randn(gen, (B, Sq, Hq, D), 1.0, dtype).transpose(1, 2) if case["fused"]
+                else _randn(gen, (B, Hq, Sq, D), 1.0, dtype))
+    return q, k, v, grad
+
+
+def prepare(case, seed):
+    tmb.register_mojo_devices()
+    q, k, v, grad = _inputs(case, seed)
+    kind = case["kind"]
+    state = {"kind": kind, "q": q, "k": k, "v": v, "causal": case["mask"] == "causal", "scale": case["D"] ** -0.5,
+             "dropout": case["dropout"], "gqa": case["Hq"] != case["Hkv"]}
     if kind in ("chunk", "verify"):
         return state
     q, k, v = (tmb.from_cuda(t) for t in (q, k, v))
     if kind == "train":
         torch.mojo.manual_seed(seed)   # where the dropout masks of this state's passes start
-        # the gradient arrives in the layout the output is handed on in: (B, S, H, D) behind a fused projection
-        grad = (_randn(gen, (B, Sq, Hq, D), 1.0, dtype).transpose(1, 2) if case["fused"]
-                else _randn(gen, (B, Hq, Sq, D), 1.0, dtype))
         state["grad"] = tmb.from_cuda(grad)
         q, k, v = (t.requires_grad_() for t in (q, k, v))
     state.update(q=q, k=k, v=v)
@@ -160,6 +169,53 @@ def run(state):
     forward = raw.flash_fwd if kind == "chunk" else raw.flash_fwd_splitkv
     out, lse = forward(q, k, v, causal=_lib.CAUSAL_BOTTOM_RIGHT)
     return {"out": out, "lse": lse}
+
+
+_EXACT_SCORES = 1 << 28   # 64-bit scores held at a time
+
+
+def exact(case, seed):
+    """The same outputs in 64 bits, one key/value head at a time and as many query rows as fit."""
+    if case["dropout"]:
+        return None   # the mask is this package's own random stream
+    B, Hq, Hkv, Sq, Sk, D = (case[n] for n in ("B", "Hq", "Hkv", "Sq", "Sk", "D"))
+    if 8 * B * Hq * Sq * Sk * D > 1e14:
+        return None   # too long in 64 bits
+    q, k, v, grad = _inputs(case, seed)
+    group, scale, kind = Hq // Hkv, D ** -0.5, case["kind"]
+    f64 = {"dtype": torch.float64, "device": "cuda"}
+    res = {"out": torch.empty((B, Hq, Sq, D), **f64)}
+    if kind == "train":
+        res.update(dq=torch.empty((B, Hq, Sq, D), **f64), dk=torch.zeros((B, Hkv, Sk, D), **f64),
+                   dv=torch.zeros((B, Hkv, Sk, D), **f64))
+    elif kind != "forward":
+        res["lse"] = torch.empty((B, Hq, Sq), **f64)
+    rows = max(1, _EXACT_SCORES // (group * Sk))
+    col = torch.arange(Sk, device="cuda")
+    for b in range(B):
+        for h in range(Hkv):
+            heads = slice(h * group, (h + 1) * group)
+            k64, v64 = k[b, h].double(), v[b, h].double()
+            for r0 in range(0, Sq, rows):
+                r = slice(r0, min(Sq, r0 + rows))
+                q64 = q[b, heads, r].double() * scale
+                s = q64 @ k64.T
+                if case["mask"] != "none":
+                    last = torch.arange(r.start, r.stop, device="cuda") + (Sk - Sq if case["mask"] == "suffix" else 0)
+                    s.masked_fill_(col > last[:, None], -torch.inf)
+                lse = torch.logsumexp(s, dim=-1)
+                p = s.sub_(lse[..., None]).exp_()
+                o = p @ v64
+                res["out"][b, heads, r] = o
+                if kind == "train":
+                    g = grad[b, heads, r].double()
+                    res["dv"][b, h] += torch.einsum("gqk,gqd->kd", p, g)
+                    ds = p.mul_((g @ v64.T).sub_((g * o).sum(-1, keepdim=True)))
+                    res["dq"][b, heads, r] = ds @ k64 * scale
+                    res["dk"][b, h] += torch.einsum("gqk,gqd->kd", ds, q64)
+                elif kind != "forward":
+                    res["lse"][b, heads, r] = lse
+    return res
 
 
 def _visible(case):
