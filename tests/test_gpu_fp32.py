@@ -1,0 +1,77 @@
+"""The exact-fp32 kernels at the edges of their tiles, on the GPU: rows and columns around 32, 64 and
+128, both block shapes (few blocks take the short one, many the tall one), grouped heads, both causal
+alignments, dropout, and views of a fused projection, against the same attention in float64."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle.philox import keep_mask
+from torch_mojo_backend_b200 import raw
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # B, Hq, Hkv, Sq, Sk, D, causal mode, dropout
+    (1, 2, 2, 1, 2, 64, 0, 0.0),           # (over a single key dQ and dK are exactly zero: no relative error)
+    (1, 2, 1, 31, 33, 128, 2, 0.0),
+    (1, 2, 2, 65, 64, 64, 1, 0.0),
+    (1, 3, 1, 129, 63, 128, 2, 0.0),       # the first query rows see no key
+    (2, 4, 2, 96, 200, 64, 1, 0.25),
+    (1, 2, 2, 130, 70, 128, 0, 0.5),
+    (19, 8, 8, 130, 129, 64, 1, 0.0),      # 456 tall blocks each way
+    (19, 8, 4, 193, 321, 64, 2, 0.2),
+    (25, 6, 6, 65, 66, 128, 1, 0.0),       # 300 tall blocks
+    (13, 12, 6, 60, 130, 128, 0, 0.3),
+]
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,mode,p", CASES)
+def test_fp32_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p):
+    g = torch.Generator().manual_seed(Sq * 1000 + Sk)
+    scale = D ** -0.5
+    # q is a view into a wider row, as a fused projection gives it
+    q = torch.randn(B, Sq, Hq, 2 * D, generator=g)[..., :D].transpose(1, 2)
+    k, v = (torch.randn(B, Hkv, Sk, D, generator=g) for _ in range(2))
+    dout = torch.randn(B, Hq, Sq, D, generator=g)
+    dropout = (p, 11, 5) if p else None
+    qc = torch.empty(B, Sq, Hq, 2 * D, device="cuda")[..., :D].transpose(1, 2).copy_(q)
+    kc, vc = k.cuda(), v.cuda()
+    out, lse = raw.flash_fwd(qc, kc, vc, causal=mode, scale=scale, dropout=dropout)
+    dq, dk, dv = raw.flash_bwd(dout.cuda(), qc, kc, vc, out, lse, causal=mode, scale=scale, dropout=dropout)
+    torch.cuda.synchronize()
+    keep, inv = keep_mask(B, Hq, Sq, Sk, p, 11, 5)
+    ref = reference(q.numpy(), k.numpy(), v.numpy(), dout.numpy(), mode, scale, keep, inv)
+    for name, got in (("out", out), ("lse", lse), ("dq", dq), ("dk", dk), ("dv", dv)):
+        want = ref[name]
+        got = got.double().cpu().numpy()
+        seen = np.isfinite(want)
+        assert np.array_equal(seen, np.isfinite(got)), name
+        # sums of up to n = max(Sq * Hq / Hkv, Sk) + D fp32 terms: error at most about n * 2^-24 of the
+        # sum of magnitudes; the observed one grows like sqrt(n).  2^-24 * 350 = 2.1e-5.
+        err = np.linalg.norm(got[seen] - want[seen]) / max(np.linalg.norm(want[seen]), 1e-30)
+        assert err < 2e-5, f"{name}: relative error {err:.2e}"
+
+
+def reference(q, k, v, do, mode, scale, keep, inv):
+    q, k, v, do = (x.astype(np.float64) for x in (q, k, v, do))
+    B, Hq, Sq, D = q.shape
+    Hkv, Sk = k.shape[1], k.shape[2]
+    kk, vv = (np.repeat(x, Hq // Hkv, axis=1) for x in (k, v))
+    s = np.einsum("bhqd,bhkd->bhqk", q, kk) * scale
+    if mode:
+        off = Sk - Sq if mode == 2 else 0
+        s[:, :, np.arange(Sk)[None, :] > np.arange(Sq)[:, None] + off] = -np.inf
+    m = s.max(-1, keepdims=True)
+    e = np.exp(s - np.where(np.isfinite(m), m, 0.0))
+    l = e.sum(-1, keepdims=True)
+    with np.errstate(divide="ignore", invalid="ignore"):
+        pr = np.where(l > 0, e / l, 0.0)
+        lse = np.where(l > 0, m + np.log(l), -np.inf)[..., 0]
+    pd = pr * keep * inv
+    out = pd @ vv
+    dp = (do @ np.swapaxes(vv, -1, -2)) * keep * inv
+    ds = pr * (dp - (do * out).sum(-1, keepdims=True))
+    fold = lambda x: x.reshape(B, Hkv, Hq // Hkv, Sk, D).sum(2)
+    return {"out": out, "lse": lse, "dq": ds @ kk * scale, "dk": fold(np.swapaxes(ds, -1, -2) @ q * scale),
+            "dv": fold(np.swapaxes(pd, -1, -2) @ do)}
