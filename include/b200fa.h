@@ -202,6 +202,16 @@ int b200fa_bwd_no_alloc(const b200fa_tensor4* q, const b200fa_tensor4* k, const 
 size_t b200fa_no_alloc_scratch_bytes(void);
 
 /*
+ * b200fa_fwd for a piece - some batch entries or whole groups of heads - of a problem with
+ * `whole_heads` = batch * query heads in all (at least the piece's own).  How a small forward is dealt
+ * to the SMs depends on that number, and with it the order of some sums; a piece computed through this
+ * call has the bits that one call over the whole problem would give it.
+ */
+int b200fa_fwd_piece(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,
+                     const b200fa_tensor4* out, float* lse, int dtype, int causal, float scale,
+                     int64_t whole_heads, void* stream, int device, uint32_t* status_word);
+
+/*
  * Same contracts as b200fa_fwd / b200fa_bwd, but always run the exact-fp32 SIMT kernels
  * whatever the storage type (16-bit inputs are widened to fp32 on load).  They exist so the
  * tensor-core kernels can be cross-checked on the device at sizes where a CPU comparison

@@ -46,6 +46,38 @@ def t64(x):
     return x.float().numpy().astype(np.float64)
 
 
+# Forward calls with few (batch, head, query tile) units, whose K/V blocks are dealt to the CTAs of a
+# cluster: unequal shares, shares without a block, rows without a key, one key, ragged edges.
+SPLIT = [
+    # dtype, B, Hq, Hkv, Sq, Sk, D, mode
+    (torch.bfloat16, 1, 2, 1, 256, 4224, 128, 2),
+    (torch.float16, 1, 3, 3, 300, 2000, 128, 2),
+    (torch.bfloat16, 1, 8, 8, 1024, 1024, 128, 1),
+    (torch.float16, 1, 2, 1, 600, 300, 128, 2),
+    (torch.bfloat16, 1, 4, 4, 129, 1153, 64, 2),
+    (torch.float16, 2, 2, 2, 1000, 1000, 64, 1),
+    (torch.bfloat16, 1, 2, 2, 33, 700, 64, 0),
+    (torch.bfloat16, 1, 2, 2, 20, 1025, 128, 1),
+    (torch.float16, 1, 4, 2, 257, 1, 128, 0),
+]
+
+
+@pytest.mark.parametrize("dtype,B,Hq,Hkv,Sq,Sk,D,mode", SPLIT)
+def test_forward_split_over_clusters(dtype, B, Hq, Hkv, Sq, Sk, D, mode):
+    q, k, v, _ = draw(dtype, B, Hq, Hkv, Sq, Sk, D, Sq + Sk)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full((B, Sq, Hq, D), float("nan"), dtype=dtype, device="cuda").transpose(1, 2)
+    _, lse = raw.flash_fwd(q.cuda(), k.cuda(), v.cuda(), causal=mode, scale=D ** -0.5, out=out, status=status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    ref_out, ref_lse = O.sdpa_forward(q, k, v, mode, D ** -0.5)
+    assert_within("out", out, ref_out, TOL_16BIT, dtype)
+    sees = torch.arange(Sq) + (Sk - Sq if mode == 2 else 0) >= 0    # a row without a key has lse -inf
+    seen = sees.expand(B, Hq, Sq)
+    assert torch.equal(seen, torch.isfinite(lse.cpu()))
+    assert (lse.cpu() - ref_lse)[seen].abs().max().item() < TOL_LSE
+
+
 ALIGNED = [
     # dtype, B, Hq, Hkv, Sq, Sk, D, mode (1 top-left = torch's is_causal, 2 bottom-right = the reference kernels' rule)
     (torch.bfloat16, 2, 4, 2, 128, 320, 128, 1),

@@ -34,6 +34,7 @@ ERR_TIMEOUT = -9
 #: every symbol include/b200fa.h declares; the CPU test-suite checks the library exports them
 EXPORTED_SYMBOLS = (
     "b200fa_fwd",
+    "b200fa_fwd_piece",
     "b200fa_bwd_workspace_bytes",
     "b200fa_bwd",
     "b200fa_fwd_simt",
@@ -106,6 +107,8 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.argtypes = fwd_args
         fn.restype = ctypes.c_int
+    lib.b200fa_fwd_piece.argtypes = fwd_args[:8] + [ctypes.c_int64] + fwd_args[8:]
+    lib.b200fa_fwd_piece.restype = ctypes.c_int
     for name in ("b200fa_bwd", "b200fa_bwd_simt"):
         fn = getattr(lib, name)
         fn.argtypes = bwd_args
@@ -182,9 +185,10 @@ def causal_code(causal) -> int:
 
 def fwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, dtype: int, causal,
         scale: float, stream: int, device: int, status_ptr: int = 0, *, simt: bool = False,
-        dropout=None) -> int:
+        dropout=None, whole_heads: int = 0) -> int:
     """Raw forward call; returns the library's status code.  `causal` is a bool or one of
-    CAUSAL_*; `dropout` is None or ``(p, seed, offset)``."""
+    CAUSAL_*; `dropout` is None or ``(p, seed, offset)``; `whole_heads`, if not 0, is batch * query
+    heads of the problem this call computes a piece of (see b200fa_fwd_piece)."""
     head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), ctypes.c_void_p(lse_ptr),
             dtype, causal_code(causal), ctypes.c_float(scale))
     tail = (ctypes.c_void_p(stream), device, ctypes.c_void_p(status_ptr))
@@ -192,6 +196,8 @@ def fwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, dtype: i
         p, seed, offset = dropout
         return load().b200fa_fwd_dropout(*head, ctypes.c_float(p), ctypes.c_uint64(seed), ctypes.c_uint64(offset),
                                          1 if simt else 0, *tail)
+    if whole_heads and not simt:
+        return load().b200fa_fwd_piece(*head, whole_heads, *tail)
     fn = load().b200fa_fwd_simt if simt else load().b200fa_fwd
     return fn(*head, *tail)
 

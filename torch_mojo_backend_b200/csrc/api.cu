@@ -203,6 +203,7 @@ struct Options {
   int parts = 7;
   float dropout_p = 0.f;
   uint64_t seed = 0, offset = 0;
+  int64_t whole_heads = 0;   // 0: the call is a whole problem
 };
 
 // causal argument -> (flag, diagonal offset); false if it is not one of the three modes
@@ -253,6 +254,7 @@ int fwd_impl(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tens
   p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status_word;
+  p.whole_heads = opt.whole_heads > 0 ? opt.whole_heads : B * Hq;
   p.tiles_per_cta = fwd_tiles();
   p.wait_budget = wait_budget();
 
@@ -406,6 +408,15 @@ int b200fa_fwd(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_te
                const b200fa_tensor4* out, float* lse, int dtype, int causal, float scale, void* stream,
                int device, uint32_t* status_word) {
   return fwd_impl(q, k, v, out, lse, dtype, causal, scale, stream, device, status_word, Options{});
+}
+
+int b200fa_fwd_piece(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,
+                     const b200fa_tensor4* out, float* lse, int dtype, int causal, float scale, int64_t whole_heads,
+                     void* stream, int device, uint32_t* status_word) {
+  if (q && whole_heads < q->shape[0] * q->shape[1]) return B200FA_ERR_BAD_SHAPE;
+  Options opt;
+  opt.whole_heads = whole_heads;
+  return fwd_impl(q, k, v, out, lse, dtype, causal, scale, stream, device, status_word, opt);
 }
 
 int b200fa_fwd_simt(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,

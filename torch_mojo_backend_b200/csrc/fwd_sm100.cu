@@ -25,6 +25,7 @@
 // 64 with their own S columns: P of a half (16-bit, two per column) overwrites the first 32 of
 // that half's S columns and is consumed as the TMEM A-operand of the P V MMA, and the softmax of
 // one half runs while the tensor pipe works on the other.
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -70,9 +71,89 @@ struct FwdSched {
   int group;       // heads scheduled together so their K/V stay L2-resident
   int nkv_total;   // ceil(Sk / 128)
   bool one_tile;   // the one-tile-per-CTA kernel (two CTAs per SM)
+  int splits;      // CTAs (one cluster) that share a query unit's K/V blocks; 1: no cluster
 };
 
-template <int kD, bool kBf16, bool kCausal, bool kDropout, int kTiles>
+// The last step of a split unit, by the four epilogue warps of each of its kPeers CTAs: a CTA merges
+// its share of the unit's rows.  `s_o`, `s_l`, `s_m` are this CTA's accumulators and row statistics
+// (its peers' lie at the same offsets), `s_w` is scratch of its own.  A peer's shared memory is some
+// hundreds of cycles away, so a thread first turns one row's statistics into weights, and the rows
+// are then summed with eight 16-byte loads in flight per thread (one row and peer at a time, with
+// the statistics read row by row, the merge took 25 us at kPeers = 2).
+template <int kD, int kTiles, bool kBf16, int kPeers>
+__device__ __forceinline__ void merge_split(const FwdParams& p, const uint8_t* s_o, const float* s_l, const float* s_m,
+                                            uint8_t* s_w, int rank, int b, int h, int row0) {
+  constexpr int kShare = kTiles * kBM / kPeers;   // rows, at most the 128 threads
+  const int tid = threadIdx.x & 127;
+  float* weights = reinterpret_cast<float*>(s_w);  // [row][peer]: what the peer's O is multiplied by
+  if (tid < kShare) {
+    const int lr = rank * kShare + tid;   // row of the unit
+    const uint32_t al = smem_u32(s_l + lr), am = smem_u32(s_m + lr);
+    float l[kPeers], m[kPeers], top = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int r = 0; r < kPeers; ++r) {
+      l[r] = peer_load_f32(al, r);
+      m[r] = peer_load_f32(am, r);
+    }
+#pragma unroll
+    for (int r = 0; r < kPeers; ++r) {
+      if (l[r] != 0.f) top = fmaxf(top, m[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < kPeers; ++r) {
+      m[r] = l[r] != 0.f ? ex2_approx((m[r] - top) * p.scale_log2) : 0.f;   // (nothing to add from a peer that saw no key of this row)
+      sum = fmaf(l[r], m[r], sum);
+    }
+    const float inv = sum == 0.f ? 0.f : 1.f / sum;   // (a NaN stays one)
+#pragma unroll
+    for (int r = 0; r < kPeers; ++r) weights[tid * kPeers + r] = l[r] != 0.f ? m[r] * inv : 0.f;
+    if (row0 + lr < p.Sq) {
+      p.lse[(static_cast<int64_t>(b) * p.Hq + h) * p.Sq + row0 + lr] = sum > 0.f ? top * p.scale + logf(sum) : -INFINITY;
+    }
+  }
+  named_bar_sync(1, 128);
+  constexpr int kLanes = kD / 4;                  // 16-byte pieces of a row, one per thread
+  constexpr int kStep = 128 / kLanes;             // rows side by side
+  constexpr int kBatch = 8 / kPeers;              // rows of a thread whose loads are in flight together
+  const int piece = tid % kLanes;
+  const uint32_t base = smem_u32(s_o);
+  static_assert(kShare % (kStep * kBatch) == 0, "whole batches");
+#pragma unroll 1
+  for (int i0 = tid / kLanes; i0 < kShare; i0 += kStep * kBatch) {
+    if (row0 + rank * kShare + i0 >= p.Sq) break;
+    float4 o[kBatch][kPeers];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int lr = rank * kShare + i0 + u * kStep;
+#pragma unroll
+      for (int r = 0; r < kPeers; ++r) o[u][r] = peer_load_f32x4(base + (lr * kD + ((piece ^ (lr & 7)) << 2)) * 4, r);
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = i0 + u * kStep, q_row = row0 + rank * kShare + i;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < kPeers; ++r) {
+        const float w = weights[i * kPeers + r];
+        if (w != 0.f) {   // a peer without a block of this row's tile has not written its O
+          acc.x = fmaf(o[u][r].x, w, acc.x);
+          acc.y = fmaf(o[u][r].y, w, acc.y);
+          acc.z = fmaf(o[u][r].z, w, acc.z);
+          acc.w = fmaf(o[u][r].w, w, acc.w);
+        }
+      }
+      if (q_row < p.Sq) {
+        uint16_t* dst = reinterpret_cast<uint16_t*>(p.out.ptr) + static_cast<int64_t>(b) * p.out.sb +
+                        static_cast<int64_t>(h) * p.out.sh + static_cast<int64_t>(q_row) * p.out.ss + piece * 4;
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<kBf16>(acc.x, acc.y), pack2<kBf16>(acc.z, acc.w));
+      }
+    }
+  }
+}
+
+// kSplit: the K/V blocks of a query unit are dealt to the CTAs of a cluster, which merge their
+// (max, sum, O) through distributed shared memory at the end (choose_splits says when).
+template <int kD, bool kBf16, bool kCausal, bool kDropout, int kTiles, bool kSplit>
 __global__ void __launch_bounds__(FwdCfg<kD, kTiles>::kThreads, kTiles == 2 ? 1 : 2)
 fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
            const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const FwdParams p,
@@ -101,8 +182,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  // a launch whose status word already reports a failed wait is not worth running
-  if (status_is_set(p.status)) return;
+  // a launch whose status word already reports a failed wait is not worth running (the CTAs of a
+  // cluster read each other's shared memory, so there none of them may leave early)
+  if (!kSplit && status_is_set(p.status)) return;
+  const int unit = kSplit ? static_cast<int>(blockIdx.x) / sched.splits : static_cast<int>(blockIdx.x);
+  const int rank = kSplit ? static_cast<int>(blockIdx.x) - unit * sched.splits : 0;   // in the cluster
+  bool peers_met = false;   // this thread has been through the cluster barrier before the merge
 
   // ---- which (pair, head, batch) this CTA owns: head groups keep K/V in L2, and inside a
   // group the heaviest (latest) causal pairs are scheduled first.
@@ -110,9 +195,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
   int pair, bh;
   {
     const int per_group = sched.group * sched.npairs;
-    const int g = blockIdx.x / per_group;
+    const int g = unit / per_group;
     const int gsize = min(sched.group, total_bh - g * sched.group);
-    const int within = blockIdx.x - g * per_group;
+    const int within = unit - g * per_group;
     pair = sched.npairs - 1 - within / gsize;
     bh = g * sched.group + within % gsize;
   }
@@ -138,6 +223,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
       n_t[t] = sched.nkv_total;
     }
   }
+  int j_first = 0;   // this CTA's first K/V block
+  if constexpr (kSplit) {
+    const int n_all = max(n_t[0], n_t[1]);
+    j_first = n_all * rank / sched.splits;
+    const int j_end = n_all * (rank + 1) / sched.splits;
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) n_t[t] = max(0, min(n_t[t], j_end) - j_first);
+  }
   const int n_max = max(n_t[0], n_t[1]);
 
   // Lane 0 of the producer warp sets up the barriers and at once issues the loads that need
@@ -153,11 +246,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
   // K/V ring entry `seq`: K_j for even seq, V_j for odd, j = seq / 2; Q rides along with K_0
   auto produce = [&](int seq) {
     const int slot = seq % Cfg::kStages;
-    const int j = seq >> 1;
+    const int j = j_first + (seq >> 1);
     if (seq == 0) {
       // Q tile 0 rides ahead of K_0, Q tile 1 right behind it
       if (n_t[0] > 0) load_tile(&mapQ, sQ, &q_full[0], row0, h);
-      load_tile(&mapK, sKV + slot * Cfg::kTileBytes, &kv_full[slot], 0, hk);
+      load_tile(&mapK, sKV + slot * Cfg::kTileBytes, &kv_full[slot], j * kBN, hk);
       if (kTiles == 2 && n_t[1] > 0) load_tile(&mapQ, sQ + Cfg::kTileBytes, &q_full[1], row0 + kBM, h);
     } else {
       load_tile((seq & 1) ? &mapV : &mapK, sKV + slot * Cfg::kTileBytes, &kv_full[slot], j * kBN, hk);
@@ -220,7 +313,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
     for (int j = 0; j < nblk; ++j) {
       uint32_t keep_bits[4] = {0, 0, 0, 0};   // dropout: one bit per column of this row of the KV block
       if constexpr (kDropout) {
-        dropout_row_bits(p.drop, b * p.Hq + h, q_row, j * kBN, keep_bits);
+        dropout_row_bits(p.drop, b * p.Hq + h, q_row, (j_first + j) * kBN, keep_bits);
       }
       // The 128 key columns of a block are scored, exponentiated and fed to P V in two halves of
       // 64, each with its own S columns: while this warp works on one half, the tensor pipe runs
@@ -232,7 +325,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
         tc_fence_after();
         uint32_t s[64];
         float* sf = reinterpret_cast<float*>(s);
-        const int col0 = j * kBN + half * 64;
+        const int col0 = (j_first + j) * kBN + half * 64;
         // mask: causal diagonal and/or columns beyond Sk
         const bool need_mask = (kCausal && (col0 + 63 > row0 + t * kBM + p.causal_off)) || (col0 + 64 > p.Sk);
         auto load_scores = [&]() {
@@ -393,10 +486,52 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
       }
       return true;
     };
-    // (a tile that sees its last KV block a step before the other is written out while the other still runs)
-    if (!epilogue(0)) goto teardown;
-    if constexpr (kTiles == 2) {
-      if (!epilogue(1)) goto teardown;
+    if constexpr (kSplit) {
+      // Every MMA of both tiles has completed: the K/V ring is free and takes the unnormalised fp32
+      // O of this CTA, 16-byte pieces of a row permuted by its index.
+      float* sO = reinterpret_cast<float*>(sKV);
+      static_assert(kTiles * kBM * kD * 4 <= Cfg::kStages * Cfg::kTileBytes, "O of every tile fits the ring");
+#pragma unroll
+      for (int t = 0; t < kTiles; ++t) {
+        if (n_t[t] > 0) {
+          // (a wait that gave up has set the status word; these warps go on all the same, since they
+          // meet at a named barrier below and their peers read what they have)
+          if (mbar_wait(&sc_full[t], 0, abort_flag, p.status, 0x200 + t, p.wait_budget))
+            (void)mbar_wait(&o_full[t], 0, abort_flag, p.status, 0x210 + t, p.wait_budget);
+        } else {
+          sMsg[t * 128 + row] = 0.f;
+          sMax[t * 128 + row] = -INFINITY;
+        }
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int t = 0; t < kTiles; ++t) {
+        if (n_t[t] == 0) continue;
+        const uint32_t tO = tmem_base + lane_off + (t == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
+#pragma unroll
+        for (int cidx = 0; cidx < kD / 32; ++cidx) {
+          uint32_t o[32];
+          tmem_ld32(tO + cidx * 32, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int v = 0; v < 8; ++v) {
+            const int piece = cidx * 8 + v;
+            *reinterpret_cast<uint4*>(sO + (t * kBM + row) * kD + ((piece ^ (row & 7)) << 2)) =
+                make_uint4(o[v * 4], o[v * 4 + 1], o[v * 4 + 2], o[v * 4 + 3]);
+          }
+        }
+      }
+      cluster_sync();
+      peers_met = true;
+      if (sched.splits == 2) merge_split<kD, kTiles, kBf16, 2>(p, sKV, sMsg, sMax, sQ, rank, b, h, row0);
+      else if (sched.splits == 4) merge_split<kD, kTiles, kBf16, 4>(p, sKV, sMsg, sMax, sQ, rank, b, h, row0);
+      else merge_split<kD, kTiles, kBf16, 8>(p, sKV, sMsg, sMax, sQ, rank, b, h, row0);
+    } else {
+      // (a tile that sees its last KV block a step before the other is written out while the other still runs)
+      if (!epilogue(0)) goto teardown;
+      if constexpr (kTiles == 2) {
+        if (!epilogue(1)) goto teardown;
+      }
     }
   } else {
     reg_dealloc<Cfg::kRegRest>();
@@ -520,8 +655,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
 
 teardown:
 #undef B200FA_WAIT
+  if constexpr (kSplit) {
+    // every thread of the cluster takes part in both barriers, on every path that leads here
+    __syncwarp();
+    if (!peers_met) cluster_sync();
+  }
   // the staged output tiles must have been read before shared memory is given back
-  if (warp == Cfg::kEpiWarp0 && lane == 0) tma_store_wait_read();
+  if (!kSplit && warp == Cfg::kEpiWarp0 && lane == 0) tma_store_wait_read();
   tc_fence_before();
   __syncthreads();
   if (warp == Cfg::kMmaWarp0) {
@@ -529,13 +669,14 @@ teardown:
     tc_fence_after();
     tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
+  if constexpr (kSplit) cluster_sync();   // no CTA leaves while a peer may still read its shared memory
 }
 
-template <int kD, bool kBf16, bool kCausal, bool kDropout, int kTiles>
+template <int kD, bool kBf16, bool kCausal, bool kDropout, int kTiles, bool kSplit>
 cudaError_t launch_tiles(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                        const FwdParams& p, const FwdSched& sched, cudaStream_t stream) {
   using Cfg = FwdCfg<kD, kTiles>;
-  auto kern = fwd_kernel<kD, kBf16, kCausal, kDropout, kTiles>;
+  auto kern = fwd_kernel<kD, kBf16, kCausal, kDropout, kTiles, kSplit>;
   // cudaFuncSetAttribute once per device for THIS kernel (the flags are statics of this function
   // template: kernels of the same signature must not share them), safe against concurrent first calls
   static std::once_flag once[64];
@@ -553,18 +694,82 @@ cudaError_t launch_tiles(const CUtensorMap& mq, const CUtensorMap& mk, const CUt
   }
   if (e != cudaSuccess) return e;
   const int grid = sched.npairs * p.B * p.Hq;
-  kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(mq, mk, mv, mo, p, sched);
-  return cudaGetLastError();
+  if constexpr (kSplit) {
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = sched.splits;
+    cluster.val.clusterDim.y = 1;
+    cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid * sched.splits);
+    cfg.blockDim = dim3(Cfg::kThreads);
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cfg.stream = stream;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, mo, p, sched);
+  } else {
+    kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(mq, mk, mv, mo, p, sched);
+    return cudaGetLastError();
+  }
+}
+
+// CTAs per query unit.  A grid that leaves SMs idle (few heads, short query blocks against a long
+// cache) has its K/V blocks split over clusters of 2, 4 or 8 CTAs.  The estimate, in units of one
+// K/V block of work: a CTA costs its blocks, a fixed part (set-up, first loads, epilogue) and, with
+// peers, the exchange and merge of the accumulators; the grid then takes no less than its longest
+// CTA, its total over the resident CTAs, and the waves that the longest so many CTAs need.  A split
+// has to promise 5 %.  Measured (us, B200, D = 128 bf16, 1 / 2 / 4 / 8 CTAs per unit, the choice in brackets):
+//   Hq32 Sq512 Sk16896 causal (64 units)  224 / [141] / 144 / 205   Hq16 Sq1024 Sk9000 (64)    125 / [78] / 89 / 135
+//   Hq8 Sq32 Sk4096 (8)                   53 / 33 / 23 / [16]       Hq8 S4096 causal (128)     62 / [51] / 78 / 135
+//   B4 Hq16 S300 unmasked (128)           [14] / 29 / 48 / 100      D=64 B2 Hq16 Sq256 Sk8192  86 / 49 / [38] / 45
+int choose_splits(const FwdParams& p, const FwdSched& sched) {
+  const int rows = (sched.one_tile ? 1 : 2) * kBM;
+  const int per_sm = sched.one_tile ? 2 : 1;
+  // SMs that clusters of 1, 2, 4 and 8 CTAs of one per SM can fill: they do not cross a GPC (measured: the
+  // 34th cluster of 4 and the 16th of 8 wait for a second wave)
+  constexpr int kSMs[4] = {148, 148, 132, 120};
+  const double fixed = p.D == 64 ? 5.0 : 3.0;   // in K/V blocks; the merge costs about as much again
+  const int64_t heads = p.whole_heads;   // a piece of a problem is split as the whole is: the same bits
+  if (heads > kSMs[0] * per_sm || heads * sched.npairs > kSMs[0] * per_sm) return 1;
+  int best = 1;
+  double best_cost = 0.0;
+  for (int c = 1, lg = 0; c <= 8; c *= 2, ++lg) {
+    const int slots = kSMs[lg] * per_sm;
+    const double extra = c == 1 ? fixed : 2.0 * fixed;
+    double total = 0.0, cost = 0.0;
+    int64_t ctas = 0;
+    for (int u = sched.npairs - 1; u >= 0; --u) {   // the longest first
+      int n = sched.nkv_total;
+      if (p.causal) {
+        const int last = std::min((u + 1) * rows, p.Sq) - 1 + p.causal_off;
+        n = last < 0 ? 1 : std::min(n, last / kBN + 1);
+      }
+      const double one = static_cast<double>(n) / c + extra;
+      total += one * heads * c;
+      ctas += heads * c;
+      cost = std::max(cost, static_cast<double>((ctas + slots - 1) / slots) * one);
+    }
+    cost = std::max(cost, total / slots);
+    if (c == 1 || cost < 0.95 * best_cost) {
+      best = c;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 template <int kD, bool kBf16, bool kCausal, bool kDropout>
 cudaError_t launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                        const FwdParams& p, FwdSched sched, cudaStream_t stream) {
-  if (sched.one_tile) {
-    sched.npairs = (p.Sq + kBM - 1) / kBM;
-    return launch_tiles<kD, kBf16, kCausal, kDropout, 1>(mq, mk, mv, mo, p, sched, stream);
+  if (sched.one_tile) sched.npairs = (p.Sq + kBM - 1) / kBM;
+  if constexpr (!kDropout) {
+    sched.splits = p.tiles_per_cta != 0 ? 1 : choose_splits(p, sched);
+    constexpr int kTilesChosen = kD == 64 ? 1 : 2;   // what choose_one_tile says unless it is overridden
+    if (sched.splits > 1) return launch_tiles<kD, kBf16, kCausal, false, kTilesChosen, true>(mq, mk, mv, mo, p, sched, stream);
   }
-  return launch_tiles<kD, kBf16, kCausal, kDropout, 2>(mq, mk, mv, mo, p, sched, stream);
+  return sched.one_tile ? launch_tiles<kD, kBf16, kCausal, kDropout, 1, false>(mq, mk, mv, mo, p, sched, stream)
+                        : launch_tiles<kD, kBf16, kCausal, kDropout, 2, false>(mq, mk, mv, mo, p, sched, stream);
 }
 
 // Which kernel shape.  Two CTAs per SM with one query tile each hide a CTA's set-up, first loads
@@ -611,6 +816,7 @@ cudaError_t launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream,
   if (group > total_bh) group = total_bh;
   sched.group = static_cast<int>(group);
   sched.one_tile = choose_one_tile(p, p.tiles_per_cta);
+  sched.splits = 1;
   cudaError_t e;
   if (p.D == 128) {
     e = bf16 ? launch_mask<128, true>(mq, mk, mv, mo, p, sched, stream)

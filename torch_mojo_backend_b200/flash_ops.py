@@ -9,8 +9,10 @@ an ineligible call raises ``NotImplementedError`` from the forward.
 
 from __future__ import annotations
 
+import contextlib
 import math
 import os
+import threading
 
 import torch
 
@@ -189,6 +191,21 @@ def _dropout_arg(dropout_p: float, philox):
 
 
 # --------------------------------------------------------------------------- forward
+_piece = threading.local()
+
+
+@contextlib.contextmanager
+def piece_of(whole_heads: int):
+    """Forwards of this thread inside the block compute pieces of a problem of `whole_heads` (batch *
+    query heads) and give the bits that one call over the whole would."""
+    before = getattr(_piece, "heads", 0)
+    _piece.heads = int(whole_heads)
+    try:
+        yield
+    finally:
+        _piece.heads = before
+
+
 def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is_causal: bool,
                   scale: float | None, dropout_p: float = 0.0, philox=(0, 0)):
     """Allocate ``out`` (same dtype as q) and ``lse`` (fp32, (B,Hq,Sq)), enqueue the forward
@@ -216,8 +233,10 @@ def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is
         CALL_COUNTERS["forward_split_kv"] += 1
         return out, lse, q_used, k_used, v_used
     _log(f"fwd B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={seq_k} D={head_dim} causal={is_causal} p={dropout_p}")
+    whole = getattr(_piece, "heads", 0)
+    piece = {"whole_heads": whole} if whole else {}
     rc = _lib.fwd(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, code, bool(is_causal), float(scale),
-                  _stream_for(index), index, _status_ptr(index), dropout=_dropout_arg(dropout_p, philox))
+                  _stream_for(index), index, _status_ptr(index), dropout=_dropout_arg(dropout_p, philox), **piece)
     _check(rc, "b200fa_fwd")
     return out, lse, q_used, k_used, v_used
 

@@ -18,6 +18,8 @@ from __future__ import annotations
 
 import torch
 
+from . import flash_ops
+
 
 class PendingPass:
     """One enqueued pass of a ``HostAttentionPipeline``: its pinned host result tensors and the
@@ -110,7 +112,8 @@ class HostAttentionPipeline:
                 uploaded.record(s_in)
             with torch.cuda.stream(s_run):
                 s_run.wait_event(uploaded)
-                fwd = flash_fwd(dev_in[0], dev_in[1], dev_in[2], 0.0, is_causal, False, scale=scale)
+                with flash_ops.piece_of(q.shape[0] * q.shape[1]):
+                    fwd = flash_fwd(dev_in[0], dev_in[1], dev_in[2], 0.0, is_causal, False, scale=scale)
                 o, lse = fwd[0], fwd[1]
                 g = ()
                 if backward:
@@ -150,6 +153,4 @@ class HostAttentionPipeline:
         self._pending.clear()
         main.synchronize()
         # a kernel that gave up on an internal wait has left its results undefined: say so here
-        from . import flash_ops
-
         flash_ops.check_status(self.index)
