@@ -74,7 +74,7 @@ class Tensor4(ctypes.Structure):
     def make(cls, ptr: int, shape: Sequence[int], stride: Sequence[int]) -> "Tensor4":
         if len(shape) != 4 or len(stride) != 4:
             raise ValueError("b200fa tensors are 4-D (batch, heads, seq, head_dim)")
-        return cls(ctypes.c_void_p(ptr), (ctypes.c_int64 * 4)(*shape), (ctypes.c_int64 * 4)(*stride))
+        return cls(ptr, tuple(shape), tuple(stride))
 
 
 class B200FAError(RuntimeError):
@@ -189,13 +189,11 @@ def fwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, dtype: i
     """Raw forward call; returns the library's status code.  `causal` is a bool or one of
     CAUSAL_*; `dropout` is None or ``(p, seed, offset)``; `whole_heads`, if not 0, is batch * query
     heads of the problem this call computes a piece of (see b200fa_fwd_piece)."""
-    head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), ctypes.c_void_p(lse_ptr),
-            dtype, causal_code(causal), ctypes.c_float(scale))
-    tail = (ctypes.c_void_p(stream), device, ctypes.c_void_p(status_ptr))
+    head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), lse_ptr, dtype, int(causal), scale)
+    tail = (stream, device, status_ptr)
     if dropout is not None:
         p, seed, offset = dropout
-        return load().b200fa_fwd_dropout(*head, ctypes.c_float(p), ctypes.c_uint64(seed), ctypes.c_uint64(offset),
-                                         1 if simt else 0, *tail)
+        return load().b200fa_fwd_dropout(*head, p, seed, offset, 1 if simt else 0, *tail)
     if whole_heads and not simt:
         return load().b200fa_fwd_piece(*head, whole_heads, *tail)
     fn = load().b200fa_fwd_simt if simt else load().b200fa_fwd
@@ -210,14 +208,12 @@ def bwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, dout: Tensor4, lse_ptr
     the three backward kernels (see b200fa_bwd_parts); `dropout` is None or ``(p, seed, offset)``
     and must repeat the forward's."""
     head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), ctypes.byref(dout),
-            ctypes.c_void_p(lse_ptr), ctypes.byref(dq), ctypes.byref(dk), ctypes.byref(dv),
-            ctypes.c_void_p(workspace_ptr), ctypes.c_size_t(workspace_bytes), dtype, causal_code(causal),
-            ctypes.c_float(scale))
-    tail = (ctypes.c_void_p(stream), device, ctypes.c_void_p(status_ptr))
+            lse_ptr, ctypes.byref(dq), ctypes.byref(dk), ctypes.byref(dv), workspace_ptr, workspace_bytes, dtype,
+            int(causal), scale)
+    tail = (stream, device, status_ptr)
     if dropout is not None:
         p, seed, offset = dropout
-        return load().b200fa_bwd_dropout(*head, ctypes.c_float(p), ctypes.c_uint64(seed), ctypes.c_uint64(offset),
-                                         1 if simt else 0, *tail)
+        return load().b200fa_bwd_dropout(*head, p, seed, offset, 1 if simt else 0, *tail)
     if parts != 7:
         return load().b200fa_bwd_parts(*head, *tail, parts)
     fn = load().b200fa_bwd_simt if simt else load().b200fa_bwd
@@ -233,9 +229,8 @@ def fwd_splitkv(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, 
                 status_ptr: int = 0) -> int:
     """Raw split-KV (decode) forward; returns the library's status code."""
     return load().b200fa_fwd_splitkv(
-        ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), ctypes.c_void_p(lse_ptr),
-        ctypes.c_void_p(workspace_ptr), ctypes.c_size_t(workspace_bytes), dtype, causal_code(causal),
-        ctypes.c_float(scale), ctypes.c_void_p(stream), device, ctypes.c_void_p(status_ptr))
+        ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), lse_ptr, workspace_ptr,
+        workspace_bytes, dtype, int(causal), scale, stream, device, status_ptr)
 
 
 def dropout_threshold(p: float) -> int:

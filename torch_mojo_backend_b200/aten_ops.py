@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from . import device_module, flash_ops
-from .tensor import TorchMojoTensor, payload
+from .tensor import _DIRECT, TorchMojoTensor, payload
 
 _aten_ops_registry: list[tuple[str, object]] = []
 
@@ -210,11 +210,25 @@ for _name, _overload in (
     ("aten::squeeze.dim", torch.ops.aten.squeeze.dim),
     ("aten::expand", torch.ops.aten.expand.default),
     ("aten::as_strided", torch.ops.aten.as_strided.default),
-    ("aten::alias", torch.ops.aten.alias.default),
-    ("aten::detach", torch.ops.aten.detach.default),
     ("aten::unbind.int", torch.ops.aten.unbind.int),
 ):
     _register_view(_name, _overload)
+
+
+@register_aten_op("aten::alias")
+def mojo_alias(self):
+    base = payload(self)
+    view = TorchMojoTensor._wrap(base._holder, base._ptr, base._shape, base._strides, base._offset, base._dtype,
+                                 base._device_index, base._is_contiguous)
+    if hasattr(base, "_philox"):
+        view._philox = base._philox
+    return view
+
+
+@register_aten_op("aten::detach")
+def mojo_detach(self):
+    # autograd takes one of every output it saves
+    return mojo_alias(self)
 
 
 # ------------------------------------------------------------------------- the hot path
@@ -222,3 +236,11 @@ register_aten_op("aten::_scaled_dot_product_flash_attention")(flash_ops.scaled_d
 register_aten_op("aten::_scaled_dot_product_flash_attention_backward")(
     flash_ops.scaled_dot_product_flash_attention_backward
 )
+
+_DIRECT.update({
+    torch.ops.aten.detach.default: mojo_detach,
+    torch.ops.aten.alias.default: mojo_alias,
+    torch.ops.aten._scaled_dot_product_flash_attention.default: flash_ops.scaled_dot_product_flash_attention,
+    torch.ops.aten._scaled_dot_product_flash_attention_backward.default:
+        flash_ops.scaled_dot_product_flash_attention_backward,
+})

@@ -16,7 +16,7 @@ import threading
 
 import torch
 
-from . import _lib, device_module
+from . import _lib, device_module, tensor
 from .tensor import TorchMojoTensor, payload
 
 _DTYPE_CODES = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
@@ -52,7 +52,7 @@ def _log(msg: str) -> None:
 
 def _stream_for(index: int) -> int:
     """The CUDA stream (as an integer handle) every mojo op on device `index` is ordered on."""
-    return torch.cuda.current_stream(index).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 # --------------------------------------------------------------------------- device status word
@@ -225,9 +225,9 @@ def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is
     code = _DTYPE_CODES[q._dtype]
     if not dropout_p and _decode_shaped(batch, heads_q, heads_kv, seq, seq_k):
         nbytes = _lib.fwd_splitkv_workspace_bytes(batch, heads_q, heads_kv, seq, seq_k, head_dim)
-        workspace = TorchMojoTensor._alloc((nbytes,), torch.uint8, index)
+        workspace = tensor._alloc_holder(nbytes, index)
         _log(f"fwd_splitkv B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={seq_k} D={head_dim}")
-        rc = _lib.fwd_splitkv(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, workspace._ptr, nbytes,
+        rc = _lib.fwd_splitkv(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, workspace.data_ptr(), nbytes,
                               code, bool(is_causal), float(scale), _stream_for(index), index, _status_ptr(index))
         _check(rc, "b200fa_fwd_splitkv")
         CALL_COUNTERS["forward_split_kv"] += 1
@@ -298,10 +298,10 @@ def flash_backward(dout, q, k, v, out, lse, is_causal: bool, scale: float, dropo
     dv = _alloc_like_layout(v._shape, q._dtype, index, bthd_stored(v_used))
     code = _DTYPE_CODES[q._dtype]
     nbytes = _lib.bwd_workspace_bytes(batch, heads_q, heads_kv, seq, head_dim, code)
-    workspace = TorchMojoTensor._alloc((nbytes,), torch.uint8, index)
+    workspace = tensor._alloc_holder(nbytes, index)
     _log(f"bwd B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={k._shape[2]} D={head_dim} causal={is_causal} p={dropout_p}")
     rc = _lib.bwd(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out_used), _t4(dout_used), lse_used._ptr,
-                  _t4(dq), _t4(dk), _t4(dv), workspace._ptr, nbytes, code, bool(is_causal), float(scale),
+                  _t4(dq), _t4(dk), _t4(dv), workspace.data_ptr(), nbytes, code, bool(is_causal), float(scale),
                   _stream_for(index), index, _status_ptr(index), dropout=_dropout_arg(dropout_p, philox))
     _check(rc, "b200fa_bwd")
     # `workspace` drops here: the allocator re-uses it only for work queued later on this stream

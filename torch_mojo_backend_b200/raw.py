@@ -31,7 +31,7 @@ def t4(t: torch.Tensor) -> _lib.Tensor4:
 
 def _stream_and_device(t: torch.Tensor) -> tuple[int, int]:
     dev = t.device.index if t.device.index is not None else torch.cuda.current_device()
-    return torch.cuda.current_stream(dev).cuda_stream, dev
+    return torch._C._cuda_getCurrentRawStream(dev), dev
 
 
 def default_scale(head_dim: int) -> float:

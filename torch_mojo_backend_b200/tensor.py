@@ -18,21 +18,43 @@ import torch
 
 from . import device_module
 
-_WRAPPER_DEVICE_TYPE = "privateuseone"
+_WRAPPER_DEVICE = torch.device("privateuseone", 0)
+_mojo_devices: dict[int, torch.device] = {}
+_cuda_devices: dict[int, torch.device] = {}
+
+#: operators whose kernels __torch_dispatch__ calls itself (filled when they are registered): one trip
+#: through the dispatcher and its argument boxing less, 10-30 us of host time a call
+_DIRECT: dict = {}
+
+
+def _mojo_device(index: int) -> torch.device:
+    dev = _mojo_devices.get(index)
+    if dev is None:
+        dev = _mojo_devices[index] = torch.device("mojo", index)
+    return dev
+
+
+def _cuda_device(index: int) -> torch.device:
+    dev = _cuda_devices.get(index)
+    if dev is None:
+        dev = _cuda_devices[index] = torch.device("cuda", index)
+    return dev
 
 
 def _row_major_strides(shape) -> tuple[int, ...]:
     strides = []
     acc = 1
-    for dim in reversed(tuple(shape)):
+    for dim in reversed(shape):
         strides.append(acc)
-        acc *= max(int(dim), 1)
-    return tuple(reversed(strides))
+        if dim > 1:
+            acc *= dim
+    strides.reverse()
+    return tuple(strides)
 
 
 def _compute_contiguous(shape, strides) -> bool:
     expected = 1
-    for dim, stride in zip(reversed(tuple(shape)), reversed(tuple(strides))):
+    for dim, stride in zip(reversed(shape), reversed(strides)):
         if dim == 1:
             continue
         if stride != expected:
@@ -68,7 +90,7 @@ def pinned_empty(shape, dtype: torch.dtype) -> torch.Tensor:
 
 def _alloc_holder(nbytes: int, index: int) -> torch.Tensor:
     """One device allocation: a flat byte buffer on CUDA device `index` (never zero bytes)."""
-    return torch.empty((max(int(nbytes), 1),), dtype=torch.uint8, device=torch.device("cuda", index))
+    return torch.empty((max(int(nbytes), 1),), dtype=torch.uint8, device=_cuda_device(index))
 
 
 def _holder_ptr(holder: torch.Tensor) -> int:
@@ -82,67 +104,77 @@ class TorchMojoTensor(torch.Tensor):
 
     @classmethod
     def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
-        if not all(issubclass(cls, t) for t in types):
-            return NotImplemented
+        for t in types:
+            if t is not cls and not issubclass(cls, t):
+                return NotImplemented
         # Redispatch below the Python key so the call reaches the PrivateUse1 kernels
         # registered in aten_ops.py (reference: deferred_compile.py:53-58).
         with torch._C._DisableTorchDispatch():
-            return func(*args, **(kwargs or {}))
+            return _DIRECT.get(func, func)(*args, **(kwargs or {}))
 
     __torch_function__ = torch._C._disabled_torch_function_impl
 
     # ------------------------------------------------------------------ construction
     @classmethod
     def _make(cls, holder, ptr, shape, strides, offset, dtype, index, contiguous=None) -> "TorchMojoTensor":
-        shape = tuple(int(s) for s in shape)
-        strides = tuple(int(s) for s in strides)
+        shape = tuple(map(int, shape))
+        strides = tuple(map(int, strides))
+        if contiguous is None:
+            contiguous = _compute_contiguous(shape, strides)
+        return cls._wrap(holder, int(ptr), shape, strides, int(offset), dtype, int(index), contiguous)
+
+    @classmethod
+    def _wrap(cls, holder, ptr, shape, strides, offset, dtype, index, contiguous) -> "TorchMojoTensor":
+        """`_make` with every argument already in its final form (ints, tuples of ints)."""
         res = torch.Tensor._make_wrapper_subclass(
             cls,
             shape,
             strides=strides,
-            storage_offset=int(offset),
+            storage_offset=offset,
             dtype=dtype,
             layout=torch.strided,
-            device=torch.device(_WRAPPER_DEVICE_TYPE, 0),
+            device=_WRAPPER_DEVICE,
             requires_grad=False,
         )
-        res._holder = holder
-        res._ptr = int(ptr)
-        res._shape = shape
-        res._strides = strides
-        res._offset = int(offset)
-        res._dtype = dtype
-        res._itemsize = torch.empty((), dtype=dtype).element_size()
-        res._numel = math.prod(shape)
-        res._device_index = int(index)
-        res._torch_device = torch.device("mojo", int(index))
-        res._is_contiguous = _compute_contiguous(shape, strides) if contiguous is None else contiguous
+        res.__dict__.update(
+            _holder=holder,
+            _ptr=ptr,
+            _shape=shape,
+            _strides=strides,
+            _offset=offset,
+            _dtype=dtype,
+            _itemsize=dtype.itemsize,
+            _numel=math.prod(shape),
+            _device_index=index,
+            _torch_device=_mojo_device(index),
+            _is_contiguous=contiguous,
+        )
         return res
 
     @classmethod
     def _alloc(cls, shape, dtype: torch.dtype, index: int | None = None) -> "TorchMojoTensor":
         """A new contiguous uninitialised tensor (one device allocation)."""
         index = device_module.current_device() if index is None else index
-        shape = tuple(int(s) for s in shape)
-        itemsize = torch.empty((), dtype=dtype).element_size()
-        holder = _alloc_holder(math.prod(shape) * itemsize, index)
-        return cls._make(holder, _holder_ptr(holder), shape, _row_major_strides(shape), 0, dtype, index, True)
+        shape = tuple(map(int, shape))
+        holder = _alloc_holder(math.prod(shape) * dtype.itemsize, index)
+        return cls._wrap(holder, _holder_ptr(holder), shape, _row_major_strides(shape), 0, dtype, index, True)
 
     @classmethod
     def _alloc_strided(cls, shape, strides, dtype: torch.dtype, index: int | None = None) -> "TorchMojoTensor":
         """A new tensor with the given (non-overlapping) strides, e.g. BTHD-stored BHSD."""
         index = device_module.current_device() if index is None else index
-        shape = tuple(int(s) for s in shape)
-        strides = tuple(int(s) for s in strides)
-        itemsize = torch.empty((), dtype=dtype).element_size()
+        shape = tuple(map(int, shape))
+        strides = tuple(map(int, strides))
         extent = 1 + sum((d - 1) * s for d, s in zip(shape, strides)) if math.prod(shape) else 0
-        holder = _alloc_holder(extent * itemsize, index)
-        return cls._make(holder, _holder_ptr(holder), shape, strides, 0, dtype, index)
+        holder = _alloc_holder(extent * dtype.itemsize, index)
+        return cls._wrap(holder, _holder_ptr(holder), shape, strides, 0, dtype, index,
+                         _compute_contiguous(shape, strides))
 
     @classmethod
     def _view_of(cls, base: "TorchMojoTensor", shape, strides, offset, contiguous=None) -> "TorchMojoTensor":
         """A zero-copy view sharing base's holder; `offset` is absolute, in elements."""
-        ptr = base._ptr + (int(offset) - base._offset) * base._itemsize
+        offset = int(offset)
+        ptr = base._ptr + (offset - base._offset) * base._itemsize
         view = cls._make(base._holder, ptr, shape, strides, offset, base._dtype, base._device_index, contiguous)
         if hasattr(base, "_philox"):
             # the (seed, offset) pair an rng_state tensor carries on the host survives detach / alias
@@ -173,8 +205,11 @@ class TorchMojoTensor(torch.Tensor):
         """The same memory as a plain CUDA tensor (for copies and DLPack export)."""
         holder = self._holder
         if holder.dtype == torch.uint8 and holder.dim() == 1:
-            nbytes = holder.numel() - holder.numel() % self._itemsize
-            typed = holder[:nbytes].view(self._dtype) if nbytes else holder.new_empty((0,), dtype=self._dtype)
+            nbytes = holder.numel()
+            spare = nbytes % self._itemsize
+            if spare:
+                holder = holder[: nbytes - spare]
+            typed = holder.view(self._dtype) if nbytes > spare else holder.new_empty((0,), dtype=self._dtype)
             return torch.as_strided(typed, self._shape, self._strides, self._offset)
         # adopted foreign CUDA tensor: offset is relative to its own first element
         flat_extent_ok = holder.dtype == self._dtype
