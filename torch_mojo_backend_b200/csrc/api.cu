@@ -337,24 +337,32 @@ int bwd_impl(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tens
   return e == cudaSuccess ? B200FA_OK : B200FA_ERR_CUDA;
 }
 
-// Key splits of the split-KV forward.  The partial kernel keeps three 4-warp CTAs per SM (444 at
-// a time on 148 SMs) when a KV head has up to eight query rows, two with more, and a grid runs
-// for about (its waves) x (keys in a split + a fixed cost per CTA worth some 192 keys: prologue,
-// merge of the warps, the partial written and combined).  Among the split counts up to 64 with
-// at least 256 keys a split, take the cheapest by that model; the first found wins a tie, which
-// is the one with fewer splits.
-int splitkv_splits(int64_t B, int64_t Hkv, int64_t rows, int64_t Sk, int* split_len) {
-  const int64_t slots = (rows <= 8 ? 3 : 2) * 148;
+// Key splits of the split-KV forward: the count up to 64, of at least 256 keys each, that the model
+// below finds cheapest; the first found wins a tie, which is the one with fewer splits.
+// The grid runs in waves of the CTAs that fit: by registers, 3 and 2 per SM of the 16-bit kernel at
+// D = 128 (up to 8 query rows per KV head, and more), 4 and 3 at D = 64; 2 and 1 of the fp32 kernel (up
+// to 4 rows, and more).  A wave costs its keys and a fixed part worth some 192 keys (prologue, merge of
+// the warps, the partial written and combined); a wave that is not full gives each of its CTAs more of
+// HBM, until about 0.85 of the CTAs that fit saturate it.  Measured (us, B200; before = every wave taken
+// as full, 3 or 2 CTAs per SM whatever the type and D):
+//   B8 Hq32 Hkv8 Sk32768 D128 bf16     170 -> 165 (6 splits)     16 rows: B16 Hq32 Hkv8 Sq4 Sk16384  193 -> 182 (2)
+//   16 rows, D64: B8 Hkv8 Sk8000 fp16  44.4 -> 34.9 (6)          fp32: B8 Hkv8 Sk8192 D128 4 rows    121 -> 95 (4)
+//   fp32: B4 Hkv2 Sk5000 D64 16 rows   47.2 -> 30.8 (16)         fp32: B4 Hkv12 Sk9000 D64 1 row     51.2 -> 43.9 (6)
+int splitkv_splits(int64_t B, int64_t Hkv, int64_t rows, int64_t Sk, int64_t D, bool fp32, int* split_len) {
+  const int64_t per_sm = fp32 ? (rows <= 4 ? 2 : 1) : D == 64 ? (rows <= 8 ? 4 : 3) : (rows <= 8 ? 3 : 2);
+  const int64_t slots = per_sm * 148;
   int64_t max_n = (Sk + 255) / 256;
   if (max_n > 64) max_n = 64;
   if (max_n < 1) max_n = 1;
-  int64_t best_n = 1, best_len = (Sk + 63) / 64 * 64, best_cost = -1;
+  int64_t best_n = 1, best_len = (Sk + 63) / 64 * 64;
+  double best_cost = -1.0;
   for (int64_t cand = 1; cand <= max_n; ++cand) {
     const int64_t len = ((Sk + cand - 1) / cand + 63) / 64 * 64;
     const int64_t n = (Sk + len - 1) / len;
-    const int64_t waves = (B * Hkv * n + slots - 1) / slots;
-    const int64_t cost = waves * (len + 192);
-    if (best_cost < 0 || cost < best_cost) {
+    const int64_t full = B * Hkv * n / slots, rest = B * Hkv * n % slots;
+    double cost = static_cast<double>(full) * (len + 192);
+    if (rest > 0) cost += len * std::max(0.85, static_cast<double>(rest) / slots) + 192.0;
+    if (best_cost < 0.0 || cost < best_cost) {
       best_cost = cost;
       best_n = n;
       best_len = len;
@@ -500,8 +508,11 @@ int b200fa_bwd_simt(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200
 size_t b200fa_fwd_splitkv_workspace_bytes(int64_t batch, int64_t heads_q, int64_t heads_kv, int64_t seqlen_q,
                                           int64_t seqlen_k, int64_t head_dim) {
   if (batch <= 0 || heads_q <= 0 || heads_kv <= 0 || seqlen_q <= 0 || seqlen_k <= 0 || head_dim <= 0) return 0;
+  // (the size is asked for without the element type: enough for either)
   int split_len = 0;
-  const int n = splitkv_splits(batch, heads_kv, heads_q / heads_kv * seqlen_q, seqlen_k, &split_len);
+  const int64_t group_rows = heads_q / heads_kv * seqlen_q;
+  const int n = std::max(splitkv_splits(batch, heads_kv, group_rows, seqlen_k, head_dim, false, &split_len),
+                         splitkv_splits(batch, heads_kv, group_rows, seqlen_k, head_dim, true, &split_len));
   const size_t rows = static_cast<size_t>(batch) * heads_q * seqlen_q * n;
   return align256(rows * head_dim * 4) + align256(rows * 2 * 4) + align256(static_cast<size_t>(batch) * heads_kv * 4);
 }
@@ -533,7 +544,7 @@ int b200fa_fwd_splitkv(const b200fa_tensor4* q, const b200fa_tensor4* k, const b
   const size_t need = b200fa_fwd_splitkv_workspace_bytes(B, Hq, Hkv, Sq, Sk, D);
   if (!workspace || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
     return B200FA_ERR_WORKSPACE;
-  p.nsplit = splitkv_splits(B, Hkv, Hq / Hkv * Sq, Sk, &p.split_len);
+  p.nsplit = splitkv_splits(B, Hkv, Hq / Hkv * Sq, Sk, D, dtype == kF32, &p.split_len);
   const size_t rows = static_cast<size_t>(B) * Hq * Sq * p.nsplit;
   p.part_o = reinterpret_cast<float*>(workspace);
   p.part_ml = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(rows * D * 4));
