@@ -77,6 +77,23 @@ __device__ __forceinline__ uint32_t dropout_bits16(const DropoutParams& d, int b
   return bits;
 }
 
+// 32 x 32 bits across a warp, transposed: bit e of lane l becomes bit l of lane e.  Five exchanges of
+// halves; 32 ballots cost five times the instructions.
+__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t keep_even = 0x0000ffffu;   // columns whose index has bit j clear
+#pragma unroll
+  for (int j = 16; j >= 1; j >>= 1) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, x, j);
+    const bool up = lane & j;
+    const uint32_t moved = up ? other >> j : other << j;
+    const uint32_t own = up ? ~keep_even : keep_even;
+    x = (x & own) | (moved & ~own);
+    keep_even ^= keep_even << (j >> 1);
+  }
+  return x;
+}
+
 // keep-bits of the 128 key columns [col0, col0 + 128) of one query row (col0 a multiple of 128):
 // bits[w] bit i <-> column col0 + 32*w + i
 __device__ __forceinline__ void dropout_row_bits(const DropoutParams& d, int bh, int row, int col0,
