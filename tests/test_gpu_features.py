@@ -78,6 +78,24 @@ def test_forward_split_over_clusters(dtype, B, Hq, Hkv, Sq, Sk, D, mode):
     assert (lse.cpu() - ref_lse)[seen].abs().max().item() < TOL_LSE
 
 
+@pytest.mark.parametrize("Hq,Sq,Sk,D,mode", [(1, 256, 4096, 128, 2), (2, 300, 3000, 64, 0), (64, 1024, 1024, 128, 1)])
+def test_a_launch_whose_status_word_is_set_writes_nothing(Hq, Sq, Sk, D, mode):
+    """Whether the K/V blocks are dealt to clusters (the first two shapes) or not."""
+    q, k, v, _ = draw(torch.bfloat16, 1, Hq, Hq, Sq, Sk, D, 3)
+    qc, kc, vc = q.cuda(), k.cuda(), v.cuda()
+    status = torch.full((1,), 0x57410100, dtype=torch.int32, device="cuda")
+    out, lse = torch.full_like(qc, 7.0), torch.full((1, Hq, Sq), 7.0, device="cuda")
+    raw.flash_fwd(qc, kc, vc, causal=mode, out=out, lse=lse, status=status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0x57410100
+    assert bool((out == 7.0).all()) and bool((lse == 7.0).all())
+    status.zero_()
+    raw.flash_fwd(qc, kc, vc, causal=mode, out=out, lse=lse, status=status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert_within("out", out, O.sdpa_forward(q, k, v, mode, D ** -0.5)[0], TOL_16BIT, torch.bfloat16)
+
+
 ALIGNED = [
     # dtype, B, Hq, Hkv, Sq, Sk, D, mode (1 top-left = torch's is_causal, 2 bottom-right = the reference kernels' rule)
     (torch.bfloat16, 2, 4, 2, 128, 320, 128, 1),

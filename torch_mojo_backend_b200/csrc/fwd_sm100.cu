@@ -79,12 +79,18 @@ struct FwdSched {
 // (its peers' lie at the same offsets), `s_w` is scratch of its own.  A peer's shared memory is some
 // hundreds of cycles away, so a thread first turns one row's statistics into weights, and the rows
 // are then summed with eight 16-byte loads in flight per thread (one row and peer at a time, with
-// the statistics read row by row, the merge took 25 us at kPeers = 2).
+// the statistics read row by row, the merge took 25 us at kPeers = 2).  Where a peer's abort flag
+// is up nothing is written: no wait runs behind the barrier before this, so all peers see the same.
 template <int kD, int kTiles, bool kBf16, int kPeers>
 __device__ __forceinline__ void merge_split(const FwdParams& p, const uint8_t* s_o, const float* s_l, const float* s_m,
-                                            uint8_t* s_w, int rank, int b, int h, int row0) {
+                                            uint8_t* s_w, const volatile uint32_t* abort_flag, int rank, int b, int h,
+                                            int row0) {
   constexpr int kShare = kTiles * kBM / kPeers;   // rows, at most the 128 threads
   const int tid = threadIdx.x & 127;
+  uint32_t aborted = 0;
+#pragma unroll
+  for (int r = 0; r < kPeers; ++r) aborted |= peer_load_u32(smem_u32(const_cast<const uint32_t*>(abort_flag)), r);
+  if (aborted) return;
   float* weights = reinterpret_cast<float*>(s_w);  // [row][peer]: what the peer's O is multiplied by
   if (tid < kShare) {
     const int lr = rank * kShare + tid;   // row of the unit
@@ -178,12 +184,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
   uint64_t* xturn = sc_full + 2;                // [2 tiles][4 warps] the two tiles' exponential phases take turns
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xturn + 8);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  volatile uint32_t* skip_flag = tmem_slot + 2;   // kSplit: the status word was set when this CTA started
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
   // a launch whose status word already reports a failed wait is not worth running (the CTAs of a
-  // cluster read each other's shared memory, so there none of them may leave early)
+  // cluster read each other's shared memory, so there they skip the work and meet at its barriers)
   if (!kSplit && status_is_set(p.status)) return;
   const int unit = kSplit ? static_cast<int>(blockIdx.x) / sched.splits : static_cast<int>(blockIdx.x);
   const int rank = kSplit ? static_cast<int>(blockIdx.x) - unit * sched.splits : 0;   // in the cluster
@@ -259,6 +266,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
   const int n_loads = 2 * n_max;
   constexpr int kEarlyLoads = 2;   // Q, K_0 and V_0: what the first MMAs wait for; more would only delay the sync
   if (warp == Cfg::kTmaWarp && lane == 0) {
+    const bool skip = kSplit && status_is_set(p.status);   // read here, needed behind the barriers' set-up
     mbar_init(&q_full[0], 1);
     mbar_init(&q_full[1], 1);
     for (int i = 0; i < Cfg::kStages; ++i) {
@@ -277,10 +285,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
       mbar_init(&sc_full[t], 4);
       for (int w = 0; w < 4; ++w) mbar_init(&xturn[t * 4 + w], 1);
     }
-    *abort_flag = 0;
+    *abort_flag = skip;
+    if constexpr (kSplit) *skip_flag = skip;
     fence_mbar_init();
     fence_proxy_async_smem();
-    for (int seq = 0; seq < min(n_loads, kEarlyLoads); ++seq) produce(seq);
+    if (!skip) {
+      for (int seq = 0; seq < min(n_loads, kEarlyLoads); ++seq) produce(seq);
+    }
   }
   if (warp == Cfg::kMmaWarp0) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -294,7 +305,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
 #define B200FA_WAIT(bar, parity, site) \
   if (!mbar_wait((bar), (parity), abort_flag, p.status, (site), p.wait_budget)) goto teardown
 
-  if (warp < 4 * kTiles) {
+  if (kSplit && *skip_flag) {
+    // nothing was loaded: straight to the barriers of the cluster
+  } else if (warp < 4 * kTiles) {
     // =========================== softmax warps ===========================
     reg_alloc<Cfg::kRegSoftmax>();
     const int t = warp >> 2;
@@ -523,9 +536,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUt
       }
       cluster_sync();
       peers_met = true;
-      if (sched.splits == 2) merge_split<kD, kTiles, kBf16, 2>(p, sKV, sMsg, sMax, sQ, rank, b, h, row0);
-      else if (sched.splits == 4) merge_split<kD, kTiles, kBf16, 4>(p, sKV, sMsg, sMax, sQ, rank, b, h, row0);
-      else merge_split<kD, kTiles, kBf16, 8>(p, sKV, sMsg, sMax, sQ, rank, b, h, row0);
+      if (sched.splits == 2) merge_split<kD, kTiles, kBf16, 2>(p, sKV, sMsg, sMax, sQ, abort_flag, rank, b, h, row0);
+      else if (sched.splits == 4) merge_split<kD, kTiles, kBf16, 4>(p, sKV, sMsg, sMax, sQ, abort_flag, rank, b, h, row0);
+      else merge_split<kD, kTiles, kBf16, 8>(p, sKV, sMsg, sMax, sQ, abort_flag, rank, b, h, row0);
     } else {
       // (a tile that sees its last KV block a step before the other is written out while the other still runs)
       if (!epilogue(0)) goto teardown;

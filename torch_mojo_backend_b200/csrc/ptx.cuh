@@ -322,6 +322,11 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t saddr, int rank) {
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
   return a;
 }
+__device__ __forceinline__ uint32_t peer_load_u32(uint32_t saddr, int rank) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(saddr, rank)) : "memory");
+  return v;
+}
 __device__ __forceinline__ float peer_load_f32(uint32_t saddr, int rank) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(peer_addr(saddr, rank)) : "memory");
