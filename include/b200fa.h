@@ -202,14 +202,21 @@ int b200fa_bwd_no_alloc(const b200fa_tensor4* q, const b200fa_tensor4* k, const 
 size_t b200fa_no_alloc_scratch_bytes(void);
 
 /*
- * b200fa_fwd for a piece - some batch entries or whole groups of heads - of a problem with
- * `whole_heads` = batch * query heads in all (at least the piece's own).  How a small forward is dealt
- * to the SMs depends on that number, and with it the order of some sums; a piece computed through this
- * call has the bits that one call over the whole problem would give it.
+ * b200fa_fwd and b200fa_fwd_splitkv for a piece - some batch entries or whole groups of heads - of a
+ * problem with `whole_heads` = batch * query heads in all (at least the piece's own).  How a small
+ * forward and a split-KV call are dealt to the SMs depends on that number, and with it the order of some
+ * sums; a piece computed through these calls has the bits that one call over the whole problem would give it.
  */
 int b200fa_fwd_piece(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,
                      const b200fa_tensor4* out, float* lse, int dtype, int causal, float scale,
                      int64_t whole_heads, void* stream, int device, uint32_t* status_word);
+size_t b200fa_fwd_splitkv_piece_workspace_bytes(int64_t batch, int64_t heads_q, int64_t heads_kv,
+                                                int64_t seqlen_q, int64_t seqlen_k, int64_t head_dim,
+                                                int64_t whole_heads);
+int b200fa_fwd_splitkv_piece(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,
+                             const b200fa_tensor4* out, float* lse, void* workspace, size_t workspace_bytes,
+                             int dtype, int causal, float scale, int64_t whole_heads, void* stream,
+                             int device, uint32_t* status_word);
 
 /*
  * Same contracts as b200fa_fwd / b200fa_bwd, but always run the exact-fp32 SIMT kernels

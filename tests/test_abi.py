@@ -151,6 +151,22 @@ def test_split_count_fills_whole_waves_of_the_grid():
     assert _splits_of(1, 8, 8, 1, 600, 64) <= 3 and _splits_of(2, 4, 4, 1, 200, 64) == 1
 
 
+def test_a_piece_of_a_split_kv_call_is_cut_as_the_whole():
+    al = lambda x: (x + 255) // 256 * 256
+    for B, Hq, Hkv, Sq, Sk, D in ((8, 32, 8, 1, 32768, 128), (16, 8, 8, 2, 5000, 64), (2, 12, 4, 5, 70000, 128)):
+        n, rows = _splits_of(B, Hq, Hkv, Sq, Sk, D), Hq * Sq
+        assert n != _splits_of(1, Hq, Hkv, Sq, Sk, D)
+        want = al(rows * n * D * 4) + al(rows * n * 8) + al(Hkv * 4)
+        assert _lib.fwd_splitkv_workspace_bytes(1, Hq, Hkv, Sq, Sk, D, whole_heads=B * Hq) == want
+    # a whole problem is its own piece; a piece larger than the whole is refused
+    assert (_lib.fwd_splitkv_workspace_bytes(8, 32, 8, 1, 32768, 128, whole_heads=256)
+            == _lib.fwd_splitkv_workspace_bytes(8, 32, 8, 1, 32768, 128))
+    assert _lib.fwd_splitkv_workspace_bytes(8, 32, 8, 1, 32768, 128, whole_heads=255) == 0
+    q, k = _t4(FAKE, (8, 32, 1, 128)), _t4(FAKE + 0x100000, (8, 8, 4096, 128))
+    assert _lib.fwd_splitkv(q, k, k, q, FAKE + 0x400000, FAKE + 0x500000, 1 << 30, _lib.BF16, False, 0.1, 0, 0,
+                            whole_heads=255) == _lib.ERR_BAD_SHAPE
+
+
 def test_forward_kernel_shape_setter():
     assert _lib.fwd_tiles() in (0, 1, 2)
     for tiles in (1, 2, 0):

@@ -170,3 +170,21 @@ def test_host_attention_pipeline_is_bitwise_the_single_call(mojo_registered):
     res_out, grads = pipe2.run(hq, hk, hv, None, is_causal=True)
     pipe2.synchronize()
     assert grads is None and torch.equal(res_out, out.detach().cpu())
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,dtype", [(8, 16, 4, 1, 6000, torch.bfloat16), (5, 8, 8, 3, 9000, torch.float32),
+                                                  (4, 4, 2, 200, 4096, torch.float16)])
+def test_host_attention_pipeline_is_bitwise_the_single_call_over_long_caches(mojo_registered, B, Hq, Hkv, Sq, Sk, dtype):
+    """Decode shapes (split-KV) and short query blocks, whose key splits depend on the number of heads."""
+    import torch_mojo_backend_b200 as tmb
+
+    g = torch.Generator().manual_seed(22)
+    hq, hk, hv = (tmb.pinned_empty(shape, dtype).copy_(torch.randn(shape, generator=g) * 0.5)
+                  for shape in ((B, Hq, Sq, 128), (B, Hkv, Sk, 128), (B, Hkv, Sk, 128)))
+    mq, mk, mv = (t.to("mojo") for t in (hq, hk, hv))
+    out = torch.nn.functional.scaled_dot_product_attention(mq, mk, mv, enable_gqa=Hq != Hkv).cpu()
+    pipe = tmb.HostAttentionPipeline(0, piece_bytes=1 << 20)
+    assert len(pipe.pieces(hq, hk, False)) == 2 * B
+    res, _ = pipe.run(hq, hk, hv, None, is_causal=False)
+    pipe.synchronize()
+    assert torch.equal(res, out)

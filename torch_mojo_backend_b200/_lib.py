@@ -48,6 +48,8 @@ EXPORTED_SYMBOLS = (
     "b200fa_dropout_bytes_host",
     "b200fa_fwd_splitkv_workspace_bytes",
     "b200fa_fwd_splitkv",
+    "b200fa_fwd_splitkv_piece_workspace_bytes",
+    "b200fa_fwd_splitkv_piece",
     "b200fa_set_wait_budget",
     "b200fa_wait_budget",
     "b200fa_set_fwd_tiles",
@@ -132,10 +134,14 @@ def load() -> ctypes.CDLL:
     lib.b200fa_dropout_bytes_host.restype = None
     lib.b200fa_fwd_splitkv_workspace_bytes.argtypes = [ctypes.c_int64] * 6
     lib.b200fa_fwd_splitkv_workspace_bytes.restype = ctypes.c_size_t
-    lib.b200fa_fwd_splitkv.argtypes = [t4p, t4p, t4p, t4p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t,
-                                       ctypes.c_int, ctypes.c_int, ctypes.c_float, ctypes.c_void_p, ctypes.c_int,
-                                       ctypes.c_void_p]
+    lib.b200fa_fwd_splitkv_piece_workspace_bytes.argtypes = [ctypes.c_int64] * 7
+    lib.b200fa_fwd_splitkv_piece_workspace_bytes.restype = ctypes.c_size_t
+    split_args = [t4p, t4p, t4p, t4p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int,
+                  ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+    lib.b200fa_fwd_splitkv.argtypes = split_args
     lib.b200fa_fwd_splitkv.restype = ctypes.c_int
+    lib.b200fa_fwd_splitkv_piece.argtypes = split_args[:10] + [ctypes.c_int64] + split_args[10:]
+    lib.b200fa_fwd_splitkv_piece.restype = ctypes.c_int
     lib.b200fa_set_wait_budget.argtypes = [ctypes.c_longlong]
     lib.b200fa_set_wait_budget.restype = None
     lib.b200fa_wait_budget.argtypes = []
@@ -220,17 +226,23 @@ def bwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, dout: Tensor4, lse_ptr
     return fn(*head, *tail)
 
 
-def fwd_splitkv_workspace_bytes(B: int, Hq: int, Hkv: int, Sq: int, Sk: int, D: int) -> int:
+def fwd_splitkv_workspace_bytes(B: int, Hq: int, Hkv: int, Sq: int, Sk: int, D: int, whole_heads: int = 0) -> int:
+    if whole_heads:
+        return int(load().b200fa_fwd_splitkv_piece_workspace_bytes(B, Hq, Hkv, Sq, Sk, D, whole_heads))
     return int(load().b200fa_fwd_splitkv_workspace_bytes(B, Hq, Hkv, Sq, Sk, D))
 
 
 def fwd_splitkv(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, workspace_ptr: int,
                 workspace_bytes: int, dtype: int, causal, scale: float, stream: int, device: int,
-                status_ptr: int = 0) -> int:
-    """Raw split-KV (decode) forward; returns the library's status code."""
-    return load().b200fa_fwd_splitkv(
-        ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), lse_ptr, workspace_ptr,
-        workspace_bytes, dtype, int(causal), scale, stream, device, status_ptr)
+                status_ptr: int = 0, *, whole_heads: int = 0) -> int:
+    """Raw split-KV (decode) forward; returns the library's status code.  `whole_heads` as for `fwd`
+    (the workspace is then that of the piece)."""
+    head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), lse_ptr, workspace_ptr,
+            workspace_bytes, dtype, int(causal), scale)
+    tail = (stream, device, status_ptr)
+    if whole_heads:
+        return load().b200fa_fwd_splitkv_piece(*head, whole_heads, *tail)
+    return load().b200fa_fwd_splitkv(*head, *tail)
 
 
 def dropout_threshold(p: float) -> int:

@@ -348,7 +348,8 @@ int bwd_impl(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tens
 //   B8 Hq32 Hkv8 Sk32768 D128 bf16     170 -> 165 (6 splits)     16 rows: B16 Hq32 Hkv8 Sq4 Sk16384  193 -> 182 (2)
 //   16 rows, D64: B8 Hkv8 Sk8000 fp16  44.4 -> 34.9 (6)          fp32: B8 Hkv8 Sk8192 D128 4 rows    121 -> 95 (4)
 //   fp32: B4 Hkv2 Sk5000 D64 16 rows   47.2 -> 30.8 (16)         fp32: B4 Hkv12 Sk9000 D64 1 row     51.2 -> 43.9 (6)
-int splitkv_splits(int64_t B, int64_t Hkv, int64_t rows, int64_t Sk, int64_t D, bool fp32, int* split_len) {
+// `kv_heads`: batch * KV heads, of the whole problem if the call computes a piece of one.
+int splitkv_splits(int64_t kv_heads, int64_t rows, int64_t Sk, int64_t D, bool fp32, int* split_len) {
   const int64_t per_sm = fp32 ? (rows <= 4 ? 2 : 1) : D == 64 ? (rows <= 8 ? 4 : 3) : (rows <= 8 ? 3 : 2);
   const int64_t slots = per_sm * 148;
   int64_t max_n = (Sk + 255) / 256;
@@ -359,7 +360,7 @@ int splitkv_splits(int64_t B, int64_t Hkv, int64_t rows, int64_t Sk, int64_t D, 
   for (int64_t cand = 1; cand <= max_n; ++cand) {
     const int64_t len = ((Sk + cand - 1) / cand + 63) / 64 * 64;
     const int64_t n = (Sk + len - 1) / len;
-    const int64_t full = B * Hkv * n / slots, rest = B * Hkv * n % slots;
+    const int64_t full = kv_heads * n / slots, rest = kv_heads * n % slots;
     double cost = static_cast<double>(full) * (len + 192);
     if (rest > 0) cost += len * std::max(0.85, static_cast<double>(rest) / slots) + 192.0;
     if (best_cost < 0.0 || cost < best_cost) {
@@ -505,21 +506,36 @@ int b200fa_bwd_simt(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200
                   device, status_word, opt);
 }
 
-size_t b200fa_fwd_splitkv_workspace_bytes(int64_t batch, int64_t heads_q, int64_t heads_kv, int64_t seqlen_q,
-                                          int64_t seqlen_k, int64_t head_dim) {
+size_t b200fa_fwd_splitkv_piece_workspace_bytes(int64_t batch, int64_t heads_q, int64_t heads_kv, int64_t seqlen_q,
+                                                int64_t seqlen_k, int64_t head_dim, int64_t whole_heads) {
   if (batch <= 0 || heads_q <= 0 || heads_kv <= 0 || seqlen_q <= 0 || seqlen_k <= 0 || head_dim <= 0) return 0;
+  if (heads_q < heads_kv || whole_heads < batch * heads_q) return 0;
   // (the size is asked for without the element type: enough for either)
   int split_len = 0;
-  const int64_t group_rows = heads_q / heads_kv * seqlen_q;
-  const int n = std::max(splitkv_splits(batch, heads_kv, group_rows, seqlen_k, head_dim, false, &split_len),
-                         splitkv_splits(batch, heads_kv, group_rows, seqlen_k, head_dim, true, &split_len));
+  const int64_t group = heads_q / heads_kv;
+  const int n = std::max(splitkv_splits(whole_heads / group, group * seqlen_q, seqlen_k, head_dim, false, &split_len),
+                         splitkv_splits(whole_heads / group, group * seqlen_q, seqlen_k, head_dim, true, &split_len));
   const size_t rows = static_cast<size_t>(batch) * heads_q * seqlen_q * n;
   return align256(rows * head_dim * 4) + align256(rows * 2 * 4) + align256(static_cast<size_t>(batch) * heads_kv * 4);
+}
+
+size_t b200fa_fwd_splitkv_workspace_bytes(int64_t batch, int64_t heads_q, int64_t heads_kv, int64_t seqlen_q,
+                                          int64_t seqlen_k, int64_t head_dim) {
+  return b200fa_fwd_splitkv_piece_workspace_bytes(batch, heads_q, heads_kv, seqlen_q, seqlen_k, head_dim,
+                                                  batch * heads_q);
 }
 
 int b200fa_fwd_splitkv(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,
                        const b200fa_tensor4* out, float* lse, void* workspace, size_t workspace_bytes, int dtype,
                        int causal, float scale, void* stream, int device, uint32_t* status_word) {
+  return b200fa_fwd_splitkv_piece(q, k, v, out, lse, workspace, workspace_bytes, dtype, causal, scale,
+                                  q ? q->shape[0] * q->shape[1] : 0, stream, device, status_word);
+}
+
+int b200fa_fwd_splitkv_piece(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,
+                             const b200fa_tensor4* out, float* lse, void* workspace, size_t workspace_bytes, int dtype,
+                             int causal, float scale, int64_t whole_heads, void* stream, int device,
+                             uint32_t* status_word) {
   (void)status_word;   // these kernels wait on nothing but __syncthreads
   if (!q || !k || !v || !out || !lse) return B200FA_ERR_NULL;
   if (dtype != kF32 && dtype != kBF16 && dtype != kF16) return B200FA_ERR_BAD_DTYPE;
@@ -528,7 +544,7 @@ int b200fa_fwd_splitkv(const b200fa_tensor4* q, const b200fa_tensor4* k, const b
   if (B <= 0 || Hq <= 0 || Hkv <= 0 || Sq <= 0 || Sk <= 0) return B200FA_ERR_BAD_SHAPE;
   if (B > 65535 || Hq > 65535 || Hkv > 65535 || Sk > (1 << 24)) return B200FA_ERR_BAD_SHAPE;
   if (D != 64 && D != 128) return B200FA_ERR_UNSUPPORTED;
-  if (Hq % Hkv != 0) return B200FA_ERR_BAD_SHAPE;
+  if (Hq % Hkv != 0 || whole_heads < B * Hq) return B200FA_ERR_BAD_SHAPE;
   // all query rows of a GQA group ride in one CTA
   if ((Hq / Hkv) * Sq > B200FA_SPLITKV_MAX_ROWS) return B200FA_ERR_UNSUPPORTED;
   SplitKvParams p;
@@ -541,10 +557,10 @@ int b200fa_fwd_splitkv(const b200fa_tensor4* q, const b200fa_tensor4* k, const b
   if ((rc = check_view(k, B, Hkv, Sk, D, dtype, &p.k)) != B200FA_OK) return rc;
   if ((rc = check_view(v, B, Hkv, Sk, D, dtype, &p.v)) != B200FA_OK) return rc;
   if ((rc = check_view(out, B, Hq, Sq, D, dtype, &p.out, true)) != B200FA_OK) return rc;
-  const size_t need = b200fa_fwd_splitkv_workspace_bytes(B, Hq, Hkv, Sq, Sk, D);
+  const size_t need = b200fa_fwd_splitkv_piece_workspace_bytes(B, Hq, Hkv, Sq, Sk, D, whole_heads);
   if (!workspace || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
     return B200FA_ERR_WORKSPACE;
-  p.nsplit = splitkv_splits(B, Hkv, Hq / Hkv * Sq, Sk, D, dtype == kF32, &p.split_len);
+  p.nsplit = splitkv_splits(whole_heads / (Hq / Hkv), Hq / Hkv * Sq, Sk, D, dtype == kF32, &p.split_len);
   const size_t rows = static_cast<size_t>(B) * Hq * Sq * p.nsplit;
   p.part_o = reinterpret_cast<float*>(workspace);
   p.part_ml = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(rows * D * 4));

@@ -223,18 +223,19 @@ def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is
     out = _alloc_like_layout(q._shape, q._dtype, index, bthd_stored(q_used))
     lse = TorchMojoTensor._alloc((batch, heads_q, seq), torch.float32, index)
     code = _DTYPE_CODES[q._dtype]
+    whole = getattr(_piece, "heads", 0)
+    piece = {"whole_heads": whole} if whole else {}
     if not dropout_p and _decode_shaped(batch, heads_q, heads_kv, seq, seq_k):
-        nbytes = _lib.fwd_splitkv_workspace_bytes(batch, heads_q, heads_kv, seq, seq_k, head_dim)
+        nbytes = _lib.fwd_splitkv_workspace_bytes(batch, heads_q, heads_kv, seq, seq_k, head_dim, **piece)
         workspace = tensor._alloc_holder(nbytes, index)
         _log(f"fwd_splitkv B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={seq_k} D={head_dim}")
         rc = _lib.fwd_splitkv(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, workspace.data_ptr(), nbytes,
-                              code, bool(is_causal), float(scale), _stream_for(index), index, _status_ptr(index))
+                              code, bool(is_causal), float(scale), _stream_for(index), index, _status_ptr(index),
+                              **piece)
         _check(rc, "b200fa_fwd_splitkv")
         CALL_COUNTERS["forward_split_kv"] += 1
         return out, lse, q_used, k_used, v_used
     _log(f"fwd B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={seq_k} D={head_dim} causal={is_causal} p={dropout_p}")
-    whole = getattr(_piece, "heads", 0)
-    piece = {"whole_heads": whole} if whole else {}
     rc = _lib.fwd(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, code, bool(is_causal), float(scale),
                   _stream_for(index), index, _status_ptr(index), dropout=_dropout_arg(dropout_p, philox), **piece)
     _check(rc, "b200fa_fwd")
