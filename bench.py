@@ -209,8 +209,10 @@ def shard_slices(cfg, rank: int, world: int):
     raise ValueError(f"{cfg.name} does not split over {world} ranks")
 
 
-def attention_step(raw, q, k, v, dout, cfg, bufs, status):
-    raw.flash_fwd(q, k, v, causal=cfg.causal, scale=cfg.scale, out=bufs["out"], lse=bufs["lse"], status=status)
+def attention_step(raw, q, k, v, dout, cfg, bufs, status, whole_heads=0):
+    """``whole_heads``: batch * query heads of the problem that q, k, v are a shard of (0: they are the whole)."""
+    raw.flash_fwd(q, k, v, causal=cfg.causal, scale=cfg.scale, out=bufs["out"], lse=bufs["lse"], status=status,
+                  whole_heads=whole_heads)
     if cfg.backward:
         raw.flash_bwd(dout, q, k, v, bufs["out"], bufs["lse"], causal=cfg.causal, scale=cfg.scale, dq=bufs["dq"],
                       dk=bufs["dk"], dv=bufs["dv"], workspace=bufs["ws"], status=status)
@@ -292,9 +294,10 @@ def run_ours(args):
         seed_note = SEED_NOTE_WEAK
     bufs = make_bufs(_lib, raw, q, k, v, cfg)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
+    whole_heads = cfg_full.B * cfg_full.Hq if slices is not None else 0
 
     def step():
-        attention_step(raw, q, k, v, dout, cfg, bufs, status)
+        attention_step(raw, q, k, v, dout, cfg, bufs, status, whole_heads)
 
     warmup = max(args.warmup, 3)
     for _ in range(warmup):
@@ -332,7 +335,7 @@ def run_ours(args):
 
     reps = max(args.steps, 10)
     fwd_ms = time_launches(lambda: raw.flash_fwd(q, k, v, causal=cfg.causal, scale=cfg.scale, out=bufs["out"],
-                                                 lse=bufs["lse"], status=status), reps)
+                                                 lse=bufs["lse"], status=status, whole_heads=whole_heads), reps)
     bwd_part_ms = {}
     if do_bwd:
         for name, part in (("all", 7), ("dkdv", 2), ("dq", 4)):

@@ -219,6 +219,14 @@ int b200fa_fwd_splitkv_piece(const b200fa_tensor4* q, const b200fa_tensor4* k, c
                              int device, uint32_t* status_word);
 
 /*
+ * Thread blocks that share the K/V blocks of a query unit in b200fa_fwd without dropout (1, 2, 4 or 8; 0 if
+ * the arguments are out of range; `whole_heads` as for b200fa_fwd_piece, 0: batch * heads_q): two calls
+ * with the same count, lengths and mask have the same bits row by row.  Host only.
+ */
+int b200fa_fwd_splits(int64_t batch, int64_t heads_q, int64_t seqlen_q, int64_t seqlen_k, int64_t head_dim,
+                      int dtype, int causal, int64_t whole_heads);
+
+/*
  * Same contracts as b200fa_fwd / b200fa_bwd, but always run the exact-fp32 SIMT kernels
  * whatever the storage type (16-bit inputs are widened to fp32 on load).  They exist so the
  * tensor-core kernels can be cross-checked on the device at sizes where a CPU comparison

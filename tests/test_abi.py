@@ -167,6 +167,16 @@ def test_a_piece_of_a_split_kv_call_is_cut_as_the_whole():
                             whole_heads=255) == _lib.ERR_BAD_SHAPE
 
 
+def test_forward_split_count_of_a_piece_is_the_wholes():
+    """One entry of a batch is split to fill the GPU, the batch is not; told the whole, neither is."""
+    n = lambda *a, **kw: _lib.fwd_splits(*a, _lib.BF16, 1, **kw)
+    assert n(8, 4, 1024, 1024, 64) == 1 and n(1, 4, 1024, 1024, 64) > 1
+    assert n(1, 4, 1024, 1024, 64, whole_heads=32) == 1
+    assert _lib.fwd_splits(1, 32, 512, 16896, 128, _lib.BF16, 2) == 2
+    assert _lib.fwd_splits(1, 32, 512, 16896, 128, _lib.F32, 2) == 1
+    assert _lib.fwd_splits(1, 32, 512, 16896, 96, _lib.BF16, 2) == 0 == _lib.fwd_splits(1, 0, 1, 1, 64, _lib.BF16, 0)
+
+
 def test_forward_kernel_shape_setter():
     assert _lib.fwd_tiles() in (0, 1, 2)
     for tiles in (1, 2, 0):

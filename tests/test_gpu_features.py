@@ -96,6 +96,17 @@ def test_a_launch_whose_status_word_is_set_writes_nothing(Hq, Sq, Sk, D, mode):
     assert_within("out", out, O.sdpa_forward(q, k, v, mode, D ** -0.5)[0], TOL_16BIT, torch.bfloat16)
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,mode", [(8, 4, 4, 1024, 1024, 64, 1), (4, 8, 2, 500, 3000, 128, 2),
+                                                  (6, 16, 4, 2, 9000, 128, 2), (9, 2, 2, 1, 5000, 64, 0)])
+def test_a_shard_that_is_told_the_whole_has_its_bits(B, Hq, Hkv, Sq, Sk, D, mode):
+    q, k, v, _ = (t.cuda() for t in draw(torch.float16, B, Hq, Hkv, Sq, Sk, D, 9))
+    forward = raw.flash_fwd_splitkv if Hq // Hkv * Sq <= 16 else raw.flash_fwd
+    out, lse = forward(q, k, v, causal=mode)
+    for hs, ks in ((slice(None), slice(None)), (slice(Hq // 2, Hq), slice(Hkv // 2, Hkv))):   # an entry, half its heads
+        part_out, part_lse = forward(q[1:2, hs], k[1:2, ks], v[1:2, ks], causal=mode, whole_heads=B * Hq)
+        assert torch.equal(part_out, out[1:2, hs]) and torch.equal(part_lse, lse[1:2, hs])
+
+
 ALIGNED = [
     # dtype, B, Hq, Hkv, Sq, Sk, D, mode (1 top-left = torch's is_causal, 2 bottom-right = the reference kernels' rule)
     (torch.bfloat16, 2, 4, 2, 128, 320, 128, 1),

@@ -57,6 +57,21 @@ def test_bench_shard_slices_tile_the_problem_and_agree_with_the_config_shards():
         bench.shard_slices(O.CONFIGS["C3"], 0, 3)
 
 
+def test_a_rank_computes_its_shard_as_a_piece_of_the_whole():
+    sys.path.insert(0, ROOT)
+    import bench
+
+    calls = []
+
+    class Raw:
+        flash_fwd = staticmethod(lambda *a, **kw: calls.append(kw))
+
+    c4 = O.CONFIGS["C4"]
+    bench.attention_step(Raw, 0, 0, 0, 0, c4, {"out": 0, "lse": 0}, 0, c4.B * c4.Hq)
+    bench.attention_step(Raw, 0, 0, 0, 0, c4, {"out": 0, "lse": 0}, 0)
+    assert [kw["whole_heads"] for kw in calls] == [32, 0]
+
+
 def _free_port():
     with socket.socket() as s:
         s.bind(("127.0.0.1", 0))

@@ -35,6 +35,7 @@ ERR_TIMEOUT = -9
 EXPORTED_SYMBOLS = (
     "b200fa_fwd",
     "b200fa_fwd_piece",
+    "b200fa_fwd_splits",
     "b200fa_bwd_workspace_bytes",
     "b200fa_bwd",
     "b200fa_fwd_simt",
@@ -111,6 +112,8 @@ def load() -> ctypes.CDLL:
         fn.restype = ctypes.c_int
     lib.b200fa_fwd_piece.argtypes = fwd_args[:8] + [ctypes.c_int64] + fwd_args[8:]
     lib.b200fa_fwd_piece.restype = ctypes.c_int
+    lib.b200fa_fwd_splits.argtypes = [ctypes.c_int64] * 5 + [ctypes.c_int] * 2 + [ctypes.c_int64]
+    lib.b200fa_fwd_splits.restype = ctypes.c_int
     for name in ("b200fa_bwd", "b200fa_bwd_simt"):
         fn = getattr(lib, name)
         fn.argtypes = bwd_args
@@ -204,6 +207,11 @@ def fwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, dtype: i
         return load().b200fa_fwd_piece(*head, whole_heads, *tail)
     fn = load().b200fa_fwd_simt if simt else load().b200fa_fwd
     return fn(*head, *tail)
+
+
+def fwd_splits(B: int, Hq: int, Sq: int, Sk: int, D: int, dtype: int, causal, whole_heads: int = 0) -> int:
+    """How many thread blocks share a query unit's K/V blocks in `fwd` without dropout (see b200fa_fwd_splits)."""
+    return int(load().b200fa_fwd_splits(B, Hq, Sq, Sk, D, dtype, int(causal), whole_heads))
 
 
 def bwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, dout: Tensor4, lse_ptr: int, dq: Tensor4,

@@ -428,6 +428,21 @@ int b200fa_fwd_piece(const b200fa_tensor4* q, const b200fa_tensor4* k, const b20
   return fwd_impl(q, k, v, out, lse, dtype, causal, scale, stream, device, status_word, opt);
 }
 
+int b200fa_fwd_splits(int64_t batch, int64_t heads_q, int64_t seqlen_q, int64_t seqlen_k, int64_t head_dim, int dtype,
+                      int causal, int64_t whole_heads) {
+  if (batch <= 0 || heads_q <= 0 || seqlen_q <= 0 || seqlen_k <= 0 || (head_dim != 64 && head_dim != 128)) return 0;
+  if (batch > 65535 || heads_q > 65535 || seqlen_q > (1 << 24) || seqlen_k > (1 << 24)) return 0;
+  FwdParams p;
+  std::memset(&p, 0, sizeof(p));
+  if (!causal_mode(causal, seqlen_q, seqlen_k, &p.causal, &p.causal_off)) return 0;
+  if (dtype != kBF16 && dtype != kF16) return dtype == kF32 ? 1 : 0;
+  p.B = static_cast<int>(batch); p.Hq = p.Hkv = static_cast<int>(heads_q);
+  p.Sq = static_cast<int>(seqlen_q); p.Sk = static_cast<int>(seqlen_k); p.D = static_cast<int>(head_dim);
+  p.whole_heads = whole_heads > 0 ? whole_heads : batch * heads_q;
+  p.tiles_per_cta = fwd_tiles();
+  return fwd_splits(p);
+}
+
 int b200fa_fwd_simt(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tensor4* v,
                     const b200fa_tensor4* out, float* lse, int dtype, int causal, float scale, void* stream,
                     int device, uint32_t* status_word) {

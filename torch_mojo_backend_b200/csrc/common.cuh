@@ -74,6 +74,7 @@ constexpr int kF32 = 0, kBF16 = 1, kF16 = 2;
 // Launchers implemented in the kernel translation units.  Each returns a cudaError_t and
 // adds the number of kernels it enqueued to *launches.
 cudaError_t launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream, int* launches);
+int fwd_splits(const FwdParams& p);   // CTAs that share a query unit's K/V blocks in launch_fwd_sm100 (host only)
 cudaError_t launch_fwd_simt(const FwdParams& p, int dtype, cudaStream_t stream, int* launches);
 cudaError_t launch_fwd_splitkv(const SplitKvParams& p, int dtype, cudaStream_t stream, int* launches);
 cudaError_t launch_bwd_sm100(const BwdParams& p, int dtype, cudaStream_t stream, int* launches);

@@ -737,6 +737,7 @@ cudaError_t launch_tiles(const CUtensorMap& mq, const CUtensorMap& mk, const CUt
 //   Hq8 Sq32 Sk4096 (8)                   53 / 33 / 23 / [16]       Hq8 S4096 causal (128)     62 / [51] / 78 / 135
 //   B4 Hq16 S300 unmasked (128)           [14] / 29 / 48 / 100      D=64 B2 Hq16 Sq256 Sk8192  86 / 49 / [38] / 45
 int choose_splits(const FwdParams& p, const FwdSched& sched) {
+  if (p.drop.threshold != 0 || p.tiles_per_cta != 0) return 1;   // (no split form with dropout, nor of a forced shape)
   const int rows = (sched.one_tile ? 1 : 2) * kBM;
   const int per_sm = sched.one_tile ? 2 : 1;
   // SMs that clusters of 1, 2, 4 and 8 CTAs of one per SM can fill: they do not cross a GPC (measured: the
@@ -774,10 +775,8 @@ int choose_splits(const FwdParams& p, const FwdSched& sched) {
 
 template <int kD, bool kBf16, bool kCausal, bool kDropout>
 cudaError_t launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                       const FwdParams& p, FwdSched sched, cudaStream_t stream) {
-  if (sched.one_tile) sched.npairs = (p.Sq + kBM - 1) / kBM;
+                       const FwdParams& p, const FwdSched& sched, cudaStream_t stream) {
   if constexpr (!kDropout) {
-    sched.splits = p.tiles_per_cta != 0 ? 1 : choose_splits(p, sched);
     constexpr int kTilesChosen = kD == 64 ? 1 : 2;   // what choose_one_tile says unless it is overridden
     if (sched.splits > 1) return launch_tiles<kD, kBf16, kCausal, false, kTilesChosen, true>(mq, mk, mv, mo, p, sched, stream);
   }
@@ -809,17 +808,11 @@ cudaError_t launch_mask(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
               : launch_one<kD, kBf16, false, false>(mq, mk, mv, mo, p, sched, stream);
 }
 
-}  // namespace
-
-cudaError_t launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream, int* launches) {
-  const bool bf16 = (dtype == kBF16);
-  CUtensorMap mq, mk, mv, mo;
-  if (!encode_map_16bit(&mq, p.q, p.B, p.Hq, p.Sq, p.D, kBM, bf16)) return cudaErrorInvalidValue;
-  if (!encode_map_16bit(&mk, p.k, p.B, p.Hkv, p.Sk, p.D, kBN, bf16)) return cudaErrorInvalidValue;
-  if (!encode_map_16bit(&mv, p.v, p.B, p.Hkv, p.Sk, p.D, kBN, bf16)) return cudaErrorInvalidValue;
-  if (!encode_map_16bit(&mo, p.out, p.B, p.Hq, p.Sq, p.D, kBM, bf16)) return cudaErrorInvalidValue;
+FwdSched schedule(const FwdParams& p) {
   FwdSched sched;
-  sched.npairs = (p.Sq + 2 * kBM - 1) / (2 * kBM);
+  sched.one_tile = choose_one_tile(p, p.tiles_per_cta);
+  const int rows = (sched.one_tile ? 1 : 2) * kBM;
+  sched.npairs = (p.Sq + rows - 1) / rows;
   sched.nkv_total = (p.Sk + kBN - 1) / kBN;
   // keep roughly 32 MiB of K/V hot in L2: that many heads are walked together
   const int64_t kv_bytes_per_head = static_cast<int64_t>(p.Sk) * p.D * 2 * 2;
@@ -828,8 +821,22 @@ cudaError_t launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream,
   if (group < 1) group = 1;
   if (group > total_bh) group = total_bh;
   sched.group = static_cast<int>(group);
-  sched.one_tile = choose_one_tile(p, p.tiles_per_cta);
-  sched.splits = 1;
+  sched.splits = choose_splits(p, sched);
+  return sched;
+}
+
+}  // namespace
+
+int fwd_splits(const FwdParams& p) { return schedule(p).splits; }
+
+cudaError_t launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream, int* launches) {
+  const bool bf16 = (dtype == kBF16);
+  CUtensorMap mq, mk, mv, mo;
+  if (!encode_map_16bit(&mq, p.q, p.B, p.Hq, p.Sq, p.D, kBM, bf16)) return cudaErrorInvalidValue;
+  if (!encode_map_16bit(&mk, p.k, p.B, p.Hkv, p.Sk, p.D, kBN, bf16)) return cudaErrorInvalidValue;
+  if (!encode_map_16bit(&mv, p.v, p.B, p.Hkv, p.Sk, p.D, kBN, bf16)) return cudaErrorInvalidValue;
+  if (!encode_map_16bit(&mo, p.out, p.B, p.Hq, p.Sq, p.D, kBM, bf16)) return cudaErrorInvalidValue;
+  const FwdSched sched = schedule(p);
   cudaError_t e;
   if (p.D == 128) {
     e = bf16 ? launch_mask<128, true>(mq, mk, mv, mo, p, sched, stream)

@@ -39,13 +39,15 @@ def default_scale(head_dim: int) -> float:
 
 
 def flash_fwd(q, k, v, *, causal, scale: float | None = None, out=None, lse=None, status=None,
-              simt: bool = False, dropout=None):
+              simt: bool = False, dropout=None, whole_heads: int = 0):
     """out, lse = attention forward on CUDA tensors shaped (B, H, S, D).
 
     ``out`` defaults to a new contiguous (B, Hq, Sq, D) tensor; pass a pre-allocated (possibly
     strided) tensor to choose the storage layout.  ``lse`` is fp32 (B, Hq, Sq).  ``causal`` is a
     bool (True: diagonal from the top-left corner) or one of ``_lib.CAUSAL_*``; ``dropout`` is
-    None or ``(p, philox_seed, philox_offset)``.
+    None or ``(p, philox_seed, philox_offset)``.  A call that computes a piece of a larger problem
+    (some batch entries or whole groups of heads, one rank's shard) has the bits of one call over the
+    whole if it is told the whole's batch * query heads in ``whole_heads``.
     """
     if q.device.type != "cuda":
         raise RuntimeError("b200fa kernels need CUDA memory; there is no CPU implementation")
@@ -58,15 +60,17 @@ def flash_fwd(q, k, v, *, causal, scale: float | None = None, out=None, lse=None
         lse = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device)
     stream, dev = _stream_and_device(q)
     rc = _lib.fwd(t4(q), t4(k), t4(v), t4(out), lse.data_ptr(), dtype_code(q.dtype), causal, float(scale),
-                  stream, dev, status.data_ptr() if status is not None else 0, simt=simt, dropout=dropout)
+                  stream, dev, status.data_ptr() if status is not None else 0, simt=simt, dropout=dropout,
+                  whole_heads=whole_heads)
     if rc != _lib.OK:
         raise _lib.B200FAError(rc, "b200fa_fwd")
     return out, lse
 
 
-def flash_fwd_splitkv(q, k, v, *, causal, scale: float | None = None, out=None, lse=None, workspace=None):
+def flash_fwd_splitkv(q, k, v, *, causal, scale: float | None = None, out=None, lse=None, workspace=None,
+                      whole_heads: int = 0):
     """out, lse = the split-KV (decode) forward on CUDA tensors shaped (B, H, S, D); needs
-    ``(Hq / Hkv) * Sq <= 16``."""
+    ``(Hq / Hkv) * Sq <= 16``.  ``whole_heads`` as for ``flash_fwd``."""
     if q.device.type != "cuda":
         raise RuntimeError("b200fa kernels need CUDA memory; there is no CPU implementation")
     B, Hq, Sq, D = q.shape
@@ -77,13 +81,13 @@ def flash_fwd_splitkv(q, k, v, *, causal, scale: float | None = None, out=None, 
         out = torch.empty((B, Hq, Sq, D), dtype=q.dtype, device=q.device)
     if lse is None:
         lse = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device)
-    need = _lib.fwd_splitkv_workspace_bytes(B, Hq, Hkv, Sq, Sk, D)
+    need = _lib.fwd_splitkv_workspace_bytes(B, Hq, Hkv, Sq, Sk, D, whole_heads)
     if workspace is None:
         workspace = torch.empty((need,), dtype=torch.uint8, device=q.device)
     stream, dev = _stream_and_device(q)
     rc = _lib.fwd_splitkv(t4(q), t4(k), t4(v), t4(out), lse.data_ptr(), workspace.data_ptr(),
                           workspace.numel() * workspace.element_size(), dtype_code(q.dtype), causal, float(scale),
-                          stream, dev)
+                          stream, dev, whole_heads=whole_heads)
     if rc != _lib.OK:
         raise _lib.B200FAError(rc, "b200fa_fwd_splitkv")
     return out, lse
