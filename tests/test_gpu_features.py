@@ -107,6 +107,26 @@ def test_a_shard_that_is_told_the_whole_has_its_bits(B, Hq, Hkv, Sq, Sk, D, mode
         assert torch.equal(part_out, out[1:2, hs]) and torch.equal(part_lse, lse[1:2, hs])
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_an_infinity_behind_a_vanished_probability_spreads_split_or_not(D):
+    """Zero times infinity is NaN (as in the softmax written out), also where the keys whose probabilities
+    vanish are a thread block's whole share."""
+    q = torch.ones(1, 2, 256, D, dtype=torch.float16, device="cuda")
+    k, v = torch.full((1, 2, 4096, D), 4.0, dtype=torch.float16, device="cuda"), torch.ones_like(q[:, :, :1]).repeat(1, 1, 4096, 1)
+    k[:, :, 2000:] = -12.0      # 16 sqrt(D) lower: 2^-184 at D = 64
+    v[0, 1, 4000, 5] = float("inf")
+    assert _lib.fwd_splits(1, 2, 256, 4096, D, _lib.F16, 0) > 1
+    out, lse = raw.flash_fwd(q, k, v, causal=0)
+    _lib.set_fwd_tiles(1 if D == 64 else 2)     # a forced shape is never split
+    try:
+        whole, whole_lse = raw.flash_fwd(q, k, v, causal=0)
+    finally:
+        _lib.set_fwd_tiles(0)
+    assert bool(whole[0, 1, :, 5].isnan().all()) and int(whole.isnan().sum()) == 256
+    assert torch.equal(out.isnan(), whole.isnan()) and torch.equal(out.nan_to_num(), whole.nan_to_num())
+    assert torch.allclose(lse, whole_lse, atol=1e-5)
+
+
 ALIGNED = [
     # dtype, B, Hq, Hkv, Sq, Sk, D, mode (1 top-left = torch's is_causal, 2 bottom-right = the reference kernels' rule)
     (torch.bfloat16, 2, 4, 2, 128, 320, 128, 1),

@@ -91,7 +91,7 @@ __device__ __forceinline__ void merge_split(const FwdParams& p, const uint8_t* s
 #pragma unroll
   for (int r = 0; r < kPeers; ++r) aborted |= peer_load_u32(smem_u32(const_cast<const uint32_t*>(abort_flag)), r);
   if (aborted) return;
-  float* weights = reinterpret_cast<float*>(s_w);  // [row][peer]: what the peer's O is multiplied by
+  float* weights = reinterpret_cast<float*>(s_w);  // [row][peer]: what the peer's O is multiplied by; -0: it has none
   if (tid < kShare) {
     const int lr = rank * kShare + tid;   // row of the unit
     const uint32_t al = smem_u32(s_l + lr), am = smem_u32(s_m + lr);
@@ -105,14 +105,16 @@ __device__ __forceinline__ void merge_split(const FwdParams& p, const uint8_t* s
     for (int r = 0; r < kPeers; ++r) {
       if (l[r] != 0.f) top = fmaxf(top, m[r]);
     }
+    uint32_t wrote = 0;
 #pragma unroll
     for (int r = 0; r < kPeers; ++r) {
+      wrote |= (m[r] != -INFINITY ? 1u : 0u) << r;
       m[r] = l[r] != 0.f ? ex2_approx((m[r] - top) * p.scale_log2) : 0.f;   // (nothing to add from a peer that saw no key of this row)
       sum = fmaf(l[r], m[r], sum);
     }
     const float inv = sum == 0.f ? 0.f : 1.f / sum;   // (a NaN stays one)
 #pragma unroll
-    for (int r = 0; r < kPeers; ++r) weights[tid * kPeers + r] = l[r] != 0.f ? m[r] * inv : 0.f;
+    for (int r = 0; r < kPeers; ++r) weights[tid * kPeers + r] = (wrote >> r) & 1u ? m[r] * inv : -0.f;
     if (row0 + lr < p.Sq) {
       p.lse[(static_cast<int64_t>(b) * p.Hq + h) * p.Sq + row0 + lr] = sum > 0.f ? top * p.scale + logf(sum) : -INFINITY;
     }
@@ -140,8 +142,10 @@ __device__ __forceinline__ void merge_split(const FwdParams& p, const uint8_t* s
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int r = 0; r < kPeers; ++r) {
+        // a peer without a block of this row's tile has not written its O; one whose weight is zero
+        // adds its zeros (and its infinities, as the kernel without peers does)
         const float w = weights[i * kPeers + r];
-        if (w != 0.f) {   // a peer without a block of this row's tile has not written its O
+        if (__float_as_uint(w) != 0x80000000u) {
           acc.x = fmaf(o[u][r].x, w, acc.x);
           acc.y = fmaf(o[u][r].y, w, acc.y);
           acc.z = fmaf(o[u][r].z, w, acc.z);
