@@ -210,18 +210,6 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       const int m_tile = m_start + i % per_head;
       const float4* lse2 = reinterpret_cast<const float4*>(sStat + stage * 256 + wg * 32);
       const float4* dps = lse2 + 32;
-      // dropout: bit e of `keep` <-> query column e of these 32.  Lane L draws the bits of query
-      // row L against this warp's 32 key rows (two Philox calls), and the warp transposes them.
-      // Drawn here, it runs while S^T is on its way.
-      uint32_t keep = 0xffffffffu;
-      if constexpr (kDropout) {
-        const int h_now = hk * group + i / per_head;
-        const int q_glob = m_tile * kTile + wg * 32 + lane;
-        const int blk = (n0 + (warp & 3) * 32) >> 4;
-        const uint32_t mine = dropout_bits16(p.drop, b * p.Hq + h_now, q_glob, blk) |
-                              (dropout_bits16(p.drop, b * p.Hq + h_now, q_glob, blk + 1) << 16);
-        keep = warp_transpose_bits(mine);
-      }
       // ---- P^T = exp2(S^T * c - lse2).  S^T is pulled into registers in one go and released
       // at once, so the S^T MMA of the next step can run while the exponentials do;
       // P^T goes to shared memory (the A operand of dV += P^T dO) instead of back over S^T.
@@ -255,6 +243,17 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         for (int e = 0; e < 32; ++e) {
           if (e < first_q) pf[e] = 0.f;
         }
+      }
+      // dropout: bit e of `keep` <-> query column e of these 32.  Lane L draws the bits of query
+      // row L against this warp's 32 key rows (two Philox calls), and the warp transposes them.
+      uint32_t keep = 0xffffffffu;
+      if constexpr (kDropout) {
+        const int h_now = hk * group + i / per_head;
+        const int q_glob = m_tile * kTile + wg * 32 + lane;
+        const int blk = (n0 + (warp & 3) * 32) >> 4;
+        const uint32_t mine = dropout_bits16(p.drop, b * p.Hq + h_now, q_glob, blk) |
+                              (dropout_bits16(p.drop, b * p.Hq + h_now, q_glob, blk + 1) << 16);
+        keep = warp_transpose_bits(mine);
       }
       // the previous step's dV MMA must have finished reading the P^T tile
       if (i > 0) { B200FA_WAIT(p_empty, (i - 1) & 1, 0x502); }
@@ -600,16 +599,6 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
     for (int j = 0; j < n_tiles; ++j) {
       const int buf = j & 1;
       const uint32_t tS = tmem_base + lane_off + kTmemS + buf * 128 + wg * 64;
-      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};   // dropout: bit e of keep[ch] <-> key column ch*32 + e of this half
-      if constexpr (kDropout) {
-        const int blk = (j * kTile + wg * 64) >> 4;
-        const int bh = b * p.Hq + h;
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-          keep[ch] = dropout_bits16(p.drop, bh, m0 + r, blk + 2 * ch) |
-                     (dropout_bits16(p.drop, bh, m0 + r, blk + 2 * ch + 1) << 16);
-        }
-      }
       B200FA_WAIT(&s_full[buf], (j >> 1) & 1, 0x900);
       tc_fence_after();
       float pf[64];
@@ -640,6 +629,16 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
           for (int e = 0; e < 32; ++e) {
             if (e > last_e) pf[ch * 32 + e] = 0.f;
           }
+        }
+      }
+      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};   // dropout: bit e of keep[ch] <-> key column ch*32 + e of this half
+      if constexpr (kDropout) {
+        const int blk = (j * kTile + wg * 64) >> 4;
+        const int bh = b * p.Hq + h;
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+          keep[ch] = dropout_bits16(p.drop, bh, m0 + r, blk + 2 * ch) |
+                     (dropout_bits16(p.drop, bh, m0 + r, blk + 2 * ch + 1) << 16);
         }
       }
       B200FA_WAIT(dp_full, j & 1, 0x910);
