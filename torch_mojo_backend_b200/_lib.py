@@ -198,7 +198,8 @@ def fwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, dtype: i
     """Raw forward call; returns the library's status code.  `causal` is a bool or one of
     CAUSAL_*; `dropout` is None or ``(p, seed, offset)``; `whole_heads`, if not 0, is batch * query
     heads of the problem this call computes a piece of (see b200fa_fwd_piece)."""
-    head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), lse_ptr, dtype, int(causal), scale)
+    head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), lse_ptr, dtype, causal_code(causal),
+            scale)
     tail = (stream, device, status_ptr)
     if dropout is not None:
         p, seed, offset = dropout
@@ -211,7 +212,7 @@ def fwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, dtype: i
 
 def fwd_splits(B: int, Hq: int, Sq: int, Sk: int, D: int, dtype: int, causal, whole_heads: int = 0) -> int:
     """How many thread blocks share a query unit's K/V blocks in `fwd` without dropout (see b200fa_fwd_splits)."""
-    return int(load().b200fa_fwd_splits(B, Hq, Sq, Sk, D, dtype, int(causal), whole_heads))
+    return int(load().b200fa_fwd_splits(B, Hq, Sq, Sk, D, dtype, causal_code(causal), whole_heads))
 
 
 def bwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, dout: Tensor4, lse_ptr: int, dq: Tensor4,
@@ -223,7 +224,7 @@ def bwd(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, dout: Tensor4, lse_ptr
     and must repeat the forward's."""
     head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), ctypes.byref(dout),
             lse_ptr, ctypes.byref(dq), ctypes.byref(dk), ctypes.byref(dv), workspace_ptr, workspace_bytes, dtype,
-            int(causal), scale)
+            causal_code(causal), scale)
     tail = (stream, device, status_ptr)
     if dropout is not None:
         p, seed, offset = dropout
@@ -246,7 +247,7 @@ def fwd_splitkv(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, 
     """Raw split-KV (decode) forward; returns the library's status code.  `whole_heads` as for `fwd`
     (the workspace is then that of the piece)."""
     head = (ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), lse_ptr, workspace_ptr,
-            workspace_bytes, dtype, int(causal), scale)
+            workspace_bytes, dtype, causal_code(causal), scale)
     tail = (stream, device, status_ptr)
     if whole_heads:
         return load().b200fa_fwd_splitkv_piece(*head, whole_heads, *tail)
@@ -254,7 +255,7 @@ def fwd_splitkv(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, lse_ptr: int, 
 
 
 def dropout_threshold(p: float) -> int:
-    return int(load().b200fa_dropout_threshold(ctypes.c_float(p)))
+    return int(load().b200fa_dropout_threshold(p))
 
 
 def dropout_bytes_host(seed: int, offset: int, batch_head: int, row: int, col_block: int) -> bytes:
@@ -286,8 +287,7 @@ def status_to_error(status_value: int) -> int:
 
 
 def selftest_wait_timeout(status_ptr: int, budget_cycles: int, stream: int, device: int) -> int:
-    return load().b200fa_selftest_wait_timeout(ctypes.c_void_p(status_ptr), int(budget_cycles),
-                                               ctypes.c_void_p(stream), device)
+    return load().b200fa_selftest_wait_timeout(status_ptr, int(budget_cycles), stream, device)
 
 
 def no_alloc_scratch_bytes() -> int:
@@ -301,6 +301,6 @@ def bwd_no_alloc(q: Tensor4, k: Tensor4, v: Tensor4, out: Tensor4, dout: Tensor4
     array (see b200fa_bwd_no_alloc in include/b200fa.h).  The caller passes every input and
     output; this wrapper allocates nothing either.  Returns the library's status code."""
     return load().b200fa_bwd_no_alloc(
-        ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), ctypes.byref(dout),
-        ctypes.c_void_p(lse_ptr), ctypes.byref(dq), ctypes.byref(dk), ctypes.byref(dv), dtype, causal_code(causal),
-        ctypes.c_float(scale), ctypes.c_void_p(stream), device, ctypes.c_void_p(status_ptr))
+        ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(out), ctypes.byref(dout), lse_ptr,
+        ctypes.byref(dq), ctypes.byref(dk), ctypes.byref(dv), dtype, causal_code(causal), scale, stream, device,
+        status_ptr)

@@ -54,14 +54,6 @@ __host__ __device__ __forceinline__ void dropout_bytes16(const DropoutParams& d,
                 static_cast<uint32_t>(hi >> 32), out);
 }
 
-// One element (slow: a whole Philox call; the exact-fp32 SIMT kernels use it).
-__host__ __device__ __forceinline__ bool dropout_keep(const DropoutParams& d, int bh, int row, int col) {
-  uint32_t r[4];
-  dropout_bytes16(d, bh, row, col >> 4, r);
-  const uint32_t byte = (r[(col >> 2) & 3] >> ((col & 3) * 8)) & 0xffu;
-  return byte >= d.threshold;
-}
-
 #ifdef __CUDACC__
 // keep-bits of 16 consecutive columns (bit i <-> column 16*col_block + i)
 __device__ __forceinline__ uint32_t dropout_bits16(const DropoutParams& d, int bh, int row, int col_block) {
