@@ -147,6 +147,8 @@ def test_split_count_fills_whole_waves_of_the_grid():
     # more than eight rows per KV head: two thread blocks per SM
     n16 = _splits_of(1, 32, 2, 1, 131072, 128)
     assert 2 * n16 <= 296
+    # many short caches of narrow keys: another split would only add a part-filled wave
+    assert _splits_of(28, 24, 8, 4, 1208, 64) == 1
     # a split is never shorter than 256 keys (but for the last one)
     assert _splits_of(1, 8, 8, 1, 600, 64) <= 3 and _splits_of(2, 4, 4, 1, 200, 64) == 1
 
