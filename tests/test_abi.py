@@ -179,6 +179,11 @@ def test_forward_split_count_of_a_piece_is_the_wholes():
     assert _lib.fwd_splits(1, 32, 512, 16896, 96, _lib.BF16, 2) == 0 == _lib.fwd_splits(1, 0, 1, 1, 64, _lib.BF16, 0)
 
 
+def test_short_forwards_that_a_split_would_slow_down_are_not_split():
+    assert _lib.fwd_splits(1, 2, 394, 394, 128, _lib.BF16, 1) == 1
+    assert _lib.fwd_splits(1, 32, 168, 542, 128, _lib.F16, 2) == 1
+
+
 def test_forward_kernel_shape_setter():
     assert _lib.fwd_tiles() in (0, 1, 2)
     for tiles in (1, 2, 0):

@@ -736,7 +736,10 @@ cudaError_t launch_tiles(const CUtensorMap& mq, const CUtensorMap& mk, const CUt
 // K/V block of work: a CTA costs its blocks, a fixed part (set-up, first loads, epilogue) and, with
 // peers, the exchange and merge of the accumulators; the grid then takes no less than its longest
 // CTA, its total over the resident CTAs, and the waves that the longest so many CTAs need.  A split
-// has to promise 5 %.  Measured (us, B200, D = 128 bf16, 1 / 2 / 4 / 8 CTAs per unit, the choice in brackets):
+// has to promise 10 %: of 190 random calls small enough to be split none is then slower than unsplit, and
+// they take 1.1 % more time than with each one's best count (at 5 %: Hq2 S394 causal 14.4 us for 13.1, Hq32
+// Sq168 Sk542 17.7 for 16.5).  Measured (us, B200, D = 128 bf16, 1 / 2 / 4 / 8 CTAs per unit, the choice in
+// brackets):
 //   Hq32 Sq512 Sk16896 causal (64 units)  224 / [141] / 144 / 205   Hq16 Sq1024 Sk9000 (64)    125 / [78] / 89 / 135
 //   Hq8 Sq32 Sk4096 (8)                   53 / 33 / 23 / [16]       Hq8 S4096 causal (128)     62 / [51] / 78 / 135
 //   B4 Hq16 S300 unmasked (128)           [14] / 29 / 48 / 100      D=64 B2 Hq16 Sq256 Sk8192  86 / 49 / [38] / 45
@@ -747,7 +750,7 @@ int choose_splits(const FwdParams& p, const FwdSched& sched) {
   // SMs that clusters of 1, 2, 4 and 8 CTAs of one per SM can fill: they do not cross a GPC (measured: the
   // 34th cluster of 4 and the 16th of 8 wait for a second wave)
   constexpr int kSMs[4] = {148, 148, 132, 120};
-  const double fixed = p.D == 64 ? 5.0 : 3.0;   // in K/V blocks; the merge costs about as much again
+  const double fixed = p.D == 64 ? 4.0 : 3.0;   // in K/V blocks; the merge costs about as much again
   const int64_t heads = p.whole_heads;   // a piece of a problem is split as the whole is: the same bits
   if (heads > kSMs[0] * per_sm || heads * sched.npairs > kSMs[0] * per_sm) return 1;
   int best = 1;
@@ -769,7 +772,7 @@ int choose_splits(const FwdParams& p, const FwdSched& sched) {
       cost = std::max(cost, static_cast<double>((ctas + slots - 1) / slots) * one);
     }
     cost = std::max(cost, total / slots);
-    if (c == 1 || cost < 0.95 * best_cost) {
+    if (c == 1 || cost < 0.9 * best_cost) {
       best = c;
       best_cost = cost;
     }
