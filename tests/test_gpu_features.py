@@ -46,8 +46,9 @@ def t64(x):
     return x.float().numpy().astype(np.float64)
 
 
-# Forward calls with few (batch, head, query tile) units, whose K/V blocks are dealt to the CTAs of a
-# cluster: unequal shares, shares without a block, rows without a key, one key, ragged edges.
+# Forward calls with few (batch, head, query tile) units.  The K/V blocks of the first three, the fifth and
+# the sixth are dealt to the CTAs of clusters (unequal shares, shares without a block, ragged edges); the
+# others are too short for that.
 SPLIT = [
     # dtype, B, Hq, Hkv, Sq, Sk, D, mode
     (torch.bfloat16, 1, 2, 1, 256, 4224, 128, 2),
@@ -76,6 +77,35 @@ def test_forward_split_over_clusters(dtype, B, Hq, Hkv, Sq, Sk, D, mode):
     seen = sees.expand(B, Hq, Sq)
     assert torch.equal(seen, torch.isfinite(lse.cpu()))
     assert (lse.cpu() - ref_lse)[seen].abs().max().item() < TOL_LSE
+
+
+# every cluster size at both head dimensions, rows without a key among them
+SPLIT_COUNTS = [
+    # dtype, B, Hq, Hkv, Sq, Sk, D, mode, CTAs per query unit
+    (torch.bfloat16, 1, 8, 8, 1584, 1982, 128, 0, 2),
+    (torch.float16, 1, 6, 3, 1300, 1200, 128, 2, 2),
+    (torch.float16, 1, 10, 5, 1111, 1500, 64, 0, 2),
+    (torch.bfloat16, 1, 8, 8, 1472, 1662, 64, 2, 2),
+    (torch.bfloat16, 1, 4, 4, 1537, 1000, 128, 2, 4),
+    (torch.float16, 1, 2, 1, 2600, 2300, 64, 2, 4),
+    (torch.float16, 1, 2, 2, 1500, 1300, 128, 2, 8),
+    (torch.bfloat16, 1, 1, 1, 2600, 2300, 64, 2, 8),
+]
+
+
+@pytest.mark.parametrize("dtype,B,Hq,Hkv,Sq,Sk,D,mode,splits", SPLIT_COUNTS)
+def test_forward_split_over_each_cluster_size(dtype, B, Hq, Hkv, Sq, Sk, D, mode, splits):
+    assert _lib.fwd_splits(B, Hq, Sq, Sk, D, _lib.BF16, mode) == splits
+    q, k, v, _ = draw(dtype, B, Hq, Hkv, Sq, Sk, D, Sq + Sk)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, lse = raw.flash_fwd(q.cuda(), k.cuda(), v.cuda(), causal=mode, scale=D ** -0.5, status=status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    ref_out, ref_lse = O.sdpa_forward(q, k, v, mode, D ** -0.5)
+    keyless = max(0, Sq - Sk) if mode == 2 else 0     # these rows are 0 with lse -inf
+    assert not bool(out[:, :, :keyless].any()) and bool((lse[:, :, :keyless] == -float("inf")).all())
+    assert_within("out", out[:, :, keyless:], ref_out[:, :, keyless:], TOL_16BIT, dtype)
+    assert (lse.cpu() - ref_lse)[:, :, keyless:].abs().max().item() < TOL_LSE
 
 
 @pytest.mark.parametrize("Hq,Sq,Sk,D,mode", [(1, 256, 4096, 128, 2), (2, 300, 3000, 64, 0), (64, 1024, 1024, 128, 1)])

@@ -1,5 +1,5 @@
 """The exact-fp32 kernels at the edges of their tiles, on the GPU: rows and columns around 32, 64 and
-128, both block shapes (few blocks take the short one, many the tall one), grouped heads, both causal
+128, both block shapes (problems of fewer than TALL_BLOCKS 64-row blocks take the short one), grouped heads, both causal
 alignments, dropout, and views of a fused projection, against the same attention in float64."""
 
 import numpy as np
@@ -11,6 +11,8 @@ from torch_mojo_backend_b200 import raw
 
 pytestmark = pytest.mark.gpu
 
+TALL_BLOCKS = 3 * 148
+
 CASES = [
     # B, Hq, Hkv, Sq, Sk, D, causal mode, dropout
     (1, 2, 2, 1, 2, 64, 0, 0.0),           # (over a single key dQ and dK are exactly zero: no relative error)
@@ -21,9 +23,22 @@ CASES = [
     (1, 2, 2, 130, 70, 128, 0, 0.5),
     (19, 8, 8, 130, 129, 64, 1, 0.0),      # 456 tall blocks each way
     (19, 8, 4, 193, 321, 64, 2, 0.2),
-    (25, 6, 6, 65, 66, 128, 1, 0.0),       # 300 tall blocks
+    (25, 6, 6, 65, 66, 128, 1, 0.0),
     (13, 12, 6, 60, 130, 128, 0, 0.3),
 ]
+# the tall shape in all three kernels
+TALL = [
+    (38, 6, 6, 65, 66, 128, 1, 0.0),
+    (20, 12, 6, 130, 200, 128, 2, 0.3),
+    (19, 12, 12, 128, 65, 128, 2, 0.0),    # the first query rows see no key
+    (38, 12, 6, 65, 66, 64, 0, 0.1),
+]
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,mode,p", TALL)
+def test_fp32_tall_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p):
+    assert min(B * Hq * -(-Sq // 64), B * Hkv * -(-Sk // 64)) >= TALL_BLOCKS
+    test_fp32_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p)
 
 
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,mode,p", CASES)
