@@ -257,7 +257,7 @@ int b200fa_bwd_parts(const b200fa_tensor4* q, const b200fa_tensor4* k, const b20
  * Bounded waits.  Every wait inside the tensor-core kernels gives up after a budget of SM
  * cycles (default about 2 s; environment variable B200FA_WAIT_BUDGET, or this setter; 0 restores
  * the default), writes 0x5741xxxx (xxxx = where it gave up) to the status word and lets the
- * kernel finish; later thread blocks that see a non-zero status word leave at once.
+ * kernel finish; later thread blocks that see a non-zero status word do no work and write nothing.
  * b200fa_status_to_error maps a status word read back from the device to B200FA_OK or
  * B200FA_ERR_TIMEOUT.  b200fa_selftest_wait_timeout launches a one-warp kernel whose only job
  * is to wait `budget_cycles` on a barrier nobody arrives at, so the give-up path can be tested
@@ -272,8 +272,9 @@ int b200fa_selftest_wait_timeout(uint32_t* status_word, long long budget_cycles,
  * Shape of the tensor-core forward kernel: 2 = one thread block per SM with two 128-row query
  * tiles, 1 = two thread blocks per SM with one query tile each, 0 = chosen per problem (one tile
  * at head dimension 64, two at 128; the default; environment variable B200FA_FWD_TILES).  Both
- * shapes compute the same values; the setter exists for tests and measurements.  No counterpart
- * in the reference.
+ * forced shapes compute the same values; a small problem whose shape is not forced may be split over
+ * clusters (b200fa_fwd_splits) and round differently.  The setter exists for tests and measurements.
+ * No counterpart in the reference.
  */
 void b200fa_set_fwd_tiles(int tiles);
 int b200fa_fwd_tiles(void);

@@ -8,7 +8,7 @@ through the two flash operators the `mojo` device registers
 (``aten::_scaled_dot_product_flash_attention`` and its ``_backward``) with uploads, kernels and
 downloads on three CUDA streams, so both PCIe directions and the GPU work at the same time.
 Results are bitwise those of a single call over the whole batch: the pieces go through the
-same kernels, and nothing is summed across pieces.
+same kernels, split as the whole would be, and nothing is summed across pieces.
 
 The reference has no counterpart (its benchmarks time device-resident tensors,
 benchmarks/test_attention.py:36-47); this is the host-buffer entry point of this package.
