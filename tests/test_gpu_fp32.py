@@ -1,4 +1,4 @@
-"""The exact-fp32 kernels at the edges of their tiles, on the GPU: rows and columns around 32, 64 and
+"""The fp32 kernels at the edges of their tiles, on the GPU: rows and columns around 32, 64 and
 128, both block shapes (problems of fewer than TALL_BLOCKS 64-row blocks take the short one), grouped heads, both causal
 alignments, dropout, and views of a fused projection, against the same attention in float64."""
 
@@ -90,3 +90,72 @@ def reference(q, k, v, do, mode, scale, keep, inv):
     fold = lambda x: x.reshape(B, Hkv, Hq // Hkv, Sk, D).sum(2)
     return {"out": out, "lse": lse, "dq": ds @ kk * scale, "dk": fold(np.swapaxes(ds, -1, -2) @ q * scale),
             "dv": fold(np.swapaxes(pd, -1, -2) @ do)}
+
+
+# keys of more than 96: the tensor-core forward; D = 64: the tensor-core backward at any length
+SPLIT = [
+    # B, Hq, Hkv, Sq, Sk, D, causal mode, dropout
+    (1, 2, 2, 1, 97, 64, 0, 0.0),
+    (1, 2, 1, 127, 129, 64, 2, 0.0),
+    (2, 4, 2, 129, 191, 64, 0, 0.3),
+    (1, 6, 2, 300, 193, 64, 2, 0.0),       # the first query rows see no key
+    (1, 3, 3, 257, 257, 64, 1, 0.2),
+    (3, 2, 2, 64, 640, 64, 1, 0.0),        # more key tiles than ring slots, and keys that nobody sees
+    (1, 2, 2, 1, 2, 64, 0, 0.0),
+    (1, 2, 1, 128, 129, 128, 2, 0.0),
+    (2, 4, 4, 65, 320, 128, 0, 0.25),
+    (1, 2, 2, 193, 193, 128, 1, 0.0),
+]
+
+
+def errors(B, Hq, Hkv, Sq, Sk, D, mode, p, simt):
+    g = torch.Generator().manual_seed(Sq * 1000 + Sk)
+    q, k, v, dout = (torch.randn(B, h, s, D, generator=g) for h, s in ((Hq, Sq), (Hkv, Sk), (Hkv, Sk), (Hq, Sq)))
+    dropout = (p, 11, 5) if p else None
+    qc, kc, vc = q.cuda(), k.cuda(), v.cuda()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, lse = raw.flash_fwd(qc, kc, vc, causal=mode, dropout=dropout, simt=simt, status=status)
+    grads = raw.flash_bwd(dout.cuda(), qc, kc, vc, out, lse, causal=mode, dropout=dropout, simt=simt, status=status)
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    ref = reference(q.numpy(), k.numpy(), v.numpy(), dout.numpy(), mode, D ** -0.5, *keep_mask(B, Hq, Sq, Sk, p, 11, 5))
+    res = {}
+    for name, got in zip(("out", "lse", "dq", "dk", "dv"), (out, lse, *grads)):
+        want, got = ref[name], got.double().cpu().numpy()
+        seen = np.isfinite(want)
+        assert np.array_equal(seen, np.isfinite(got)), name
+        res[name] = np.linalg.norm(got[seen] - want[seen]) / max(np.linalg.norm(want[seen]), 1e-30)
+    return res
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,mode,p", SPLIT)
+def test_fp32_on_the_tensor_cores(B, Hq, Hkv, Sq, Sk, D, mode, p):
+    # a score is short by at most D / 16 + 1 truncations of 2^-23 of its sum of magnitudes, which times the scale is
+    # 0.64 sqrt(D) for normal values: 3e-6 (D = 64) and 7.7e-6 (D = 128) on a probability, everything else is smaller
+    bound = 3e-6 if D == 64 else 7.7e-6
+    for name, err in errors(B, Hq, Hkv, Sq, Sk, D, mode, p, False).items():
+        assert err < bound, f"{name}: relative error {err:.2e}"
+
+
+@pytest.mark.parametrize("S,D", [(512, 64), (512, 128)])
+def test_fp32_tensor_core_forms_lose_no_precision(S, D):
+    fma, split = (errors(1, 4, 2, S, S, D, 1, 0.0, simt) for simt in (True, False))
+    for name in fma:   # (lse is at the rounding of its own value in both)
+        assert split[name] < 1.1 * fma[name], f"{name}: {split[name]:.2e} against {fma[name]:.2e}"
+
+
+@pytest.mark.parametrize("which,value", [("v", float("inf")), ("k", float("-inf")), ("k", float("nan")), ("q", float("inf")),
+                                         ("q", 3.4e38), ("dout", float("-inf")), ("v", 3.4e38)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_fp32_values_that_are_not_finite_spread_as_through_fp32_products(which, value, D):
+    g = torch.Generator().manual_seed(3)
+    t = {n: torch.randn(1, 2, 200, D, generator=g).cuda() for n in ("q", "k", "v", "dout")}
+    t[which][0, 1, 70, 5] = value
+    got = []
+    for simt in (True, False):
+        out, lse = raw.flash_fwd(t["q"], t["k"], t["v"], causal=0, simt=simt)
+        got.append((out, lse, *raw.flash_bwd(t["dout"], t["q"], t["k"], t["v"], out, lse, causal=0, simt=simt)))
+    for a, b in zip(*got):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+        ok = a.isfinite()
+        assert torch.allclose(a[ok], b[ok], rtol=1e-4, atol=1e-4 * float(a[ok].abs().max()))

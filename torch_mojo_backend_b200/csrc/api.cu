@@ -268,9 +268,9 @@ int fwd_impl(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tens
   // A stale error left on this thread by an earlier, unrelated runtime call must not be
   // mistaken for a launch failure.
   (void)cudaGetLastError();
-  cudaError_t e = (dtype == kF32 || opt.force_simt)
-                      ? launch_fwd_simt(p, dtype, static_cast<cudaStream_t>(stream), &launches)
-                      : launch_fwd_sm100(p, dtype, static_cast<cudaStream_t>(stream), &launches);
+  cudaError_t e = opt.force_simt ? launch_fwd_simt(p, dtype, static_cast<cudaStream_t>(stream), &launches)
+                  : dtype == kF32 ? launch_fwd_fp32(p, static_cast<cudaStream_t>(stream), &launches)
+                                  : launch_fwd_sm100(p, dtype, static_cast<cudaStream_t>(stream), &launches);
   g_launches += launches;
   if (e != cudaSuccess) note_cuda_error("b200fa_fwd", e);
   return e == cudaSuccess ? B200FA_OK : B200FA_ERR_CUDA;
@@ -329,9 +329,10 @@ int bwd_impl(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tens
   if ((rc = check_device_is_sm100(device)) != B200FA_OK) return rc;
   int launches = 0;
   (void)cudaGetLastError();
-  cudaError_t e = (dtype == kF32 || opt.force_simt)
+  cudaError_t e = opt.force_simt || (dtype == kF32 && D != 64)
                       ? launch_bwd_simt(p, dtype, static_cast<cudaStream_t>(stream), &launches)
-                      : launch_bwd_sm100(p, dtype, static_cast<cudaStream_t>(stream), &launches);
+                  : dtype == kF32 ? launch_bwd_fp32(p, static_cast<cudaStream_t>(stream), &launches)
+                                  : launch_bwd_sm100(p, dtype, static_cast<cudaStream_t>(stream), &launches);
   g_launches += launches;
   if (e != cudaSuccess) note_cuda_error("b200fa_bwd", e);
   return e == cudaSuccess ? B200FA_OK : B200FA_ERR_CUDA;

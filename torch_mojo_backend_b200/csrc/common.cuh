@@ -76,6 +76,8 @@ constexpr int kF32 = 0, kBF16 = 1, kF16 = 2;
 cudaError_t launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream, int* launches);
 int fwd_splits(const FwdParams& p);   // CTAs that share a query unit's K/V blocks in launch_fwd_sm100 (host only)
 cudaError_t launch_fwd_simt(const FwdParams& p, int dtype, cudaStream_t stream, int* launches);
+cudaError_t launch_fwd_fp32(const FwdParams& p, cudaStream_t stream, int* launches);   // fp32 on the tensor cores
+cudaError_t launch_bwd_fp32(const BwdParams& p, cudaStream_t stream, int* launches);   // ... head dim 64
 cudaError_t launch_fwd_splitkv(const SplitKvParams& p, int dtype, cudaStream_t stream, int* launches);
 cudaError_t launch_bwd_sm100(const BwdParams& p, int dtype, cudaStream_t stream, int* launches);
 cudaError_t launch_bwd_simt(const BwdParams& p, int dtype, cudaStream_t stream, int* launches);

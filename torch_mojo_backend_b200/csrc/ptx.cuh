@@ -98,6 +98,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The same by a whole converged warp, with one answer for all of its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                               uint32_t* status, uint32_t site, long long budget) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, site, budget));
+}
+
+// This thread's warp, in a form the compiler knows to be the same for the whole warp.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+
 // True when an earlier CTA of this launch (or an earlier launch sharing the status word) has
 // already reported a failed wait: later CTAs then leave at once instead of each spending its
 // own budget on a protocol that is known to be broken.
@@ -247,6 +256,28 @@ __device__ __forceinline__ void umma_ts_fast(uint32_t d_tmem, uint32_t a_tmem, u
       : "memory");
 }
 
+// The same from a converged warp: one elected lane issues.  In code that the whole warp runs, with values that
+// are the same for all of its lanes, descriptors and addresses stay in uniform registers; behind an `if (lane == 0)`
+// every MMA moves them there first, which takes the issuing lane 45 cycles an instruction (measured; with these
+// forms it is the 16 / 32 / 64 / 128 cycles that an MMA of N = 32 / 64 / 128 / 256 with A in TMEM runs).
+__device__ __forceinline__ void umma_ss_elect(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                              uint32_t idesc, bool acc) {
+  if (elect_one()) {
+    if (acc) umma_ss_fast<true>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc);
+    else     umma_ss_fast<false>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc);
+  }
+}
+__device__ __forceinline__ void umma_ts_elect(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                              bool acc) {
+  if (elect_one()) {
+    if (acc) umma_ts_fast<true>(d_tmem, a_tmem, b_lo, b_hi, idesc);
+    else     umma_ts_fast<false>(d_tmem, a_tmem, b_lo, b_hi, idesc);
+  }
+}
+__device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
+  if (elect_one()) umma_commit(bar);
+}
+
 // ---------------------------------------------------------------------------------------
 // tcgen05.ld / st, shape 32x32b: thread t of warp w touches TMEM lane 32*(w%4)+t and
 // N consecutive 32-bit columns starting at the column field of `taddr`.
@@ -271,6 +302,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
         "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
         "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+      "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
