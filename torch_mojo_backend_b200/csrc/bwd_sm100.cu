@@ -56,6 +56,8 @@ struct BwdCfg {
 
 #define B200FA_WAIT(bar, parity, site) \
   if (!mbar_wait((bar), (parity), abort_flag, p.status, (site), p.wait_budget)) goto teardown
+#define B200FA_WAIT_WARP(bar, parity, site) \
+  if (!mbar_wait_warp((bar), (parity), abort_flag, p.status, (site), p.wait_budget)) goto teardown
 
 // two exponentials on the special function unit
 __device__ __forceinline__ float2 exp2_mufu2(float2 x) { return make_float2(ex2_approx(x.x), ex2_approx(x.y)); }
@@ -100,7 +102,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   // Block order: (batch, kv head) pairs are walked `sched_group` at a time, few enough that the
   // Q / dO rows they stream stay in L2, and inside such a group the K/V tiles with the most
@@ -164,7 +166,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     for (int i = 0; i < Cfg::kStages; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&do_full[i], 1);
-      mbar_init(&qdo_empty[i], 2);   // both MMA-issuing lanes release a stage
+      mbar_init(&qdo_empty[i], 2);   // both consuming MMA warps release a stage
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
@@ -173,7 +175,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     mbar_init(dp_full, 1);
     mbar_init(p_full, 16);   // one elected arrival per compute warp
     mbar_init(ds_full, 16);
-    mbar_init(acc_full, 2);        // both MMA-issuing lanes
+    mbar_init(acc_full, 2);        // both accumulating MMA warps
     mbar_init(s_free, 16);
     mbar_init(p_empty, 1);
     mbar_init(staged, 16);
@@ -192,7 +194,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp < 16) {
     // =========================== compute warps ===========================
@@ -357,14 +359,16 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
   } else if (warp >= 16 && warp <= 18) {
     // =========================== MMA issuers ===========================
-    // A tcgen05.mma only issues once the tensor pipe has room, so an issuing lane is stalled
+    // A tcgen05.mma only issues once the tensor pipe has room, so an issuing warp is stalled
     // for about as long as its MMAs run, and it handles its waits strictly in program order.
-    // The three dependency chains of a step therefore get a lane each, so none of them waits
-    // behind another chain's operands:
+    // The three dependency chains of a step therefore get a warp each, so none of them waits
+    // behind another chain's operands.  Each runs converged, with one elected lane per MMA: behind an
+    // `if (lane == 0)` every MMA cost its lane 45 cycles of operand moves (B200, us, both kernels' MMAs so issued,
+    // before / after: dK/dV B4 Hq32 Hkv8 S4096 D128 causal 1074 / 1021, B8 H12 S1024 D64 61.6 / 54.6; dQ 729 / 701, 46.9 / 42.3):
     //   warp 16: S^T of the next step      (needs the next Q tile and S^T of this step in registers)
     //   warp 17: dK, then dP^T of the next step   (needs dS^T, the next dO tile)
     //   warp 18: dV                        (needs P^T in shared memory); frees the Q/dO stage
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc_st = umma_idesc(kBf16, false, false, 128, 128);  // S^T, dP^T
       constexpr uint32_t idesc_acc = umma_idesc(kBf16, false, true, 128, kD);   // dV (A in smem), dK (A in TMEM)
       const uint32_t tWork = tmem_base + kTmemWork, tDV = tmem_base + kTmemDV, tDK = tmem_base + kTmemDK;
@@ -382,78 +386,75 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 #pragma unroll
         for (int kk = 0; kk < kD / 16; ++kk) {
           const uint32_t off = umma_off((kk >> 2) * kSubTileBytes + (kk & 3) * 32);
-          if (kk == 0) umma_ss_fast<false>(d_tmem, a.lo + off, a.hi, bd.lo + b_stage_lo + off, bd.hi, idesc_st);
-          else         umma_ss_fast<true>(d_tmem, a.lo + off, a.hi, bd.lo + b_stage_lo + off, bd.hi, idesc_st);
+          umma_ss_elect(d_tmem, a.lo + off, a.hi, bd.lo + b_stage_lo + off, bd.hi, idesc_st, kk > 0);
         }
       };
       constexpr uint32_t kStageLo = umma_off(2 * Cfg::kTileBytes);
       if (warp == 16) {
-        B200FA_WAIT(kv_full, 0, 0x700);
+        B200FA_WAIT_WARP(kv_full, 0, 0x700);
         for (int i = 0; i < steps; ++i) {
           const int stage = i % Cfg::kStages;
-          B200FA_WAIT(&q_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x711);
+          B200FA_WAIT_WARP(&q_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x711);
           // the dK MMA of step i - 2 must have consumed dS^T from this work buffer
-          if (i >= 2) { B200FA_WAIT(&buf_free[i & 1], ((i >> 1) - 1) & 1, 0x714); }
+          if (i >= 2) { B200FA_WAIT_WARP(&buf_free[i & 1], ((i >> 1) - 1) & 1, 0x714); }
           tc_fence_after();
           issue_kmajor(tWork + (i & 1) * 128, kK, kQ, stage * kStageLo);
-          umma_commit(&s_full[i & 1]);
+          umma_commit_elect(&s_full[i & 1]);
         }
       } else if (warp == 17) {
-        B200FA_WAIT(kv_full, 0, 0x720);
+        B200FA_WAIT_WARP(kv_full, 0, 0x720);
         if (steps > 0) {
-          B200FA_WAIT(&do_full[0], 0, 0x702);
-          B200FA_WAIT(s_free, 0, 0x703);     // dP^T goes where S^T was once it sits in registers
+          B200FA_WAIT_WARP(&do_full[0], 0, 0x702);
+          B200FA_WAIT_WARP(s_free, 0, 0x703);     // dP^T goes where S^T was once it sits in registers
           tc_fence_after();
           issue_kmajor(tWork, kV, kDO, 0);
-          umma_commit(dp_full);
+          umma_commit_elect(dp_full);
         }
         for (int i = 0; i < steps; ++i) {
           const int stage = i % Cfg::kStages;
           const uint32_t stage_lo = stage * kStageLo;
           // dK += dS^T Q   (A = 16-bit dS^T in the work buffer)
           const uint32_t tDP = tWork + (i & 1) * 128;
-          B200FA_WAIT(&q_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x716);
-          B200FA_WAIT(ds_full, i & 1, 0x712);
+          B200FA_WAIT_WARP(&q_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x716);
+          B200FA_WAIT_WARP(ds_full, i & 1, 0x712);
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const uint32_t a_col = (kk >> 1) * 32 + (kk & 1) * 8;
             const uint32_t b_lo = mQ.lo + stage_lo + umma_off(kk * 2048);
-            if (kk == 0 && i == 0) umma_ts_fast<false>(tDK, tDP + a_col, b_lo, mQ.hi, idesc_acc);
-            else                   umma_ts_fast<true>(tDK, tDP + a_col, b_lo, mQ.hi, idesc_acc);
+            umma_ts_elect(tDK, tDP + a_col, b_lo, mQ.hi, idesc_acc, !(kk == 0 && i == 0));
           }
-          umma_commit(&qdo_empty[stage]);   // this lane is done with Q_i (dK) and dO_i (dP^T)
-          umma_commit(&buf_free[i & 1]);
+          umma_commit_elect(&qdo_empty[stage]);   // this warp is done with Q_i (dK) and dO_i (dP^T)
+          umma_commit_elect(&buf_free[i & 1]);
           if (i + 1 < steps) {
             // dP^T of the next step replaces S^T of the next step in the other work buffer
             const int nstage = (i + 1) % Cfg::kStages;
-            B200FA_WAIT(&do_full[nstage], static_cast<uint32_t>(((i + 1) / Cfg::kStages) & 1), 0x713);
-            B200FA_WAIT(s_free, (i + 1) & 1, 0x717);
+            B200FA_WAIT_WARP(&do_full[nstage], static_cast<uint32_t>(((i + 1) / Cfg::kStages) & 1), 0x713);
+            B200FA_WAIT_WARP(s_free, (i + 1) & 1, 0x717);
             tc_fence_after();
             issue_kmajor(tWork + ((i + 1) & 1) * 128, kV, kDO, nstage * kStageLo);
-            umma_commit(dp_full);
+            umma_commit_elect(dp_full);
           }
         }
-        umma_commit(acc_full);
+        umma_commit_elect(acc_full);
       } else {
         for (int i = 0; i < steps; ++i) {
           const int stage = i % Cfg::kStages;
           const uint32_t stage_lo = stage * kStageLo;
           // dV += P^T dO   (A = P^T tile in shared memory, K-major over the query index)
-          B200FA_WAIT(&do_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x715);
-          B200FA_WAIT(p_full, i & 1, 0x710);
+          B200FA_WAIT_WARP(&do_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x715);
+          B200FA_WAIT_WARP(p_full, i & 1, 0x710);
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const uint32_t a_off = umma_off((kk >> 2) * kSubTileBytes + (kk & 3) * 32);
             const uint32_t b_lo = mDO.lo + stage_lo + umma_off(kk * 2048);
-            if (kk == 0 && i == 0) umma_ss_fast<false>(tDV, kP.lo + a_off, kP.hi, b_lo, mDO.hi, idesc_acc);
-            else                   umma_ss_fast<true>(tDV, kP.lo + a_off, kP.hi, b_lo, mDO.hi, idesc_acc);
+            umma_ss_elect(tDV, kP.lo + a_off, kP.hi, b_lo, mDO.hi, idesc_acc, !(kk == 0 && i == 0));
           }
-          umma_commit(p_empty);
-          umma_commit(&qdo_empty[stage]);   // this lane is done with dO_i; S^T of Q_i completed long ago
+          umma_commit_elect(p_empty);
+          umma_commit_elect(&qdo_empty[stage]);   // this warp is done with dO_i; S^T of Q_i completed long ago
         }
-        umma_commit(acc_full);
+        umma_commit_elect(acc_full);
       }
     }
   } else if (warp == 19) {
@@ -515,7 +516,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int m_tiles = (p.S + kTile - 1) / kTile;
   const int m_tile = m_tiles - 1 - static_cast<int>(blockIdx.x);  // heaviest (latest) causal tiles first
@@ -583,7 +584,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp < 8) {
     // =========================== compute warps ===========================
@@ -713,9 +714,9 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
   } else if (warp == 8 || warp == 9) {
     // =========================== MMA issuers ===========================
     // Warp 8: dQ += dS_j K_j, then S of tile j+2 into the buffer dS_j just left.
-    // Warp 9: dP of tile j+1.  Separate lanes so that neither chain stalls behind the other's
-    // operands (an issuing lane is blocked while the tensor pipe is full).
-    if (lane == 0) {
+    // Warp 9: dP of tile j+1.  Separate warps so that neither chain stalls behind the other's
+    // operands (an issuing warp is blocked while the tensor pipe is full).
+    {
       constexpr uint32_t idesc_s = umma_idesc(kBf16, false, false, 128, 128);   // S, dP
       constexpr uint32_t idesc_dq = umma_idesc(kBf16, false, true, 128, kD);    // dQ (A from TMEM, K MN-major)
       const uint32_t tDP = tmem_base + kTmemDP, tDQ = tmem_base + kTmemDQ;
@@ -726,25 +727,24 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
 #pragma unroll
         for (int kk = 0; kk < kD / 16; ++kk) {
           const uint32_t off = umma_off((kk >> 2) * kSubTileBytes + (kk & 3) * 32);
-          if (kk == 0) umma_ss_fast<false>(d_tmem, a.lo + off, a.hi, bd.lo + b_slot_lo + off, bd.hi, idesc_s);
-          else         umma_ss_fast<true>(d_tmem, a.lo + off, a.hi, bd.lo + b_slot_lo + off, bd.hi, idesc_s);
+          umma_ss_elect(d_tmem, a.lo + off, a.hi, bd.lo + b_slot_lo + off, bd.hi, idesc_s, kk > 0);
         }
       };
       constexpr uint32_t kTileLo = umma_off(Cfg::kTileBytes);
       if (warp == 8) {
         // prologue: S_0, S_1
         if (n_tiles > 0) {
-          B200FA_WAIT(q_full, 0, 0xa00);
-          B200FA_WAIT(&k_full[0], 0, 0xa01);
+          B200FA_WAIT_WARP(q_full, 0, 0xa00);
+          B200FA_WAIT_WARP(&k_full[0], 0, 0xa01);
           tc_fence_after();
           issue_kmajor(tmem_base + kTmemS, kQ, kK, 0);
-          umma_commit(&s_full[0]);
+          umma_commit_elect(&s_full[0]);
         }
         if (n_tiles > 1) {
-          B200FA_WAIT(&k_full[1], 0, 0xa02);
+          B200FA_WAIT_WARP(&k_full[1], 0, 0xa02);
           tc_fence_after();
           issue_kmajor(tmem_base + kTmemS + 128, kQ, kK, kTileLo);
-          umma_commit(&s_full[1]);
+          umma_commit_elect(&s_full[1]);
         }
         int kslot = 0;  // ring slot of K_j
         for (int j = 0; j < n_tiles; ++j) {
@@ -752,43 +752,42 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
           const uint32_t tSj = tmem_base + kTmemS + buf * 128;
           const int k2slot = (kslot == 0) ? 2 : kslot - 1;   // slot of K_{j+2} = (j + 2) % 3
           // compute has written dS_j over S_j
-          B200FA_WAIT(ds_full, j & 1, 0xa10);
+          B200FA_WAIT_WARP(ds_full, j & 1, 0xa10);
           tc_fence_after();
           // dQ += dS_j K_j   (A = 16-bit dS in the S_j columns, B = K_j rows as the contraction index)
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const uint32_t a_col = (kk < 4) ? kk * 8 : 64 + (kk - 4) * 8;
             const uint32_t b_lo = mK.lo + kslot * kTileLo + umma_off(kk * 2048);
-            if (kk == 0 && j == 0) umma_ts_fast<false>(tDQ, tSj + a_col, b_lo, mK.hi, idesc_dq);
-            else                   umma_ts_fast<true>(tDQ, tSj + a_col, b_lo, mK.hi, idesc_dq);
+            umma_ts_elect(tDQ, tSj + a_col, b_lo, mK.hi, idesc_dq, !(kk == 0 && j == 0));
           }
-          umma_commit(&k_empty[kslot]);
+          umma_commit_elect(&k_empty[kslot]);
           if (j + 2 < n_tiles) {
             // S of tile j+2 re-uses this S buffer
-            B200FA_WAIT(&k_full[k2slot], static_cast<uint32_t>(((j + 2) / 3) & 1), 0xa11);
+            B200FA_WAIT_WARP(&k_full[k2slot], static_cast<uint32_t>(((j + 2) / 3) & 1), 0xa11);
             tc_fence_after();
             issue_kmajor(tSj, kQ, kK, k2slot * kTileLo);
-            umma_commit(&s_full[buf]);
+            umma_commit_elect(&s_full[buf]);
           }
           if (++kslot == 3) kslot = 0;
         }
-        umma_commit(acc_full);
+        umma_commit_elect(acc_full);
       } else if (n_tiles > 0) {
         // dP_0, then dP_{j+1} whenever the compute warps have consumed dP_j
-        B200FA_WAIT(do_full, 0, 0xa20);
-        B200FA_WAIT(&v_full[0], 0, 0xa03);
+        B200FA_WAIT_WARP(do_full, 0, 0xa20);
+        B200FA_WAIT_WARP(&v_full[0], 0, 0xa03);
         tc_fence_after();
         issue_kmajor(tDP, kDO, kV, 0);
-        umma_commit(dp_full);
-        umma_commit(&v_empty[0]);
+        umma_commit_elect(dp_full);
+        umma_commit_elect(&v_empty[0]);
         for (int j = 0; j + 1 < n_tiles; ++j) {
           const int vslot = (j + 1) & 1;
-          B200FA_WAIT(&v_full[vslot], ((j + 1) >> 1) & 1, 0xa12);
-          B200FA_WAIT(ds_full, j & 1, 0xa13);
+          B200FA_WAIT_WARP(&v_full[vslot], ((j + 1) >> 1) & 1, 0xa12);
+          B200FA_WAIT_WARP(ds_full, j & 1, 0xa13);
           tc_fence_after();
           issue_kmajor(tDP, kDO, kV, vslot * kTileLo);
-          umma_commit(dp_full);
-          umma_commit(&v_empty[vslot]);
+          umma_commit_elect(dp_full);
+          umma_commit_elect(&v_empty[vslot]);
         }
       }
     }
@@ -818,6 +817,7 @@ teardown:
   }
 }
 #undef B200FA_WAIT
+#undef B200FA_WAIT_WARP
 
 // ------------------------------------------------------------------------------------------
 // preprocess: dpsum = rowsum(dO * O), lse2 = lse * log2(e), per (b, h, row), padded to a
