@@ -10,7 +10,7 @@ import pytest
 import torch
 
 from oracle import sdpa_oracle as O
-from tests.helpers import TOL_16BIT, TOL_FP32, TOL_LSE, assert_within, golden_names, load_golden
+from tests.helpers import TOL_16BIT, TOL_FP32, TOL_LSE, assert_within, golden_names, load_golden, parity_report
 from torch_mojo_backend_b200 import _lib, raw
 
 pytestmark = pytest.mark.gpu
@@ -120,6 +120,28 @@ def test_unmasked_attention_over_another_key_length(dtype, B, Hq, Hkv, Sq, Sk, D
         assert_within("simt out", s_out, ref_out, tol, dtype)
         assert_within("simt dk", s_dk, rdk, tol, dtype)
         assert_within("simt dq", s_dq, rdq, tol, dtype)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("group,Sq,causal,p", [
+    # 1, 2, ... query tiles for a thread block of the dK/dV kernel: each fill of its rings of three and four and of its two
+    # score buffers, ragged ends, a diagonal, dropout
+    (1, 100, False, 0.0), (1, 256, False, 0.0), (1, 300, False, 0.0), (2, 200, False, 0.0), (1, 640, True, 0.0),
+    (3, 250, True, 0.0), (1, 897, False, 0.2), (5, 260, True, 0.2)])
+def test_backward_over_every_fill_of_its_rings(D, group, Sq, causal, p):
+    dtype = torch.float16 if D == 64 else torch.bfloat16
+    g = torch.Generator().manual_seed(20260925 + Sq + group)
+    Sk = Sq if causal else 200
+    draw = lambda h, s, std: (torch.randn(2, h, s, D, generator=g) * std).to(dtype).cuda()
+    q, k, v, dout = draw(2 * group, Sq, 0.5), draw(2, Sk, 0.5), draw(2, Sk, 0.5), draw(2 * group, Sq, 1.0)
+    drop = (p, 77, 5) if p else None
+    got, want = {}, {}
+    for res, simt in ((got, False), (want, True)):
+        out, lse = raw.flash_fwd(q, k, v, causal=causal, simt=simt, dropout=drop)
+        res["dq"], res["dk"], res["dv"] = raw.flash_bwd(dout, q, k, v, out, lse, causal=causal, simt=simt, dropout=drop)
+    for name in got:
+        # both round to the type: the contract's tolerance plus an ulp of the reference's own rounding
+        assert parity_report(name, got[name], want[name], tol_for(dtype), dtype, ref_is_rounded=True)["over_widened"] == 0
 
 
 def test_randomised_shapes_agree_with_the_exact_fp32_kernels():

@@ -19,9 +19,9 @@
 // as the A operand of dQ += dS K).  S and dP are computed twice (7 tile GEMMs per tile pair
 // instead of 5), every accumulator lives in TMEM, and the results are deterministic.
 //
-// Both kernels: warps 0-3 and 4-7 are two compute warpgroups that split the 128 score
-// columns of a tile in halves (thread <-> TMEM lane), warps 8 and 9 each issue one of the two
-// independent MMA chains (the dK/dV kernel uses warp 10 for a third), the next warp drives TMA.
+// dK/dV kernel: warps 0-15 are four compute warpgroups that split the 128 score columns of a tile in
+// quarters (thread <-> TMEM lane), warp 16 issues every MMA, warp 17 drives TMA.  dQ kernel: warps 0-3 and
+// 4-7 split the columns in halves, warps 8 and 9 each issue one of two independent MMA chains, warp 10 drives TMA.
 #include <mutex>
 
 #include "common.cuh"
@@ -33,21 +33,21 @@ namespace {
 
 constexpr int kTile = 128;
 constexpr int kThreads = 384;        // dQ kernel: 8 compute warps + 4
-constexpr int kDkdvThreads = 640;    // dK/dV kernel: 16 compute warps + 4
+constexpr int kDkdvThreads = 576;    // dK/dV kernel: 16 compute warps + 2
 constexpr int kSubTileBytes = 128 * 128;
 
 template <int kD>
 struct BwdCfg {
   static constexpr int kTileBytes = kTile * kD * 2;
   static constexpr int kSub = kD / 64;
-  static constexpr int kStages = 2;
-  // resident pair of tiles, then kStages pairs of streamed tiles, then per-stage row statistics
+  // dK/dV kernel: the resident pair of tiles, the rings of streamed tiles, then the row statistics of two steps
+  static constexpr int kQStages = kD == 128 ? 3 : 4, kDoStages = kD == 128 ? 2 : 4;
   static constexpr int kOffResident = 0;
-  static constexpr int kOffStream = 2 * kTileBytes;
-  static constexpr int kOffP = kOffStream + kStages * 2 * kTileBytes;     // dK/dV kernel: 128 x 128 16-bit P^T tile
-  static constexpr int kOffStat = kOffP + 128 * 128 * 2;                  // [stage][lse2|dpsum][128] fp32
-  static constexpr int kOffBars = kOffStat + kStages * 2 * 128 * 4;
-  static constexpr int kNumBars = 20;
+  static constexpr int kOffQ = 2 * kTileBytes;
+  static constexpr int kOffDo = kOffQ + kQStages * kTileBytes;
+  static constexpr int kOffStat = kOffDo + kDoStages * kTileBytes;        // [step & 1][lse2|dpsum][128] fp32
+  static constexpr int kOffBars = kOffStat + 2 * 2 * 128 * 4;
+  static constexpr int kNumBars = 2 * kQStages + 2 * kDoStages + 14;
   // the dQ kernel keeps 2 resident + 3 K + 2 V tiles and no per-stage statistics
   static constexpr int kOffDqBars = 7 * kTileBytes;
   static constexpr int kSmemBytes =
@@ -76,29 +76,32 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 const __grid_constant__ CUtensorMap mapDK, const __grid_constant__ CUtensorMap mapDV,
                 const BwdParams p, const int sched_group) {
   using Cfg = BwdCfg<kD>;
-  // TMEM: two 128-column work buffers (step i uses buffer i & 1 for S^T, then dP^T, then dS^T),
-  // then the dV and dK accumulators.
-  constexpr int kTmemWork = 0, kTmemDV = 256, kTmemDK = 256 + kD;
+  // TMEM: two 128-column work buffers (step i has S^T in buffer i & 1, then P^T and dS^T, 16-bit, in its place),
+  // the dV and dK accumulators, and at D = 64 a third buffer for dP^T; at D = 128 dP^T is in the other step's buffer.
+  constexpr bool kOwnDp = kD == 64;
+  constexpr int kTmemWork = 0, kTmemDV = 256, kTmemDK = 256 + kD, kTmemDP = 384;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem + Cfg::kOffResident;
   uint8_t* sV = sK + Cfg::kTileBytes;
-  uint8_t* sQ = smem + Cfg::kOffStream;                          // stage s: sQ + s * 2 * tile, dO right behind
-  uint8_t* sP = smem + Cfg::kOffP;                               // 16-bit P^T, [key row][query column], swizzled
+  uint8_t* sQ = smem + Cfg::kOffQ;
+  uint8_t* sDO = smem + Cfg::kOffDo;
   float* sStat = reinterpret_cast<float*>(smem + Cfg::kOffStat);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBars);
-  uint64_t* kv_full = bars;                        // [1]
-  uint64_t* q_full = kv_full + 1;                  // [kStages]  Q tile + lse2
-  uint64_t* do_full = q_full + Cfg::kStages;       // [kStages]  dO tile + dpsum
-  uint64_t* qdo_empty = do_full + Cfg::kStages;    // [kStages]
-  uint64_t* s_full = qdo_empty + Cfg::kStages;     // [2]  S^T ready in work buffer b
-  uint64_t* buf_free = s_full + 2;                 // [2]  dK MMA has consumed dS^T from work buffer b
-  uint64_t* dp_full = buf_free + 2;                // dP^T ready
-  uint64_t* p_full = dp_full + 1;                  // P^T written  (8 warp arrivals)
-  uint64_t* ds_full = p_full + 1;                  // dS^T written (8 warp arrivals)
+  uint64_t* k_full = bars;                         // [1]
+  uint64_t* v_full = k_full + 1;                   // [1]
+  uint64_t* q_full = v_full + 1;                   // [kQStages]
+  uint64_t* q_empty = q_full + Cfg::kQStages;      // [kQStages]  dK MMA (and S^T before it) done
+  uint64_t* do_full = q_empty + Cfg::kQStages;     // [kDoStages]
+  uint64_t* do_empty = do_full + Cfg::kDoStages;   // [kDoStages]  dV MMA (and dP^T before it) done
+  uint64_t* stat_full = do_empty + Cfg::kDoStages; // [2]  lse2 and dpsum of a step
+  uint64_t* stat_empty = stat_full + 2;            // [2]
+  uint64_t* s_full = stat_empty + 2;               // [2]  S^T ready in work buffer b
+  uint64_t* dp_full = s_full + 2;                  // dP^T ready
+  uint64_t* dp_free = dp_full + 1;                 // dP^T read into registers (16 warp arrivals)
+  uint64_t* p_full = dp_free + 1;                  // P^T written  (16 warp arrivals)
+  uint64_t* ds_full = p_full + 1;                  // dS^T written (16 warp arrivals)
   uint64_t* acc_full = ds_full + 1;                // dK, dV complete
-  uint64_t* s_free = acc_full + 1;                 // S^T read into registers (8 warp arrivals)
-  uint64_t* p_empty = s_free + 1;                  // dV MMA has consumed the P^T tile
-  uint64_t* staged = p_empty + 1;                  // dV and dK tiles staged in shared memory (16 warp arrivals)
+  uint64_t* staged = acc_full + 1;                 // dV and dK tiles staged in shared memory (16 warp arrivals)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -142,50 +145,62 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 #pragma unroll
     for (int cs = 0; cs < Cfg::kSub; ++cs) tma_load_4d(dst + cs * kSubTileBytes, map, bar, cs * 64, srow, head, b);
   };
-  // Q (with lse2) and dO (with dpsum) of step i into ring stage i % kStages
-  auto load_step = [&](int i) {
-    const int stage = i % Cfg::kStages;
-    const int h = hk * group + i / per_head;
-    const int m_tile = m_start + i % per_head;
-    const int64_t stat_off = (static_cast<int64_t>(b) * p.Hq + h) * p.Spad + m_tile * kTile;
-    float* st = sStat + stage * 256;
-    uint8_t* q_dst = sQ + stage * 2 * Cfg::kTileBytes;
-    mbar_arrive_expect_tx(&q_full[stage], Cfg::kTileBytes + 512);
-    load_tile(&mapQ, q_dst, &q_full[stage], m_tile * kTile, h);
-    bulk_load_1d(st, p.lse_log2 + stat_off, 512, &q_full[stage]);
-    mbar_arrive_expect_tx(&do_full[stage], Cfg::kTileBytes + 512);
-    load_tile(&mapDO, q_dst + Cfg::kTileBytes, &do_full[stage], m_tile * kTile, h);
-    bulk_load_1d(st + 128, p.dpsum + stat_off, 512, &do_full[stage]);
+  // Q, dO and the row statistics of step i into their rings
+  auto load_q = [&](int i) {
+    const int stage = i % Cfg::kQStages;
+    mbar_arrive_expect_tx(&q_full[stage], Cfg::kTileBytes);
+    load_tile(&mapQ, sQ + stage * Cfg::kTileBytes, &q_full[stage], (m_start + i % per_head) * kTile, hk * group + i / per_head);
   };
-  if (warp == 19 && lane == 0) {
+  auto load_do = [&](int i) {
+    const int stage = i % Cfg::kDoStages;
+    mbar_arrive_expect_tx(&do_full[stage], Cfg::kTileBytes);
+    load_tile(&mapDO, sDO + stage * Cfg::kTileBytes, &do_full[stage], (m_start + i % per_head) * kTile, hk * group + i / per_head);
+  };
+  auto load_stat = [&](int i) {
+    const int64_t off = (static_cast<int64_t>(b) * p.Hq + hk * group + i / per_head) * p.Spad + (m_start + i % per_head) * kTile;
+    float* st = sStat + (i & 1) * 256;
+    mbar_arrive_expect_tx(&stat_full[i & 1], 1024);
+    bulk_load_1d(st, p.lse_log2 + off, 512, &stat_full[i & 1]);
+    bulk_load_1d(st + 128, p.dpsum + off, 512, &stat_full[i & 1]);
+  };
+  if (warp == 17 && lane == 0) {
     tma_prefetch_desc(&mapK);
     tma_prefetch_desc(&mapQ);
     tma_prefetch_desc(&mapDO);
     tma_prefetch_desc(&mapV);
-    mbar_init(kv_full, 1);
-    for (int i = 0; i < Cfg::kStages; ++i) {
+    mbar_init(k_full, 1);
+    mbar_init(v_full, 1);
+    for (int i = 0; i < Cfg::kQStages; ++i) {
       mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+    }
+    for (int i = 0; i < Cfg::kDoStages; ++i) {
       mbar_init(&do_full[i], 1);
-      mbar_init(&qdo_empty[i], 2);   // both consuming MMA warps release a stage
+      mbar_init(&do_empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
+      mbar_init(&stat_full[i], 1);
+      mbar_init(&stat_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&buf_free[i], 1);
     }
     mbar_init(dp_full, 1);
-    mbar_init(p_full, 16);   // one elected arrival per compute warp
+    mbar_init(dp_free, 16);   // one elected arrival per compute warp
+    mbar_init(p_full, 16);
     mbar_init(ds_full, 16);
-    mbar_init(acc_full, 2);        // both accumulating MMA warps
-    mbar_init(s_free, 16);
-    mbar_init(p_empty, 1);
+    mbar_init(acc_full, 1);
     mbar_init(staged, 16);
     *abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(kv_full, 2 * Cfg::kTileBytes);
-    load_tile(&mapK, sK, kv_full, n0, hk);
-    if (steps > 0) load_step(0);
-    load_tile(&mapV, sV, kv_full, n0, hk);
+    mbar_arrive_expect_tx(k_full, Cfg::kTileBytes);
+    load_tile(&mapK, sK, k_full, n0, hk);
+    if (steps > 0) {
+      load_q(0);
+      load_stat(0);
+      load_do(0);
+    }
+    mbar_arrive_expect_tx(v_full, Cfg::kTileBytes);
+    load_tile(&mapV, sV, v_full, n0, hk);
   }
   if (warp == 16) {
     tmem_alloc(tmem_slot, 512);
@@ -203,31 +218,18 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tWork = tmem_base + lane_off + kTmemWork + wg * 32;
     const float c = p.scale_log2;
-    // this thread's 64 bytes (32 query columns) of its row of the 128-byte-swizzled P^T tile
-    uint8_t* p_row = sP + (wg >> 1) * kSubTileBytes + j * 128;
-    const int chunk0 = (wg & 1) * 4;
     for (int i = 0; i < steps; ++i) {
-      const int stage = i % Cfg::kStages;
-      const uint32_t ring_phase = static_cast<uint32_t>((i / Cfg::kStages) & 1);
       const int m_tile = m_start + i % per_head;
-      const float4* lse2 = reinterpret_cast<const float4*>(sStat + stage * 256 + wg * 32);
+      const float4* lse2 = reinterpret_cast<const float4*>(sStat + (i & 1) * 256 + wg * 32);
       const float4* dps = lse2 + 32;
-      // ---- P^T = exp2(S^T * c - lse2).  S^T is pulled into registers in one go and released
-      // at once, so the S^T MMA of the next step can run while the exponentials do;
-      // P^T goes to shared memory (the A operand of dV += P^T dO) instead of back over S^T.
-      // S^T, dP^T and dS^T of this step live one after the other in work buffer i & 1
-      const uint32_t tS = tWork + (i & 1) * 128, tDP = tS;
+      // ---- P^T = exp2(S^T * c - lse2).  P^T and then dS^T (16-bit) take the columns of S^T that this warp has read
+      const uint32_t tS = tWork + (i & 1) * 128, tDP = kOwnDp ? tWork + kTmemDP : tWork + ((i + 1) & 1) * 128;
       B200FA_WAIT(&s_full[i & 1], (i >> 1) & 1, 0x500);
-      // lse2 rode in with the Q tile; observing its barrier directly makes the bulk copy visible here
-      B200FA_WAIT(&q_full[stage], ring_phase, 0x501);
+      B200FA_WAIT(&stat_full[i & 1], (i >> 1) & 1, 0x501);
       tc_fence_after();
       float pf[32];
-      {
-        tmem_ld32(tS, reinterpret_cast<uint32_t*>(pf));
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive_warp(s_free);
-      }
+      tmem_ld32(tS, reinterpret_cast<uint32_t*>(pf));
+      tmem_wait_ld();
       const float2 c2 = make_float2(c, c);
 #pragma unroll
       for (int e4 = 0; e4 < 8; ++e4) {
@@ -257,33 +259,33 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                               (dropout_bits16(p.drop, b * p.Hq + h_now, q_glob, blk + 1) << 16);
         keep = warp_transpose_bits(mine);
       }
-      // the previous step's dV MMA must have finished reading the P^T tile
-      if (i > 0) { B200FA_WAIT(p_empty, (i - 1) & 1, 0x502); }
+      {
+        uint32_t pk[16];
 #pragma unroll
-      for (int chunk = 0; chunk < 4; ++chunk) {
-        float pd[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          pd[e] = pf[chunk * 8 + e];
-          if constexpr (kDropout) pd[e] = ((keep >> (chunk * 8 + e)) & 1u) ? pd[e] * p.drop.inv_keep : 0.f;
+        for (int e = 0; e < 16; ++e) {
+          float p0 = pf[2 * e], p1 = pf[2 * e + 1];
+          if constexpr (kDropout) {
+            p0 = (keep >> (2 * e)) & 1u ? p0 * p.drop.inv_keep : 0.f;
+            p1 = (keep >> (2 * e)) & 2u ? p1 * p.drop.inv_keep : 0.f;
+          }
+          pk[e] = pack2<kBf16>(p0, p1);
         }
-        uint4 w;
-        w.x = pack2<kBf16>(pd[0], pd[1]);
-        w.y = pack2<kBf16>(pd[2], pd[3]);
-        w.z = pack2<kBf16>(pd[4], pd[5]);
-        w.w = pack2<kBf16>(pd[6], pd[7]);
-        *reinterpret_cast<uint4*>(p_row + (((chunk0 + chunk) ^ (j & 7)) << 4)) = w;
+        tmem_st16(tS, pk);
       }
-      fence_proxy_async_smem();
+      tmem_wait_st();
+      tc_fence_before();
       mbar_arrive_warp(p_full);
       // ---- dS^T = P^T * (dP^T - dpsum)
       B200FA_WAIT(dp_full, i & 1, 0x510);
-      B200FA_WAIT(&do_full[stage], ring_phase, 0x511);
       tc_fence_after();
       {
         uint32_t d[32];
         tmem_ld32(tDP, d);
         tmem_wait_ld();
+        if constexpr (!kOwnDp) {   // S^T of the next step goes there
+          tc_fence_before();
+          mbar_arrive_warp(dp_free);
+        }
         const float* df = reinterpret_cast<const float*>(d);
         uint32_t pk[16];
 #pragma unroll
@@ -304,7 +306,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           pk[e4 * 2] = pack2<kBf16>(s0.x, s0.y);
           pk[e4 * 2 + 1] = pack2<kBf16>(s1.x, s1.y);
         }
-        tmem_st16(tDP, pk);
+        tmem_st16(tS + 16, pk);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -314,7 +316,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     B200FA_WAIT(acc_full, 0, 0x520);
     tc_fence_after();
     {
-      // The 16-bit dV and dK tiles are staged in the Q / dO ring (every MMA that read it has
+      // The 16-bit dV and dK tiles are staged in the Q ring (every MMA that read it has
       // completed) in the swizzled box layout and leave through TMA stores: whole 128-byte
       // lines, key rows past the end of the sequence clipped by the tensor map.
       constexpr int kQuarter = kD / 4;
@@ -357,115 +359,103 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         tma_store_wait_read();
       }
     }
-  } else if (warp >= 16 && warp <= 18) {
-    // =========================== MMA issuers ===========================
-    // A tcgen05.mma only issues once the tensor pipe has room, so an issuing warp is stalled
-    // for about as long as its MMAs run, and it handles its waits strictly in program order.
-    // The three dependency chains of a step therefore get a warp each, so none of them waits
-    // behind another chain's operands.  Each runs converged, with one elected lane per MMA: behind an
-    // `if (lane == 0)` every MMA cost its lane 45 cycles of operand moves (B200, us, both kernels' MMAs so issued,
-    // before / after: dK/dV B4 Hq32 Hkv8 S4096 D128 causal 1074 / 1021, B8 H12 S1024 D64 61.6 / 54.6; dQ 729 / 701, 46.9 / 42.3):
-    //   warp 16: S^T of the next step      (needs the next Q tile and S^T of this step in registers)
-    //   warp 17: dK, then dP^T of the next step   (needs dS^T, the next dO tile)
-    //   warp 18: dV                        (needs P^T in shared memory); frees the Q/dO stage
-    {
-      constexpr uint32_t idesc_st = umma_idesc(kBf16, false, false, 128, 128);  // S^T, dP^T
-      constexpr uint32_t idesc_acc = umma_idesc(kBf16, false, true, 128, kD);   // dV (A in smem), dK (A in TMEM)
-      const uint32_t tWork = tmem_base + kTmemWork, tDV = tmem_base + kTmemDV, tDK = tmem_base + kTmemDK;
-      // Descriptors: fixed high word + start-address low word.  K-major form for the S^T / dP^T
-      // operands and the P^T tile, MN-major form (LBO = next 64-column sub-tile) when Q / dO
-      // are the B operand of an accumulating MMA.
-      const UmmaDesc kK = umma_desc_split(smem_u32(sK), 16, 1024), kV = umma_desc_split(smem_u32(sV), 16, 1024),
-                     kQ = umma_desc_split(smem_u32(sQ), 16, 1024),
-                     kDO = umma_desc_split(smem_u32(sQ) + Cfg::kTileBytes, 16, 1024),
-                     kP = umma_desc_split(smem_u32(sP), 16, 1024);
-      const UmmaDesc mQ = umma_desc_split(smem_u32(sQ), kSubTileBytes, 1024),
-                     mDO = umma_desc_split(smem_u32(sQ) + Cfg::kTileBytes, kSubTileBytes, 1024);
-      // D[128 x 128] = A[128 x kD] * B[128 x kD]^T, both K-major
-      auto issue_kmajor = [&](uint32_t d_tmem, const UmmaDesc& a, const UmmaDesc& bd, uint32_t b_stage_lo) {
+  } else if (warp == 16) {
+    // =========================== MMA issuer ===========================
+    // One warp issues all four products, so that the order on the tensor pipe is the program's: what a later
+    // product overwrites in tensor memory, the earlier ones have read.  It runs converged, with one elected lane
+    // per MMA (behind an `if (lane == 0)` every MMA cost its lane 45 cycles of operand moves).
+    // The bound at D = 128: a step's MMAs take 2048 cycles, and the 6 KB that shared memory moves per 64 of them (two
+    // operands of S^T and dP^T, one of dV and dK, the tiles coming in) as long again.  P^T therefore goes to tensor
+    // memory over the scores it came from, and not to a tile in shared memory (whose stores and reads took 768 cycles
+    // more a step, and its 32 KB the place of a third Q stage); dP^T needs the other buffer for that, so S^T of the
+    // next step starts when dP^T has been read.  At D = 64 tensor memory has room for a third buffer, and S^T runs a
+    // step ahead.  B200, us, with P^T in shared memory / this: B4 Hq32 Hkv8 S4096 D128 bf16 causal 964 / 903,
+    // B8 H16 S2048 D128 fp16 492 / 467, B8 H12 S1024 D64 bf16 causal 57.8 / 51.4, B8 H16 S4096 D64 fp16 1246 / 1033.
+    constexpr uint32_t idesc_st = umma_idesc(kBf16, false, false, 128, 128);  // S^T, dP^T
+    constexpr uint32_t idesc_acc = umma_idesc(kBf16, false, true, 128, kD);   // dV, dK (A in TMEM)
+    const uint32_t tWork = tmem_base + kTmemWork, tDV = tmem_base + kTmemDV, tDK = tmem_base + kTmemDK;
+    const UmmaDesc kK = umma_desc_split(smem_u32(sK), 16, 1024), kV = umma_desc_split(smem_u32(sV), 16, 1024);
+    const UmmaDesc kQ = umma_desc_split(smem_u32(sQ), 16, 1024);                         // ring base, K-major
+    const UmmaDesc kDO = umma_desc_split(smem_u32(sDO), 16, 1024);
+    const UmmaDesc mQ = umma_desc_split(smem_u32(sQ), kSubTileBytes, 1024);              // ring base, MN-major
+    const UmmaDesc mDO = umma_desc_split(smem_u32(sDO), kSubTileBytes, 1024);
+    constexpr uint32_t kTileLo = umma_off(Cfg::kTileBytes);
+    // acc[128 x 128] = A[128 x D] * B[128 x D]^T, both K-major
+    auto issue_kmajor = [&](uint32_t d_tmem, const UmmaDesc& a, const UmmaDesc& bd, uint32_t b_stage_lo) {
 #pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t off = umma_off((kk >> 2) * kSubTileBytes + (kk & 3) * 32);
-          umma_ss_elect(d_tmem, a.lo + off, a.hi, bd.lo + b_stage_lo + off, bd.hi, idesc_st, kk > 0);
-        }
-      };
-      constexpr uint32_t kStageLo = umma_off(2 * Cfg::kTileBytes);
-      if (warp == 16) {
-        B200FA_WAIT_WARP(kv_full, 0, 0x700);
-        for (int i = 0; i < steps; ++i) {
-          const int stage = i % Cfg::kStages;
-          B200FA_WAIT_WARP(&q_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x711);
-          // the dK MMA of step i - 2 must have consumed dS^T from this work buffer
-          if (i >= 2) { B200FA_WAIT_WARP(&buf_free[i & 1], ((i >> 1) - 1) & 1, 0x714); }
-          tc_fence_after();
-          issue_kmajor(tWork + (i & 1) * 128, kK, kQ, stage * kStageLo);
-          umma_commit_elect(&s_full[i & 1]);
-        }
-      } else if (warp == 17) {
-        B200FA_WAIT_WARP(kv_full, 0, 0x720);
-        if (steps > 0) {
-          B200FA_WAIT_WARP(&do_full[0], 0, 0x702);
-          B200FA_WAIT_WARP(s_free, 0, 0x703);     // dP^T goes where S^T was once it sits in registers
-          tc_fence_after();
-          issue_kmajor(tWork, kV, kDO, 0);
-          umma_commit_elect(dp_full);
-        }
-        for (int i = 0; i < steps; ++i) {
-          const int stage = i % Cfg::kStages;
-          const uint32_t stage_lo = stage * kStageLo;
-          // dK += dS^T Q   (A = 16-bit dS^T in the work buffer)
-          const uint32_t tDP = tWork + (i & 1) * 128;
-          B200FA_WAIT_WARP(&q_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x716);
-          B200FA_WAIT_WARP(ds_full, i & 1, 0x712);
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t a_col = (kk >> 1) * 32 + (kk & 1) * 8;
-            const uint32_t b_lo = mQ.lo + stage_lo + umma_off(kk * 2048);
-            umma_ts_elect(tDK, tDP + a_col, b_lo, mQ.hi, idesc_acc, !(kk == 0 && i == 0));
-          }
-          umma_commit_elect(&qdo_empty[stage]);   // this warp is done with Q_i (dK) and dO_i (dP^T)
-          umma_commit_elect(&buf_free[i & 1]);
-          if (i + 1 < steps) {
-            // dP^T of the next step replaces S^T of the next step in the other work buffer
-            const int nstage = (i + 1) % Cfg::kStages;
-            B200FA_WAIT_WARP(&do_full[nstage], static_cast<uint32_t>(((i + 1) / Cfg::kStages) & 1), 0x713);
-            B200FA_WAIT_WARP(s_free, (i + 1) & 1, 0x717);
-            tc_fence_after();
-            issue_kmajor(tWork + ((i + 1) & 1) * 128, kV, kDO, nstage * kStageLo);
-            umma_commit_elect(dp_full);
-          }
-        }
-        umma_commit_elect(acc_full);
-      } else {
-        for (int i = 0; i < steps; ++i) {
-          const int stage = i % Cfg::kStages;
-          const uint32_t stage_lo = stage * kStageLo;
-          // dV += P^T dO   (A = P^T tile in shared memory, K-major over the query index)
-          B200FA_WAIT_WARP(&do_full[stage], static_cast<uint32_t>((i / Cfg::kStages) & 1), 0x715);
-          B200FA_WAIT_WARP(p_full, i & 1, 0x710);
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t a_off = umma_off((kk >> 2) * kSubTileBytes + (kk & 3) * 32);
-            const uint32_t b_lo = mDO.lo + stage_lo + umma_off(kk * 2048);
-            umma_ss_elect(tDV, kP.lo + a_off, kP.hi, b_lo, mDO.hi, idesc_acc, !(kk == 0 && i == 0));
-          }
-          umma_commit_elect(p_empty);
-          umma_commit_elect(&qdo_empty[stage]);   // this warp is done with dO_i; S^T of Q_i completed long ago
-        }
-        umma_commit_elect(acc_full);
+      for (int kk = 0; kk < kD / 16; ++kk) {
+        const uint32_t off = umma_off((kk >> 2) * kSubTileBytes + (kk & 3) * 32);
+        umma_ss_elect(d_tmem, a.lo + off, a.hi, bd.lo + b_stage_lo + off, bd.hi, idesc_st, kk > 0);
       }
+    };
+    // acc[128 x D] += A[128 x 128] (16-bit, in TMEM from `a_tmem`: 16 columns of every 32) * B[128 x D]
+    auto issue_acc = [&](uint32_t d_tmem, uint32_t a_tmem, const UmmaDesc& bd, uint32_t b_stage_lo, bool first) {
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        umma_ts_elect(d_tmem, a_tmem + (kk >> 1) * 32 + (kk & 1) * 8, bd.lo + b_stage_lo + umma_off(kk * 2048), bd.hi, idesc_acc,
+                      !(kk == 0 && first));
+    };
+    int q_next = 0, do_next = 0;               // ring stage that the next S^T, dP^T reads
+    uint32_t q_phase = 0, do_phase = 0;
+    int q_stage = 0, do_stage = 0;             // ring stage that the next dK, dV reads
+#define B200FA_ISSUE_S(step)                                                  \
+  do {                                                                        \
+    B200FA_WAIT_WARP(&q_full[q_next], q_phase, 0x711);                        \
+    tc_fence_after();                                                         \
+    issue_kmajor(tWork + ((step) & 1) * 128, kK, kQ, q_next * kTileLo);       \
+    umma_commit_elect(&s_full[(step) & 1]);                                   \
+    if (++q_next == Cfg::kQStages) { q_next = 0; q_phase ^= 1; }              \
+  } while (0)
+#define B200FA_ISSUE_DP(step)                                                 \
+  do {                                                                        \
+    B200FA_WAIT_WARP(&do_full[do_next], do_phase, 0x713);                     \
+    tc_fence_after();                                                         \
+    issue_kmajor(kOwnDp ? tWork + kTmemDP : tWork + (((step) + 1) & 1) * 128, kV, kDO, do_next * kTileLo); \
+    umma_commit_elect(dp_full);                                               \
+    if (++do_next == Cfg::kDoStages) { do_next = 0; do_phase ^= 1; }          \
+  } while (0)
+    if (steps > 0) {
+      B200FA_WAIT_WARP(k_full, 0, 0x700);
+      B200FA_ISSUE_S(0);
+      B200FA_WAIT_WARP(v_full, 0, 0x701);
+      B200FA_ISSUE_DP(0);
+      if (kOwnDp && steps > 1) B200FA_ISSUE_S(1);
     }
-  } else if (warp == 19) {
+    for (int i = 0; i < steps; ++i) {
+      const uint32_t tS = tWork + (i & 1) * 128;
+      if (!kOwnDp && i + 1 < steps) {
+        // S^T of the next step goes ahead of this one's dV: it is what the compute warps wait for
+        B200FA_WAIT_WARP(dp_free, i & 1, 0x717);
+        B200FA_ISSUE_S(i + 1);
+      }
+      B200FA_WAIT_WARP(p_full, i & 1, 0x710);
+      tc_fence_after();
+      issue_acc(tDV, tS, mDO, do_stage * kTileLo, i == 0);          // dV += P^T dO
+      umma_commit_elect(&do_empty[do_stage]);
+      B200FA_WAIT_WARP(ds_full, i & 1, 0x712);
+      tc_fence_after();
+      issue_acc(tDK, tS + 16, mQ, q_stage * kTileLo, i == 0);       // dK += dS^T Q
+      umma_commit_elect(&q_empty[q_stage]);
+      umma_commit_elect(&stat_empty[i & 1]);
+      if (i + 1 < steps) B200FA_ISSUE_DP(i + 1);
+      if (kOwnDp && i + 2 < steps) B200FA_ISSUE_S(i + 2);
+      if (++q_stage == Cfg::kQStages) q_stage = 0;
+      if (++do_stage == Cfg::kDoStages) do_stage = 0;
+    }
+    umma_commit_elect(acc_full);
+#undef B200FA_ISSUE_S
+#undef B200FA_ISSUE_DP
+  } else if (warp == 17) {
     // =========================== TMA producer ===========================
     if (lane == 0) {
       // step 0 went out before the block-wide synchronisation
       for (int i = 1; i < steps; ++i) {
-        if (i >= Cfg::kStages) {
-          B200FA_WAIT(&qdo_empty[i % Cfg::kStages], ((i / Cfg::kStages) - 1) & 1, 0x800);
-        }
-        load_step(i);
+        if (i >= Cfg::kQStages) { B200FA_WAIT(&q_empty[i % Cfg::kQStages], ((i / Cfg::kQStages) - 1) & 1, 0x800); }
+        load_q(i);
+        if (i >= Cfg::kDoStages) { B200FA_WAIT(&do_empty[i % Cfg::kDoStages], ((i / Cfg::kDoStages) - 1) & 1, 0x801); }
+        load_do(i);
+        if (i >= 2) { B200FA_WAIT(&stat_empty[i & 1], ((i >> 1) - 1) & 1, 0x802); }
+        load_stat(i);
       }
     }
   }
@@ -499,7 +489,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
   // the tensor pipe within the shared-memory budget.
   uint8_t* sQ = smem + Cfg::kOffResident;
   uint8_t* sDO = sQ + Cfg::kTileBytes;
-  uint8_t* sK = smem + Cfg::kOffStream;                       // [3] tiles
+  uint8_t* sK = smem + 2 * Cfg::kTileBytes;                   // [3] tiles
   uint8_t* sV = sK + 3 * Cfg::kTileBytes;                     // [2] tiles
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffDqBars);
   uint64_t* q_full = bars;                         // [1]  Q tile
