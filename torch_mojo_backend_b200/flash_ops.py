@@ -43,11 +43,11 @@ def _decode_shaped(batch: int, heads_q: int, heads_kv: int, seq_q: int, seq_k: i
     return seq_k >= _SPLITKV_MIN_KEYS and rows <= _lib.SPLITKV_MAX_ROWS
 
 
-def _log(msg: str) -> None:
+def _log(msg: str, *values) -> None:
     """B200FA_LOG=1 prints one line per native call (the reference gates its eager logging the
     same way, torch_mojo_backend/flags.py:6-33)."""
     if os.environ.get("B200FA_LOG", "0") not in ("", "0"):
-        print(f"[b200fa] {msg}", flush=True)
+        print("[b200fa] " + msg % values, flush=True)
 
 
 def _stream_for(index: int) -> int:
@@ -228,18 +228,34 @@ def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is
     if not dropout_p and _decode_shaped(batch, heads_q, heads_kv, seq, seq_k):
         nbytes = _lib.fwd_splitkv_workspace_bytes(batch, heads_q, heads_kv, seq, seq_k, head_dim, **piece)
         workspace = tensor._alloc_holder(nbytes, index)
-        _log(f"fwd_splitkv B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={seq_k} D={head_dim}")
+        _log("fwd_splitkv B=%d Hq=%d Hkv=%d Sq=%d Sk=%d D=%d", batch, heads_q, heads_kv, seq, seq_k, head_dim)
         rc = _lib.fwd_splitkv(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, workspace.data_ptr(), nbytes,
                               code, bool(is_causal), float(scale), _stream_for(index), index, _status_ptr(index),
                               **piece)
         _check(rc, "b200fa_fwd_splitkv")
         CALL_COUNTERS["forward_split_kv"] += 1
         return out, lse, q_used, k_used, v_used
-    _log(f"fwd B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={seq_k} D={head_dim} causal={is_causal} p={dropout_p}")
+    _log("fwd B=%d Hq=%d Hkv=%d Sq=%d Sk=%d D=%d causal=%s p=%s", batch, heads_q, heads_kv, seq, seq_k, head_dim, is_causal,
+         dropout_p)
     rc = _lib.fwd(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, code, bool(is_causal), float(scale),
                   _stream_for(index), index, _status_ptr(index), dropout=_dropout_arg(dropout_p, philox), **piece)
     _check(rc, "b200fa_fwd")
     return out, lse, q_used, k_used, v_used
+
+
+def forward_with_its_own_mask(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, dropout_p: float,
+                              is_causal: bool, scale: float | None):
+    """``(out, lse, (seed, offset))`` of inputs that ``flash_inputs`` has accepted; the Philox state the dropout mask
+    is drawn from is reserved here."""
+    CALL_COUNTERS["aten::_scaled_dot_product_flash_attention"] += 1
+    dropout_p = float(dropout_p)
+    philox = (0, 0)
+    if dropout_p:
+        if q._holder.is_cuda and torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("mojo attention with dropout cannot be captured: every replay would draw the same mask")
+        philox = device_module._reserve_philox_state(q._device_index, q._shape[0] * q._shape[1])
+    out, lse, _, _, _ = flash_forward(q, k, v, is_causal, scale, dropout_p, philox)
+    return out, lse, philox
 
 
 def scaled_dot_product_flash_attention(query, key, value, dropout_p=0.0, is_causal=False,
@@ -264,18 +280,15 @@ def scaled_dot_product_flash_attention(query, key, value, dropout_p=0.0, is_caus
             "head_dim 64 or 128, Hq % Hkv == 0, 0 <= dropout_p < 1 and a positive finite scale"
         )
     q, k, v = inputs
-    CALL_COUNTERS["aten::_scaled_dot_product_flash_attention"] += 1
     index = q._device_index
-    dropout_p = float(dropout_p)
-    seed = offset = 0
-    if dropout_p:
-        seed, offset = device_module._reserve_philox_state(index, q._shape[0] * q._shape[1])
-    out, lse, _, _, _ = flash_forward(q, k, v, is_causal, scale, dropout_p, (seed, offset))
+    out, lse, (seed, offset) = forward_with_its_own_mask(q, k, v, dropout_p, is_causal, scale)
     rng_state = TorchMojoTensor._alloc((2,), torch.uint64, index)
-    if dropout_p:
-        # the pair as two signed 64-bit patterns (uint64 copies are not universally supported)
-        host = torch.tensor([seed, offset], dtype=torch.uint64).view(torch.int64)
-        rng_state._cuda_view().view(torch.int64).copy_(host)
+    if float(dropout_p):
+        # the pair as two signed 64-bit patterns (uint64 fills are not universally supported), by two fills: a copy from
+        # host memory waits for all that the stream still has to do
+        words = rng_state._cuda_view().view(torch.int64)
+        for word, value in zip(words, (seed, offset)):
+            word.fill_(value - (1 << 64) if value >> 63 else value)
     rng_state._philox = (seed, offset)   # host-side copy: the backward needs no read-back
     unused = TorchMojoTensor._alloc((), torch.uint64, index)
     debug_attn_mask = TorchMojoTensor._alloc((0,), q._dtype, index)
@@ -300,7 +313,8 @@ def flash_backward(dout, q, k, v, out, lse, is_causal: bool, scale: float, dropo
     code = _DTYPE_CODES[q._dtype]
     nbytes = _lib.bwd_workspace_bytes(batch, heads_q, heads_kv, seq, head_dim, code)
     workspace = tensor._alloc_holder(nbytes, index)
-    _log(f"bwd B={batch} Hq={heads_q} Hkv={heads_kv} Sq={seq} Sk={k._shape[2]} D={head_dim} causal={is_causal} p={dropout_p}")
+    _log("bwd B=%d Hq=%d Hkv=%d Sq=%d Sk=%d D=%d causal=%s p=%s", batch, heads_q, heads_kv, seq, k._shape[2], head_dim,
+         is_causal, dropout_p)
     rc = _lib.bwd(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out_used), _t4(dout_used), lse_used._ptr,
                   _t4(dq), _t4(dk), _t4(dv), workspace.data_ptr(), nbytes, code, bool(is_causal), float(scale),
                   _stream_for(index), index, _status_ptr(index), dropout=_dropout_arg(dropout_p, philox))

@@ -19,6 +19,7 @@ import torch
 from . import device_module
 
 _WRAPPER_DEVICE = torch.device("privateuseone", 0)
+_make_wrapper_subclass = torch.Tensor._make_wrapper_subclass
 _mojo_devices: dict[int, torch.device] = {}
 _cuda_devices: dict[int, torch.device] = {}
 
@@ -90,7 +91,7 @@ def pinned_empty(shape, dtype: torch.dtype) -> torch.Tensor:
 
 def _alloc_holder(nbytes: int, index: int) -> torch.Tensor:
     """One device allocation: a flat byte buffer on CUDA device `index` (never zero bytes)."""
-    return torch.empty((max(int(nbytes), 1),), dtype=torch.uint8, device=_cuda_device(index))
+    return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=_cuda_device(index))
 
 
 def _holder_ptr(holder: torch.Tensor) -> int:
@@ -126,16 +127,7 @@ class TorchMojoTensor(torch.Tensor):
     @classmethod
     def _wrap(cls, holder, ptr, shape, strides, offset, dtype, index, contiguous) -> "TorchMojoTensor":
         """`_make` with every argument already in its final form (ints, tuples of ints)."""
-        res = torch.Tensor._make_wrapper_subclass(
-            cls,
-            shape,
-            strides=strides,
-            storage_offset=offset,
-            dtype=dtype,
-            layout=torch.strided,
-            device=_WRAPPER_DEVICE,
-            requires_grad=False,
-        )
+        res = _make_wrapper_subclass(cls, shape, strides, offset, dtype=dtype, device=_WRAPPER_DEVICE)
         res.__dict__.update(
             _holder=holder,
             _ptr=ptr,
