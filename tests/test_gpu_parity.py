@@ -144,6 +144,24 @@ def test_backward_over_every_fill_of_its_rings(D, group, Sq, causal, p):
         assert parity_report(name, got[name], want[name], tol_for(dtype), dtype, ref_is_rounded=True)["over_widened"] == 0
 
 
+@pytest.mark.parametrize("D,S,causal", [(64, 700, True), (64, 3900, True), (64, 1000, False), (128, 700, True)])
+def test_backward_has_the_same_bits_whichever_warp_is_first(D, S, causal):
+    """Thread blocks of few steps, many times over: the compute warps of a block drift apart by up to a step."""
+    g = torch.Generator().manual_seed(S)
+    draw = lambda h: torch.randn(2, h, S, D, generator=g).half().cuda()
+    q, k, v, dout = draw(4), draw(2), draw(2), draw(4)
+    out, lse = raw.flash_fwd(q, k, v, causal=causal)
+    want = raw.flash_bwd(dout, q, k, v, out, lse, causal=causal)
+    simt = raw.flash_bwd(dout, q, k, v, out, lse, causal=causal, simt=True)
+    for name, w, s in zip(("dq", "dk", "dv"), want, simt):
+        assert parity_report(name, w, s, tol_for(q.dtype), q.dtype, ref_is_rounded=True)["over_widened"] == 0
+    differ = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(4000 if S < 2000 else 800):
+        for w, x in zip(want, raw.flash_bwd(dout, q, k, v, out, lse, causal=causal)):
+            differ += (w.view(torch.int16) != x.view(torch.int16)).sum()
+    assert int(differ) == 0
+
+
 def test_randomised_shapes_agree_with_the_exact_fp32_kernels():
     """A seeded sweep over ragged lengths, GQA groups, head dims, dtypes, masks and (when
     unmasked) unequal key lengths: the tensor-core kernels against the exact-fp32 SIMT kernels

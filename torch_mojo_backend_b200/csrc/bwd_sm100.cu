@@ -47,7 +47,7 @@ struct BwdCfg {
   static constexpr int kOffDo = kOffQ + kQStages * kTileBytes;
   static constexpr int kOffStat = kOffDo + kDoStages * kTileBytes;        // [step & 1][lse2|dpsum][128] fp32
   static constexpr int kOffBars = kOffStat + 2 * 2 * 128 * 4;
-  static constexpr int kNumBars = 2 * kQStages + 2 * kDoStages + 14;
+  static constexpr int kNumBars = 2 * kQStages + 2 * kDoStages + 15;
   // the dQ kernel keeps 2 resident + 3 K + 2 V tiles and no per-stage statistics
   static constexpr int kOffDqBars = 7 * kTileBytes;
   static constexpr int kSmemBytes =
@@ -98,8 +98,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint64_t* s_full = stat_empty + 2;               // [2]  S^T ready in work buffer b
   uint64_t* dp_full = s_full + 2;                  // dP^T ready
   uint64_t* dp_free = dp_full + 1;                 // dP^T read into registers (16 warp arrivals)
-  uint64_t* p_full = dp_free + 1;                  // P^T written  (16 warp arrivals)
-  uint64_t* ds_full = p_full + 1;                  // dS^T written (16 warp arrivals)
+  uint64_t* p_full = dp_free + 1;                  // [2]  P^T of step i written (16 warp arrivals; two, since at D = 64 a
+                                                   //      warp may be done with P^T of the next step before another arrives)
+  uint64_t* ds_full = p_full + 2;                  // dS^T written (16 warp arrivals)
   uint64_t* acc_full = ds_full + 1;                // dK, dV complete
   uint64_t* staged = acc_full + 1;                 // dV and dK tiles staged in shared memory (16 warp arrivals)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
@@ -182,10 +183,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       mbar_init(&stat_full[i], 1);
       mbar_init(&stat_empty[i], 1);
       mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 16);   // one elected arrival per compute warp
     }
     mbar_init(dp_full, 1);
-    mbar_init(dp_free, 16);   // one elected arrival per compute warp
-    mbar_init(p_full, 16);
+    mbar_init(dp_free, 16);
     mbar_init(ds_full, 16);
     mbar_init(acc_full, 1);
     mbar_init(staged, 16);
@@ -274,7 +275,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive_warp(p_full);
+      mbar_arrive_warp(&p_full[i & 1]);
       // ---- dS^T = P^T * (dP^T - dpsum)
       B200FA_WAIT(dp_full, i & 1, 0x510);
       tc_fence_after();
@@ -428,7 +429,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         B200FA_WAIT_WARP(dp_free, i & 1, 0x717);
         B200FA_ISSUE_S(i + 1);
       }
-      B200FA_WAIT_WARP(p_full, i & 1, 0x710);
+      B200FA_WAIT_WARP(&p_full[i & 1], (i >> 1) & 1, 0x710);
       tc_fence_after();
       issue_acc(tDV, tS, mDO, do_stage * kTileLo, i == 0);          // dV += P^T dO
       umma_commit_elect(&do_empty[do_stage]);
