@@ -102,11 +102,8 @@ size_t b200fa_bwd_workspace_bytes(int64_t batch, int64_t heads_q, int64_t heads_
  * bytes, 256-byte aligned; its contents on entry are irrelevant (the library clears what it
  * needs on `stream`).
  * Everything is ordered on `stream`: work enqueued before the call is seen, work enqueued
- * after it sees dq, dk and dv.  For causal 16-bit problems one of the kernels runs on a side
- * stream of a small per-device pool the library keeps (picked by the value of `stream`), forked
- * from and joined back into `stream` with events (this also works inside stream capture); a
- * side stream and its two events are created at the first call that picks them, so make that
- * call outside capture.
+ * after it sees dq, dk and dv.  The kernels of one call may overlap (programmatic launches on
+ * `stream`, also inside stream capture); the last of them ends after all of them.
  * Replaces flash_attention_bwd_<dtype>_d<D>_causal{,_strided_qkv}
  * (torch_mojo_backend/eager_flash_attention/fa4_ops.mojo:158-226).
  */

@@ -135,9 +135,13 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
   // A launch whose status word already reports a failed wait is not worth running; the swizzled
   // tiles assume a 1024-byte aligned shared-memory window.
-  if (status_is_set(p.status)) return;
+  if (status_is_set(p.status)) {
+    cudaGridDependencySynchronize();   // (no kernel of a backward ends before the ones launched ahead of it)
+    return;
+  }
   if ((smem_u32(smem) & 1023u) != 0u) {
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, kStatusOk, 0x414c0000u);
+    cudaGridDependencySynchronize();
     return;
   }
   // Lane 0 of the producer warp sets up the barriers and at once issues the loads the first MMAs
@@ -197,11 +201,15 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     load_tile(&mapK, sK, k_full, n0, hk);
     if (steps > 0) {
       load_q(0);
-      load_stat(0);
       load_do(0);
     }
     mbar_arrive_expect_tx(v_full, Cfg::kTileBytes);
     load_tile(&mapV, sV, v_full, n0, hk);
+    // This kernel may have started before the preprocess kernel was done; only the row statistics come from that one.
+    // Once every block has them in reach the dQ kernel may start.
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (steps > 0) load_stat(0);
   }
   if (warp == 16) {
     tmem_alloc(tmem_slot, 512);
@@ -524,9 +532,16 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
     n_tiles = last < 0 ? 0 : min(nkv_total, last / kTile + 1);
   }
 
-  if (status_is_set(p.status)) return;
+  // This kernel may have started beside the dK/dV kernel.  It still ends after it: its last block waits for that, so
+  // that what is ordered behind this kernel is ordered behind both.
+  const bool last_block = blockIdx.x + 1 == gridDim.x && blockIdx.y + 1 == gridDim.y && blockIdx.z + 1 == gridDim.z;
+  if (status_is_set(p.status)) {
+    if (last_block) cudaGridDependencySynchronize();
+    return;
+  }
   if ((smem_u32(smem) & 1023u) != 0u) {
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, kStatusOk, 0x414c0001u);
+    if (last_block) cudaGridDependencySynchronize();
     return;
   }
   // Lane 0 of the producer warp sets up the barriers and at once issues the loads the first MMAs
@@ -806,6 +821,7 @@ teardown:
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  if (last_block) cudaGridDependencySynchronize();
 }
 #undef B200FA_WAIT
 #undef B200FA_WAIT_WARP
@@ -829,6 +845,7 @@ struct PreCfg {
 template <int kD, bool kBf16>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const BwdParams p) {
   using Cfg = PreCfg<kD>;
+  cudaTriggerProgrammaticLaunchCompletion();
   const int lane = threadIdx.x & 31;
   const int li = lane % Cfg::kLanesPerRow;
   const int per_head = p.Spad / Cfg::kBlockRows;
@@ -885,38 +902,6 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const BwdParams p) 
   }
 }
 
-// The dK/dV kernel and the dQ kernel only depend on the preprocess kernel, not on each other.
-// Run back to back on one stream, the second cannot start until the last, partly idle wave of
-// the first has drained; forked onto a side stream its CTAs fill those SMs as they free up.
-// Every device owns a small pool of side streams, each with a fork/join event pair, created on
-// first use and kept until the process exits; the caller's stream handle picks the pool entry,
-// so backward passes issued on different streams do not queue behind one another.  The mutex
-// covers one call's record / wait / launch / record / wait sequence on an entry.
-struct SideStream {
-  cudaStream_t stream = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-  bool tried = false;
-  std::mutex mutex;
-};
-constexpr int kSidePool = 4;
-SideStream* side_stream_for(int dev, cudaStream_t caller) {
-  static SideStream pool[64][kSidePool];
-  if (dev < 0 || dev >= 64) return nullptr;
-  const uintptr_t h = reinterpret_cast<uintptr_t>(caller);
-  SideStream& s = pool[dev][(h >> 4 ^ h >> 12) % kSidePool];
-  std::lock_guard<std::mutex> lock(s.mutex);
-  if (!s.tried) {
-    s.tried = true;
-    if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) != cudaSuccess) {
-      cudaGetLastError();
-      s.stream = nullptr;
-    }
-  }
-  return s.stream ? &s : nullptr;
-}
-
 // cudaFuncSetAttribute for one kernel, once per device, safe against concurrent first calls.
 // `once` and `result` belong to the kernel (the caller keeps them as statics of the function
 // template that names it: kernels of the same signature must not share them).
@@ -950,21 +935,8 @@ cudaError_t launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUten
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  int dev = 0;
-  cudaGetDevice(&dev);
   const int tiles = (p.S + kTile - 1) / kTile;        // query tiles: the dQ kernel's grid
   const int kv_tiles = (p.Sk + kTile - 1) / kTile;    // K/V tiles: the dK/dV kernel's grid
-  // fork: the dQ kernel goes to the side stream, behind everything enqueued so far.  Only
-  // causal problems: their CTAs differ in length, which is what leaves a long partly idle tail;
-  // with equal CTAs the tail is short and interleaving the two kernels only costs L2 hits.
-  SideStream* side = (kCausal && (p.parts & 6) == 6 && !(p.parts & 8)) ? side_stream_for(dev, stream) : nullptr;
-  std::unique_lock<std::mutex> side_lock;
-  if (side) {
-    side_lock = std::unique_lock<std::mutex>(side->mutex);
-    e = cudaEventRecord(side->fork, stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(side->stream, side->fork, 0);
-    if (e != cudaSuccess) return e;   // nothing has been enqueued on the side stream yet
-  }
   if (p.parts & 2) {
     // (batch, kv head) pairs whose streamed Q / dO rows (both, all query heads of the pair)
     // add up to about 48 MiB share a scheduling group
@@ -973,20 +945,15 @@ cudaError_t launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUten
     const int64_t pairs = static_cast<int64_t>(p.B) * p.Hkv;
     if (sched_group < 1) sched_group = 1;
     if (sched_group > pairs) sched_group = pairs;
-    k1<<<static_cast<unsigned>(kv_tiles * pairs), kDkdvThreads, Cfg::kSmemBytes, stream>>>(
-        mq, mk, mv, mdo, mdk, mdv, p, static_cast<int>(sched_group));
-    e = cudaGetLastError();
+    e = launch_early(k1, dim3(static_cast<unsigned>(kv_tiles * pairs)), kDkdvThreads, Cfg::kSmemBytes, stream, (p.parts & 1) != 0,
+                     mq, mk, mv, mdo, mdk, mdv, p, static_cast<int>(sched_group));
   }
   if (e == cudaSuccess && (p.parts & 4)) {
-    k2<<<dim3(tiles, p.Hq, p.B), kThreads, Cfg::kSmemBytes, side ? side->stream : stream>>>(mq, mk, mv, mdo, mdq, p);
-    e = cudaGetLastError();
-  }
-  if (side) {
-    // join, whatever happened in between: once the side stream has been made to wait on the
-    // caller's stream it must flow back into it (a stream capture would otherwise stay forked)
-    cudaError_t e2 = cudaEventRecord(side->join, side->stream);
-    if (e2 == cudaSuccess) e2 = cudaStreamWaitEvent(stream, side->join, 0);
-    if (e == cudaSuccess) e = e2;
+    // The dQ kernel does not need the dK/dV kernel's results, only the row statistics, and fills the SMs that the last
+    // blocks of that one leave idle.  B200, us, whole backward with the dQ kernel on a side stream behind events / each
+    // kernel launched to start early: B1 H8 S512 D128 bf16 causal 30 / 23.5, B16 H8 S1000x77 D64 fp16 55 / 48, B2 H16 S1024
+    // D128 51.6 / 47.7, B4 Hq32 Hkv8 S4096 D128 1494 / 1485, B8 H16 S2048 D128 unmasked (one after the other) 815 / 806.
+    e = launch_early(k2, dim3(tiles, p.Hq, p.B), kThreads, Cfg::kSmemBytes, stream, (p.parts & 2) != 0, mq, mk, mv, mdo, mdq, p);
   }
   return e;
 }

@@ -50,8 +50,7 @@ struct BwdParams {
   float scale_log2;
   uint32_t* status;
   long long wait_budget;
-  int parts;  // bit 0 preprocess, bit 1 dK/dV kernel, bit 2 dQ kernel (7 = the whole backward);
-              // bit 3: keep every kernel on the caller's stream (no side stream, nothing created)
+  int parts;  // bit 0 preprocess, bit 1 dK/dV kernel, bit 2 dQ kernel (7 = the whole backward)
   DropoutParams drop;
 };
 
@@ -84,6 +83,22 @@ cudaError_t launch_bwd_simt(const BwdParams& p, int dtype, cudaStream_t stream, 
 // A one-warp kernel whose only job is to wait, with `budget` SM cycles, on a barrier nobody
 // arrives at: exercises the bounded-wait give-up path without touching the attention kernels.
 cudaError_t launch_wait_timeout_selftest(uint32_t* status, long long budget, cudaStream_t stream, int* launches);
+
+// A launch that, if `early`, may start as soon as every block of the kernel ahead of it on the stream has allowed it.
+template <typename... Params, typename... Args>
+cudaError_t launch_early(void (*kern)(Params...), dim3 grid, int threads, int smem, cudaStream_t stream, bool early, Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
 
 // Encodes a 4-D tiled tensor map over a (B,H,S,D) view of 16-bit elements with a
 // {64 x box_rows x 1 x 1} box and 128-byte swizzle.  Returns false if the driver entry

@@ -1031,6 +1031,8 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
     };
     float4 vq[8], vd[8];
     if (n > 0) load_box(vq, p.q, b, h, m0, p.S, 0, tid);
+    cudaGridDependencySynchronize();   // dpsum
+    cudaTriggerProgrammaticLaunchCompletion();
     for (int j = 0; j < n; ++j) {
       load_box(vd, p.dout, b, h, m0, p.S, 0, tid);
       float nl2 = -INFINITY, ndps = 0.f;   // rows past the end, and rows that saw no key: P = 0
@@ -1104,16 +1106,20 @@ teardown:
     tmem_dealloc(tmem_base, 512);
   }
 }
-// The dQ kernel does not need the dK/dV kernel's results: it is launched to start as soon as every block of that
-// one has (each says so at once), and fills the SMs that its last blocks leave idle.  It still ends after it: block 0
-// waits for that, so that what is ordered behind the dQ kernel is ordered behind both.
+// The dK/dV kernel is launched to start when every block of the dpsum kernel has, and needs that one's results with the
+// first tile's statistics.  The dQ kernel does not need the dK/dV kernel's results: it is launched to start as soon as
+// every block of that one has seen the dpsum kernel end, and fills the SMs that its last blocks leave idle.  It still ends
+// after it: block 0 waits for that, so that what is ordered behind the dQ kernel is ordered behind both.
 template <int kD, bool kDropout>
 __global__ void __launch_bounds__(kThreads, 1) bwd_dkdv_fp32_kernel(const __grid_constant__ BwdParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  cudaTriggerProgrammaticLaunchCompletion();
-  if (status_is_set(p.status)) return;
+  if (status_is_set(p.status)) {
+    cudaGridDependencySynchronize();   // (no kernel of a backward ends before the ones launched ahead of it)
+    return;
+  }
   if ((smem_u32(smem) & 1023u) != 0u) {
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, kStatusOk, 0x414c0003u);
+    cudaGridDependencySynchronize();
     return;
   }
   dkdv_block<kD, kDropout>(p, static_cast<int>(blockIdx.x), smem);
@@ -1142,6 +1148,7 @@ struct PreF32Cfg {
 template <int kD>
 __global__ void __launch_bounds__(256) dpsum_fp32_kernel(const BwdParams p) {
   using Cfg = PreF32Cfg<kD>;
+  cudaTriggerProgrammaticLaunchCompletion();
   const int lane = threadIdx.x & 31, li = lane % Cfg::kLanes;
   const int per_head = (p.S + Cfg::kBlockRows - 1) / Cfg::kBlockRows;
   const int bh = static_cast<int>(blockIdx.x) / per_head, b = bh / p.Hq, h = bh - b * p.Hq;
@@ -1206,19 +1213,9 @@ cudaError_t launch_bwd(const BwdParams& p, cudaStream_t stream) {
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const int64_t kv_blocks = static_cast<int64_t>(p.B) * p.Hkv * ((p.Sk + kBM - 1) / kBM);
   const int64_t q_blocks = static_cast<int64_t>(p.B) * p.Hq * ((p.S + kBM - 1) / kBM);
-  k1<<<static_cast<unsigned>(kv_blocks), kThreads, DkdvF32Cfg<kD>::kSmemBytes, stream>>>(p);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  cudaLaunchAttribute early;
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(q_blocks));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = DqF32Cfg<kD>::kSmemBytes;
-  cfg.stream = stream;
-  cfg.attrs = &early;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k2, p);
+  e = launch_early(k1, dim3(static_cast<unsigned>(kv_blocks)), kThreads, DkdvF32Cfg<kD>::kSmemBytes, stream, true, p);
+  if (e != cudaSuccess) return e;
+  return launch_early(k2, dim3(static_cast<unsigned>(q_blocks)), kThreads, DqF32Cfg<kD>::kSmemBytes, stream, true, p);
 }
 
 // Few keys: the fp32 FMA kernels have less to set up and smaller tiles.
