@@ -257,6 +257,23 @@ def test_split_kv_decode_forward_matches_oracle_and_prefill_kernel(dtype, B, Hq,
     assert torch.equal(out_t, out) and torch.equal(lse_t, lse)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,D", [(1, 1, 1, 1, 64), (1, 4, 1, 3, 128), (3, 10, 2, 3, 64), (19, 16, 8, 5, 128), (57, 1, 1, 2, 128)])
+def test_split_kv_merges_as_a_cluster_or_through_the_workspace(dtype, B, Hq, Hkv, Sq, D):
+    """One split, clusters of 2 to 16 of them, and more splits or more clusters than that: the same numbers as the exact-fp32
+    forward within the contract's tolerance, and the same bits whichever piece of a batch they are computed for."""
+    for Sk in (500, 512, 700, 1100, 1900, 2304, 4000, 4400, 9000):
+        if B * Hkv * Sk > 400000:
+            continue
+        q, k, v, _ = (t.cuda() for t in draw(dtype, B, Hq, Hkv, Sq, Sk, D, 31 + Sk))
+        out, lse = raw.flash_fwd_splitkv(q, k, v, causal=2)
+        ref_out, ref_lse = raw.flash_fwd(q, k, v, causal=2, simt=True)
+        assert_within("out", out, ref_out.float(), tol_for(dtype), dtype)
+        assert_within("lse", lse, ref_lse, TOL_LSE)
+        part_out, part_lse = raw.flash_fwd_splitkv(q[:1], k[:1], v[:1], causal=2, whole_heads=B * Hq)
+        assert torch.equal(part_out, out[:1]) and torch.equal(part_lse, lse[:1])
+
+
 DROPOUT = [
     # dtype, B, Hq, Hkv, Sq, Sk, D, mode, p
     (torch.bfloat16, 2, 4, 2, 256, 256, 128, 1, 0.1),

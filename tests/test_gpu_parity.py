@@ -466,7 +466,7 @@ def test_forward_and_backward_replay_from_a_cuda_graph():
     q, k, v, do = rand_case(torch.bfloat16, 1, 8, 4, 512, 128, seed=12)
     qc, kc, vc, doc = q.cuda(), k.cuda(), v.cuda(), do.cuda()
     out, lse = raw.flash_fwd(qc, kc, vc, causal=True)
-    eager = raw.flash_bwd(doc, qc, kc, vc, out, lse, causal=True) 
+    eager = raw.flash_bwd(doc, qc, kc, vc, out, lse, causal=True)
     torch.cuda.synchronize()
     g_out, g_lse = torch.empty_like(out), torch.empty_like(lse)
     g_dq, g_dk, g_dv = (torch.empty_like(t) for t in eager)

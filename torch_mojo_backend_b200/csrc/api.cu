@@ -338,25 +338,26 @@ int bwd_impl(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tens
   return e == cudaSuccess ? B200FA_OK : B200FA_ERR_CUDA;
 }
 
-// Key splits of the split-KV forward: the count up to 64, of at least 256 keys each, that the model
+// Splits of the split-KV forward: the count up to 64, of at least 256 keys each, that the model
 // below finds cheapest; the first found wins a tie, which is the one with fewer splits.
 // The grid runs in waves of the CTAs that fit: by registers, 3 and 2 per SM of the 16-bit kernel at
 // D = 128 (up to 8 query rows per KV head, and more), 4 and 3 at D = 64; 2 and 1 of the fp32 kernel (up
 // to 4 rows, and more).  A wave costs its keys and a fixed part worth some 48 KB of them (192 keys of 16 bits
-// and D = 128: prologue, merge of the warps, the partial written and combined); 16-bit keys of D = 64 are so
-// narrow that a split more costs another 16 (its partials are read once more).  A wave that is not full
-// gives each of its CTAs more of HBM, until about 0.85 of the CTAs that fit saturate it.
-// Measured (us, B200; before = every wave taken as full, 3 or 2 CTAs per SM whatever the type and D):
-//   B8 Hq32 Hkv8 Sk32768 D128 bf16     170 -> 165 (6 splits)     16 rows: B16 Hq32 Hkv8 Sq4 Sk16384  193 -> 182 (2)
-//   16 rows, D64: B8 Hkv8 Sk8000 fp16  44.4 -> 34.9 (6)          fp32: B8 Hkv8 Sk8192 D128 4 rows    121 -> 95 (4)
-//   fp32: B4 Hkv2 Sk5000 D64 16 rows   47.2 -> 30.8 (16)         fp32: B4 Hkv12 Sk9000 D64 1 row     51.2 -> 43.9 (6)
-// With 192 keys for every width, calls of many short caches of D = 64 took a split and a wave too many: 360 KV
-// heads of 8 rows over 1536 keys 38.5 us in 3 splits, 34.9 in 1; 336 of 6 over 1236 31.6 and 29.4; 224 of 12 over
-// 1208 28.8 and 26.7.
+// and D = 128: prologue, merge of the warps); a split costs 2 KB more, and a merge through the workspace, where the
+// splits do not form a cluster, some 3 us (clearing the counters, the fences, the partials' way through L2): 64 KB of
+// keys while HBM is idle, half that when it is not.  A wave
+// that is not full gives each of its CTAs more of HBM, until about 0.85 of the CTAs that fit saturate it.
+// Clusters do not cross a GPC: what fits at once is counted as seven of 18 SMs and one of 13 (the launcher asks the device;
+// a wrong guess here costs time, not results).
+// Over 1179 random calls (1-900 KV heads, 512-131072 keys, 1-16 rows, all types) the choice takes 2.6 % more time than each
+// call's best count, in 85 of them over 10 % more; a rule that does not count the merge 5.7 %, in 237.
+// B200, us, such a rule / this: B1 Hq32 Hkv8 Sk4250 D128 bf16 15.4 / 12.5 (17 / 16 splits), B8 Hq16 Hkv4 Sq4 Sk7233
+// 33 / 28 (9 / 8), B2 Hq32 Hkv8 Sq4 Sk7698 25 / 21.5 (18 / 12).
 // `kv_heads`: batch * KV heads, of the whole problem if the call computes a piece of one.
 int splitkv_splits(int64_t kv_heads, int64_t rows, int64_t Sk, int64_t D, bool fp32, int* split_len) {
   const int64_t per_sm = fp32 ? (rows <= 4 ? 2 : 1) : D == 64 ? (rows <= 8 ? 4 : 3) : (rows <= 8 ? 3 : 2);
-  const int64_t slots = per_sm * 148, fixed = 192 * 256 / (D * (fp32 ? 4 : 2)), each = !fp32 && D == 64 ? 16 : 0;
+  const int64_t slots = per_sm * 148;
+  const double unit = 256.0 / (D * (fp32 ? 4 : 2)), fixed = 192 * unit;   // in keys; unit: 256 bytes of them
   int64_t max_n = (Sk + 255) / 256;
   if (max_n > 64) max_n = 64;
   if (max_n < 1) max_n = 1;
@@ -366,8 +367,11 @@ int splitkv_splits(int64_t kv_heads, int64_t rows, int64_t Sk, int64_t D, bool f
     const int64_t len = ((Sk + cand - 1) / cand + 63) / 64 * 64;
     const int64_t n = (Sk + len - 1) / len;
     const int64_t full = kv_heads * n / slots, rest = kv_heads * n % slots;
-    double cost = static_cast<double>(full) * (len + fixed) + static_cast<double>(each) * n;
+    const int64_t clusters = n <= 2 ? slots / 2 : 7 * (18 * per_sm / n) + 13 * per_sm / n;
+    double cost = full * (len + fixed) + 8 * unit * n;
     if (rest > 0) cost += len * std::max(0.85, static_cast<double>(rest) / slots) + fixed;
+    if (n > 1 && (n > kSplitkvCluster || kv_heads > clusters))
+      cost += 256 * unit * (1.0 - 0.5 * std::min(1.0, static_cast<double>(kv_heads * n) / slots));
     if (best_cost < 0.0 || cost < best_cost) {
       best_cost = cost;
       best_n = n;

@@ -67,6 +67,8 @@ struct SplitKvParams {
   float scale, scale_log2;
 };
 
+constexpr int kSplitkvCluster = 16;   // splits of a KV head that may merge as a cluster
+
 // dtype tags shared with the C header
 constexpr int kF32 = 0, kBF16 = 1, kF16 = 2;
 

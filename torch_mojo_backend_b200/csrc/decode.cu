@@ -23,11 +23,15 @@
 //     by shuffles for O += P V.  About 90 instructions per key and warp at 4 rows: the schedulers, not
 //     HBM, bound it (measured with 16-bit inputs before the tensor-core form existed: 0.55 of the copy
 //     rate, issue slots 59 % busy).
-// The merge (finish_split): one warp per output row combines the splits, writes out and lse.
+// The merge: finish_in_cluster where the splits of a KV head form a cluster (launch_splits says when), else finish_split,
+// through global memory.  Both add the splits up in the same order: the same bits.
+#include <atomic>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace b200fa {
 namespace {
@@ -35,6 +39,8 @@ namespace {
 constexpr int kKeyBlock = 8;        // keys per step of a warp
 constexpr int kWarpsDecode = 8;
 constexpr int kThreadsDecode = kWarpsDecode * 32;
+constexpr int kMaxCluster = kSplitkvCluster;   // splits that may merge as a cluster (more than 8 is not portable, but sm_100 has it)
+constexpr int kMaxRows = 16;
 
 template <typename T>
 __device__ __forceinline__ T st_f32(float x);
@@ -145,11 +151,58 @@ __device__ __forceinline__ void finish_split(const SplitKvParams& p, int b, int 
   if (part == 0) p.lse[row] = l > 0.f ? m * 0.6931471805599453f + logf(l) : -INFINITY;
 }
 
+// The merge by a cluster of the KV head's splits: every CTA has left its unnormalised O of row rr at
+// o + ((rr / row_tile) * tile_stride + rr % row_tile) * (kD + 2) floats and the row's (max, sum) at ml + rr, and merges its
+// share of (row, pair of elements) from its peers' shared memory.  No workspace, no counters to clear, no fences.
+template <typename T, int kD>
+__device__ __forceinline__ void finish_in_cluster(const SplitKvParams& p, int b, int hk, int rows, int tid, int nthreads,
+                                                  const float* o, int row_tile, int tile_stride, const float2* ml) {
+  cluster_sync();
+  const int group = p.Hq / p.Hkv;
+  for (int idx = static_cast<int>(blockIdx.x) * nthreads + tid; idx < rows * (kD / 2); idx += p.nsplit * nthreads) {
+    const int rr = idx / (kD / 2), d = idx % (kD / 2) * 2;
+    const uint32_t a_ml = smem_u32(ml + rr);
+    const uint32_t a_o = smem_u32(o + ((rr / row_tile) * tile_stride + rr % row_tile) * (kD + 2) + d);
+    float2 v[kMaxCluster], x[kMaxCluster];
+#pragma unroll
+    for (int sp = 0; sp < kMaxCluster; ++sp) {
+      if (sp < p.nsplit) {
+        v[sp] = peer_load_f32x2(a_ml, sp);
+        x[sp] = peer_load_f32x2(a_o, sp);
+      }
+    }
+    float m = -INFINITY, l = 0.f, o0 = 0.f, o1 = 0.f;
+#pragma unroll
+    for (int sp = 0; sp < kMaxCluster; ++sp) {
+      if (sp < p.nsplit) m = fmaxf(m, v[sp].x);
+    }
+    const float m_use = (m == -INFINITY) ? 0.f : m;
+#pragma unroll
+    for (int sp = 0; sp < kMaxCluster; ++sp) {
+      if (sp < p.nsplit) {
+        const float w = exp2f(v[sp].x - m_use);   // 0 for a split that saw no visible key
+        l = fmaf(v[sp].y, w, l);
+        o0 = fmaf(x[sp].x, w, o0);
+        o1 = fmaf(x[sp].y, w, o1);
+      }
+    }
+    const float inv = l > 0.f ? 1.f / l : 0.f;   // a row that saw no key at all: 0 with lse -inf
+    const int h = hk * group + rr / p.Sq, qi = rr % p.Sq;
+    T* dst = reinterpret_cast<T*>(p.out.ptr) + (int64_t)b * p.out.sb + (int64_t)h * p.out.sh + (int64_t)qi * p.out.ss + d;
+    dst[0] = st_f32<T>(o0 * inv);
+    dst[1] = st_f32<T>(o1 * inv);
+    if (d == 0) p.lse[((int64_t)b * p.Hq + h) * p.Sq + qi] = l > 0.f ? m * 0.6931471805599453f + logf(l) : -INFINITY;
+  }
+  cluster_sync();   // no CTA leaves while a peer may still read its shared memory
+}
+
 // kR: query rows a warp carries (the rows of the problem padded up to 1, 2, 4 or 8)
-template <typename T, int kD, int kR>
+// kCluster: the splits of a KV head are a cluster (or there is one split) and merge in shared memory
+template <typename T, int kD, int kR, bool kCluster>
 __global__ void __launch_bounds__(kThreadsDecode, kR <= 4 ? 2 : 1) splitkv_partial_kernel(const SplitKvParams p) {
   constexpr int kDP = kD / 32;   // head-dim elements per lane
-  __shared__ float sMerge[kWarpsDecode][kR][kD + 2];   // per warp and row: O, then max and sum
+  __shared__ __align__(16) float sMerge[kWarpsDecode][kR][kD + 2];   // per warp and row: O, then max and sum
+  __shared__ float2 sML[kCluster ? kMaxRows : 1];                     // max and sum of all warps
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int group = p.Hq / p.Hkv;
   const int rows = group * p.Sq;                       // <= 16
@@ -283,7 +336,7 @@ __global__ void __launch_bounds__(kThreadsDecode, kR <= 4 ? 2 : 1) splitkv_parti
     }
   }
   __syncthreads();
-  // merge the warps of a group; partial results of this split go to (B, Hq, Sq, nsplit, D) and (B, Hq, Sq, nsplit, 2)
+  // merge the warps of a group; unless a cluster merges them, partial results of this split go to (B, Hq, Sq, nsplit, D) and (B, Hq, Sq, nsplit, 2)
   for (int idx = tid; idx < ngroups * kR * kD; idx += kThreadsDecode) {
     const int g = idx / (kR * kD), r = (idx / kD) % kR, d = idx % kD;
     const int rr = g * kR + r;
@@ -297,6 +350,11 @@ __global__ void __launch_bounds__(kThreadsDecode, kR <= 4 ? 2 : 1) splitkv_parti
       acc = fmaf(sMerge[g * wpg + w][r][d], wgt, acc);
       ls = fmaf(sMerge[g * wpg + w][r][kD + 1], wgt, ls);
     }
+    if constexpr (kCluster) {
+      sMerge[g * wpg][r][d] = acc;   // (this thread alone reads and writes column d of row rr)
+      if (d == 0) sML[rr] = make_float2(mm, ls);
+      continue;
+    }
     const int h = hk * group + rr / p.Sq, qi = rr % p.Sq;
     const int64_t row = (((int64_t)b * p.Hq + h) * p.Sq + qi) * p.nsplit + split;
     p.part_o[row * kD + d] = acc;
@@ -305,7 +363,11 @@ __global__ void __launch_bounds__(kThreadsDecode, kR <= 4 ? 2 : 1) splitkv_parti
       p.part_ml[row * 2 + 1] = ls;
     }
   }
-  finish_split<T, kD>(p, b, hk, rows, tid, kThreadsDecode);
+  if constexpr (kCluster) {
+    finish_in_cluster<T, kD>(p, b, hk, rows, tid, kThreadsDecode, &sMerge[0][0][0], kR, wpg * kR, sML);
+  } else {
+    finish_split<T, kD>(p, b, hk, rows, tid, kThreadsDecode);
+  }
 }
 
 // ---- 16-bit inputs: the same pass on the warp-level tensor-core path ------------------------------
@@ -370,13 +432,14 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 __device__ __forceinline__ uint32_t reg_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
 // kNT: tiles of eight query rows (1 or 2)
-template <typename T, int kD, int kNT>
+template <typename T, int kD, int kNT, bool kCluster>
 __global__ void __launch_bounds__(kMmaWarps * 32, kNT == 1 ? 3 : 2) splitkv_partial_mma_kernel(const SplitKvParams p) {
   constexpr int kKL = kD / 32;   // 16-byte pieces of a K (and Q) row per thread
   constexpr int kVL = kD / 64;   // 16-byte pieces of a V row per thread
   constexpr int kRows = 8 * kNT;
   constexpr unsigned kFull = 0xffffffffu;
-  __shared__ float sMerge[kMmaWarps][kRows][kD + 2];   // per warp and row: O, then max and sum
+  __shared__ __align__(16) float sMerge[kMmaWarps][kRows][kD + 2];   // per warp and row: O, then max and sum
+  __shared__ float2 sML[kCluster ? kMaxRows : 1];                     // max and sum of all warps
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int group = p.Hq / p.Hkv;
   const int rows = group * p.Sq;   // <= 8 * kNT
@@ -528,7 +591,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, kNT == 1 ? 3 : 2) splitkv_part
     }
   }
   __syncthreads();
-  // merge the warps; partial results of this split go to (B, Hq, Sq, nsplit, D) and (B, Hq, Sq, nsplit, 2)
+  // merge the warps; unless a cluster merges them, partial results of this split go to (B, Hq, Sq, nsplit, D) and (B, Hq, Sq, nsplit, 2)
   for (int idx = tid; idx < rows * kD; idx += kMmaWarps * 32) {
     const int r = idx / kD, d = idx % kD;
     float mm = -INFINITY;
@@ -542,6 +605,11 @@ __global__ void __launch_bounds__(kMmaWarps * 32, kNT == 1 ? 3 : 2) splitkv_part
       acc = fmaf(sMerge[w][r][d], wgt, acc);
       ls = fmaf(sMerge[w][r][kD + 1], wgt, ls);
     }
+    if constexpr (kCluster) {
+      sMerge[0][r][d] = acc;   // (this thread alone reads and writes column d of row r)
+      if (d == 0) sML[r] = make_float2(mm, ls);
+      continue;
+    }
     const int h = hk * group + r / p.Sq, qi = r % p.Sq;
     const int64_t row = (((int64_t)b * p.Hq + h) * p.Sq + qi) * p.nsplit + split;
     p.part_o[row * kD + d] = acc;
@@ -550,19 +618,71 @@ __global__ void __launch_bounds__(kMmaWarps * 32, kNT == 1 ? 3 : 2) splitkv_part
       p.part_ml[row * 2 + 1] = ls;
     }
   }
-  finish_split<T, kD>(p, b, hk, rows, tid, kMmaWarps * 32);
+  if constexpr (kCluster) {
+    finish_in_cluster<T, kD>(p, b, hk, rows, tid, kMmaWarps * 32, &sMerge[0][0][0], kRows, 0, sML);
+  } else {
+    finish_split<T, kD>(p, b, hk, rows, tid, kMmaWarps * 32);
+  }
+}
+
+// The splits of a KV head merge as a cluster where there are few enough of them and all clusters run at once (they do not
+// cross a GPC, so the last ones of a full wave would wait for a second: 57 heads of 7 splits, D = 128, 31 us through the
+// workspace, 37 as clusters).  B200, us, whole call, through the workspace / as clusters: B4 Hq32 Hkv8 Sk1000 D128 bf16
+// (4 splits) 14.4 / 9.9, B2 Hq4 Hkv2 Sq2 Sk1364 D64 (6) 10.4 / 5.6, B20 Hq16 Hkv8 Sq2 Sk5672 D64 (3) 46.5 / 40.4,
+// B8 Hq32 Hkv8 Sk32768 D128 (6) 168 / 162, B16 Hq32 Hkv8 Sq4 Sk16384 D128 (2) 183 / 178.
+template <typename Kernel>
+cudaError_t launch_splits(Kernel kern, int threads, bool cluster, const SplitKvParams& p, cudaStream_t stream, int* resident) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = p.nsplit;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.nsplit, p.Hkv, p.B);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cluster && p.nsplit > 1 ? 1 : 0;
+  if (resident) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveClusters(resident, kern, &cfg);
+  }
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+// kAlone merges through the workspace, kCluster as a cluster.
+template <auto kAlone, auto kCluster>
+cudaError_t launch_either(int threads, const SplitKvParams& p, cudaStream_t stream) {
+  bool cluster = p.nsplit == 1;
+  if (p.nsplit > 1 && p.nsplit <= kMaxCluster) {
+    // clusters that fit the device at once, asked for once per kernel, size and device (plus one; 0: not yet)
+    static std::atomic<int> fits[64][kMaxCluster + 1];
+    int dev = 0, n = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) n = fits[dev][p.nsplit].load(std::memory_order_relaxed);
+    if (n == 0) {
+      if ((e = launch_splits(kCluster, threads, true, p, stream, &n)) != cudaSuccess) return e;
+      ++n;
+      if (dev >= 0 && dev < 64) fits[dev][p.nsplit].store(n, std::memory_order_relaxed);
+    }
+    cluster = static_cast<int64_t>(p.Hkv) * p.B < n;
+  }
+  if (cluster) return launch_splits(kCluster, threads, true, p, stream, nullptr);
+  // the per-head counters of finished splits start at zero (a memset node, not a kernel)
+  const cudaError_t e = cudaMemsetAsync(p.counters, 0, sizeof(unsigned) * p.B * p.Hkv, stream);
+  return e != cudaSuccess ? e : launch_splits(kAlone, threads, false, p, stream, nullptr);
 }
 
 template <typename T, int kD, int kR>
 cudaError_t launch_rows(const SplitKvParams& p, cudaStream_t stream) {
-  splitkv_partial_kernel<T, kD, kR><<<dim3(p.nsplit, p.Hkv, p.B), kThreadsDecode, 0, stream>>>(p);
-  return cudaGetLastError();
+  return launch_either<splitkv_partial_kernel<T, kD, kR, false>, splitkv_partial_kernel<T, kD, kR, true>>(kThreadsDecode, p, stream);
 }
 
 template <typename T, int kD, int kNT>
 cudaError_t launch_mma(const SplitKvParams& p, cudaStream_t stream) {
-  splitkv_partial_mma_kernel<T, kD, kNT><<<dim3(p.nsplit, p.Hkv, p.B), kMmaWarps * 32, 0, stream>>>(p);
-  return cudaGetLastError();
+  return launch_either<splitkv_partial_mma_kernel<T, kD, kNT, false>, splitkv_partial_mma_kernel<T, kD, kNT, true>>(kMmaWarps * 32, p,
+                                                                                                              stream);
 }
 
 template <typename T, int kD>
@@ -583,10 +703,7 @@ cudaError_t launch_t(const SplitKvParams& p, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t launch_fwd_splitkv(const SplitKvParams& p, int dtype, cudaStream_t stream, int* launches) {
-  // the per-head counters of finished splits start at zero (a memset node, not a kernel)
-  cudaError_t e = cudaMemsetAsync(p.counters, 0, sizeof(unsigned) * p.B * p.Hkv, stream);
-  if (e != cudaSuccess) return e;
-  e = cudaErrorInvalidValue;
+  cudaError_t e = cudaErrorInvalidValue;
   if (dtype == kF32) e = (p.D == 64) ? launch_t<float, 64>(p, stream) : launch_t<float, 128>(p, stream);
   else if (dtype == kBF16)
     e = (p.D == 64) ? launch_t<__nv_bfloat16, 64>(p, stream) : launch_t<__nv_bfloat16, 128>(p, stream);

@@ -369,6 +369,11 @@ __device__ __forceinline__ float peer_load_f32(uint32_t saddr, int rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(peer_addr(saddr, rank)) : "memory");
   return v;
 }
+__device__ __forceinline__ float2 peer_load_f32x2(uint32_t saddr, int rank) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(peer_addr(saddr, rank)) : "memory");
+  return v;
+}
 __device__ __forceinline__ float4 peer_load_f32x4(uint32_t saddr, int rank) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
