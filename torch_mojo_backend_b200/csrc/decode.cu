@@ -658,11 +658,14 @@ cudaError_t launch_either(int threads, const SplitKvParams& p, cudaStream_t stre
     // clusters that fit the device at once, asked for once per kernel, size and device (plus one; 0: not yet)
     static std::atomic<int> fits[64][kMaxCluster + 1];
     int dev = 0, n = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    const cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) n = fits[dev][p.nsplit].load(std::memory_order_relaxed);
     if (n == 0) {
-      if ((e = launch_splits(kCluster, threads, true, p, stream, &n)) != cudaSuccess) return e;
+      if (launch_splits(kCluster, threads, true, p, stream, &n) != cudaSuccess) {   // then never as a cluster
+        (void)cudaGetLastError();
+        n = 0;
+      }
       ++n;
       if (dev >= 0 && dev < 64) fits[dev][p.nsplit].store(n, std::memory_order_relaxed);
     }
