@@ -491,3 +491,25 @@ def test_rejected_calls_launch_nothing():
     with pytest.raises(_lib.B200FAError):
         raw.flash_fwd(q, q, q, causal=True)
     assert _lib.launch_count() == before
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_backward_of_key_tiles_that_nobody_sees(D):
+    """Causal over more keys than queries: most thread blocks of the dK/dV kernel have no step and only write zeros, and others
+    follow them on their SMs."""
+    g = torch.Generator().manual_seed(64 + D)
+    draw = lambda h, s: torch.randn(2, h, s, D, generator=g).to(torch.bfloat16).cuda()
+    Sq, Sk = 65, 9000
+    q, k, v, dout = draw(8, Sq), draw(4, Sk), draw(4, Sk), draw(8, Sq)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, lse = raw.flash_fwd(q, k, v, causal=1, status=status)
+    want = raw.flash_bwd(dout, q, k, v, out, lse, causal=1, simt=True)
+    got = raw.flash_bwd(dout, q, k, v, out, lse, causal=1, status=status)
+    for name, w, x in zip(("dq", "dk", "dv"), want, got):
+        assert parity_report(name, x, w, tol_for(q.dtype), q.dtype, ref_is_rounded=True)["over_widened"] == 0
+    assert not bool(got[1][:, :, Sq:].any()) and not bool(got[2][:, :, Sq:].any())
+    differ = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(200):
+        for w, x in zip(got, raw.flash_bwd(dout, q, k, v, out, lse, causal=1, status=status)):
+            differ += (w != x).sum()
+    assert int(differ) == 0 and int(status) == 0

@@ -197,14 +197,14 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     *abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(k_full, Cfg::kTileBytes);
-    load_tile(&mapK, sK, k_full, n0, hk);
-    if (steps > 0) {
+    if (steps > 0) {   // (else no MMA waits for a tile, and the block must not leave with copies in flight)
+      mbar_arrive_expect_tx(k_full, Cfg::kTileBytes);
+      load_tile(&mapK, sK, k_full, n0, hk);
       load_q(0);
       load_do(0);
+      mbar_arrive_expect_tx(v_full, Cfg::kTileBytes);
+      load_tile(&mapV, sV, v_full, n0, hk);
     }
-    mbar_arrive_expect_tx(v_full, Cfg::kTileBytes);
-    load_tile(&mapV, sV, v_full, n0, hk);
     // This kernel may have started before the preprocess kernel was done; only the row statistics come from that one.
     // Once every block has them in reach the dQ kernel may start.
     cudaGridDependencySynchronize();
