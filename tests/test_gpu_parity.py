@@ -513,3 +513,28 @@ def test_backward_of_key_tiles_that_nobody_sees(D):
         for w, x in zip(got, raw.flash_bwd(dout, q, k, v, out, lse, causal=1, status=status)):
             differ += (w != x).sum()
     assert int(differ) == 0 and int(status) == 0
+
+
+@pytest.mark.parametrize("dtype,D,S,causal", [(torch.float16, 64, 300, True), (torch.bfloat16, 128, 700, False), (torch.float32, 64, 300, True)])
+def test_backwards_in_turn_through_one_workspace_read_their_own_statistics(dtype, D, S, causal):
+    """The dQ kernel starts while the dK/dV kernel runs and waits for neither that nor the preprocess kernel: two problems in
+    turn, whose row statistics take the same addresses, have the bits each has alone."""
+    g = torch.Generator().manual_seed(S + D)
+    problems = []
+    for std in (0.3, 2.0):
+        q, k, v, dout = ((torch.randn(2, h, S, D, generator=g) * std).to(dtype).cuda() for h in (8, 4, 4, 8))
+        out, lse = raw.flash_fwd(q, k, v, causal=causal)
+        problems.append((dout, q, k, v, out, lse))
+    alone = []
+    for args in problems:
+        alone.append(raw.flash_bwd(*args, causal=causal))
+        torch.cuda.synchronize()
+    workspace = torch.empty(_lib.bwd_workspace_bytes(2, 8, 4, S, D, raw.dtype_code(dtype)), dtype=torch.uint8, device="cuda")
+    bits = torch.int32 if dtype == torch.float32 else torch.int16
+    differ = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(300):
+        got = [raw.flash_bwd(*args, causal=causal, workspace=workspace) for args in problems]   # nothing between the two
+        for want, grads in zip(alone, got):
+            for w, x in zip(want, grads):
+                differ += (w.view(bits) != x.view(bits)).sum()
+    assert int(differ) == 0

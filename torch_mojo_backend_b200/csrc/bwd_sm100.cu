@@ -207,8 +207,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
     // This kernel may have started before the preprocess kernel was done; only the row statistics come from that one.
     // Once every block has them in reach the dQ kernel may start.
-    cudaGridDependencySynchronize();
-    cudaTriggerProgrammaticLaunchCompletion();
+    let_the_dq_kernel_start();
     if (steps > 0) load_stat(0);
   }
   if (warp == 16) {
@@ -600,8 +599,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
     const uint32_t tDP = tmem_base + lane_off + kTmemDP + wg * 64;
     const float c = p.scale_log2;
     const int64_t stat = (static_cast<int64_t>(b) * p.Hq + h) * p.Spad + m0 + r;  // padded rows exist
-    const float nlse2 = p.lse_log2[stat];   // minus lse2
-    const float ndps = p.dpsum[stat];       // minus dpsum
+    const float nlse2 = __ldcg(p.lse_log2 + stat);   // minus lse2
+    const float ndps = __ldcg(p.dpsum + stat);       // minus dpsum
     const float2 c2 = make_float2(c, c), nl2 = make_float2(nlse2, nlse2), nd2 = make_float2(ndps, ndps);
     for (int j = 0; j < n_tiles; ++j) {
       const int buf = j & 1;

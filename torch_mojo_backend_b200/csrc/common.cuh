@@ -86,6 +86,16 @@ cudaError_t launch_bwd_simt(const BwdParams& p, int dtype, cudaStream_t stream, 
 // arrives at: exercises the bounded-wait give-up path without touching the attention kernels.
 cudaError_t launch_wait_timeout_selftest(uint32_t* status, long long budget, cudaStream_t stream, int* launches);
 
+// In the dK/dV kernels, by the threads that read the row statistics: waits for the kernel that wrote them and lets the dQ
+// kernel start.  The dQ kernel does not wait for that one itself: it starts when every block has been here, and the fence
+// orders what this thread has been shown ahead of that.  It reads the statistics from L2 (__ldcg), never through an L1
+// line that may be older.
+__device__ __forceinline__ void let_the_dq_kernel_start() {
+  cudaGridDependencySynchronize();
+  __threadfence();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+
 // A launch that, if `early`, may start as soon as every block of the kernel ahead of it on the stream has allowed it.
 template <typename... Params, typename... Args>
 cudaError_t launch_early(void (*kern)(Params...), dim3 grid, int threads, int smem, cudaStream_t stream, bool early, Args... args) {

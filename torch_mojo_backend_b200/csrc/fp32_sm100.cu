@@ -554,7 +554,7 @@ __device__ __forceinline__ void dq_rows_scalar(const BwdParams& p, int b, int h,
       dq[e] = 0.f;
     }
     const int64_t bh = static_cast<int64_t>(b) * p.Hq + h;
-    const float lse = p.lse[bh * p.S + q_row], dps = p.dpsum[bh * p.Spad + q_row];
+    const float lse = p.lse[bh * p.S + q_row], dps = __ldcg(p.dpsum + bh * p.Spad + q_row);
     const float l2 = lse != -INFINITY ? lse * kLog2e : INFINITY;
     const int last = p.causal ? min(q_row + p.causal_off, p.Sk - 1) : p.Sk - 1;
 #pragma unroll 1
@@ -646,7 +646,7 @@ __device__ __forceinline__ void dq_block(const BwdParams& p, int block, uint8_t*
       if (q_row < p.S) {
         const float lse = p.lse[static_cast<int64_t>(bh) * p.S + q_row];
         if (lse != -INFINITY) nl2 = -(lse * kLog2e);
-        ndps = -p.dpsum[static_cast<int64_t>(bh) * p.Spad + q_row];
+        ndps = -__ldcg(p.dpsum + static_cast<int64_t>(bh) * p.Spad + q_row);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -829,7 +829,7 @@ __device__ __forceinline__ void dkdv_rows_scalar(const BwdParams& p, int b, int 
         }
         s = warp_sum(s);
         dp = warp_sum(dp);
-        const float lse = p.lse[bh * p.S + q_row], dps = p.dpsum[bh * p.Spad + q_row];
+        const float lse = p.lse[bh * p.S + q_row], dps = __ldcg(p.dpsum + bh * p.Spad + q_row);
         const float pv = exp2f(s * p.scale_log2 - (lse != -INFINITY ? lse * kLog2e : INFINITY));
         const float dm = !kDropout ? 1.f : kept(p.drop, static_cast<int>(bh), q_row, key) ? p.drop.inv_keep : 0.f;
         const float ds = pv * (dp * dm - dps);
@@ -1031,8 +1031,7 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
     };
     float4 vq[8], vd[8];
     if (n > 0) load_box(vq, p.q, b, h, m0, p.S, 0, tid);
-    cudaGridDependencySynchronize();   // dpsum
-    cudaTriggerProgrammaticLaunchCompletion();
+    let_the_dq_kernel_start();
     for (int j = 0; j < n; ++j) {
       load_box(vd, p.dout, b, h, m0, p.S, 0, tid);
       float nl2 = -INFINITY, ndps = 0.f;   // rows past the end, and rows that saw no key: P = 0
@@ -1040,7 +1039,7 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
         const int64_t bh = static_cast<int64_t>(b) * p.Hq + h;
         const float lse = p.lse[bh * p.S + m0 + tid];
         if (lse != -INFINITY) nl2 = -(lse * kLog2e);
-        ndps = -p.dpsum[bh * p.Spad + m0 + tid];
+        ndps = -__ldcg(p.dpsum + bh * p.Spad + m0 + tid);
       }
       if (!slot_free(2 * j)) goto teardown;
       // The tile's statistics: a slot of theirs is written again four tiles on, when the slot rule above
