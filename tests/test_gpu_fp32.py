@@ -159,3 +159,50 @@ def test_fp32_values_that_are_not_finite_spread_as_through_fp32_products(which, 
         assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
         ok = a.isfinite()
         assert torch.allclose(a[ok], b[ok], rtol=1e-4, atol=1e-4 * float(a[ok].abs().max()))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,mode", [(128, 128, 1), (256, 256, 1), (128, 300, 2)])
+def test_fp32_a_key_of_minus_infinity_that_dropout_drops_leaves_its_row_alone(Sq, Sk, mode, D):
+    """Only the last row of a full tile sees the key, its score is minus infinity (its probability zero), and the mask drops
+    it: an ordinary row, although the score is NaN in the products of the parts."""
+    H, p = 24, 0.5
+    g = torch.Generator().manual_seed(Sk)
+    q, k, v = (torch.randn(1, H, s, D, generator=g) for s in (Sq, Sk, Sk))
+    q[:, :, Sq - 1, 3] = 1.0
+    k[:, :, Sk - 1, 3] = -float("inf")
+    keep, inv = keep_mask(1, H, Sq, Sk, p, 11, 5)
+    assert 0 < keep[0, :, Sq - 1, Sk - 1].sum() < H
+    out, lse = raw.flash_fwd(q.cuda(), k.cuda(), v.cuda(), causal=mode, dropout=(p, 11, 5))
+    with np.errstate(invalid="ignore"):
+        ref = reference(q.numpy(), k.numpy(), v.numpy(), np.zeros((1, H, Sq, D)), mode, D ** -0.5, keep, inv)
+    for name, got in (("out", out), ("lse", lse)):
+        want, got = ref[name], got.double().cpu().numpy()
+        assert np.isfinite(want).all() and np.isfinite(got).all(), name
+        assert np.linalg.norm(got - want) < 2e-5 * np.linalg.norm(want), name
+
+
+@pytest.mark.parametrize("which,value", [("v", float("inf")), ("k", float("-inf")), ("k", float("nan")), ("q", float("inf")),
+                                         ("q", 3.4e38), ("dout", float("-inf")), ("v", 3e37)])
+@pytest.mark.parametrize("Hq,Hkv,Sq,Sk,D,mode,p", [(4, 2, 129, 190, 64, 0, 0.3), (4, 2, 128, 128, 64, 1, 0.3), (2, 1, 130, 257, 64, 2, 0.0),
+                                                   (2, 2, 1, 150, 64, 0, 0.5), (4, 2, 200, 140, 64, 1, 0.2),
+                                                   (4, 2, 129, 190, 128, 0, 0.3), (2, 1, 130, 257, 128, 2, 0.3)])
+def test_fp32_values_that_are_not_finite_under_masks_and_dropout(which, value, Hq, Hkv, Sq, Sk, D, mode, p):
+    """As the FMA kernels, but for keys of the diagonal's tile that a row does not see: those multiply them by zero (NaN), the
+    tensor-core form leaves them out.  (A score of plus infinity, whose row is NaN, is left to a q that is not finite: the FMA
+    kernels lose it where the mask drops it in a row's last tile.)"""
+    g = torch.Generator().manual_seed(Sq + Sk)
+    t = {n: torch.randn(1, h, s, D, generator=g).cuda() for n, h, s in (("q", Hq, Sq), ("k", Hkv, Sk), ("v", Hkv, Sk), ("dout", Hq, Sq))}
+    t["q"][..., 5].abs_()
+    t[which][0, -1, t[which].shape[2] * 2 // 3, 5] = value
+    got = []
+    for simt in (True, False):
+        kw = {"causal": mode, "simt": simt, "dropout": (p, 11, 5) if p else None}
+        out, lse = raw.flash_fwd(t["q"], t["k"], t["v"], **kw)
+        got.append((out, lse, *raw.flash_bwd(t["dout"], t["q"], t["k"], t["v"], out, lse, **kw)))
+    for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), *got):
+        if mode == 0:
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf()), name
+        ok = a.isfinite()
+        assert bool(b[ok].isfinite().all()), name
+        assert torch.allclose(a[ok], b[ok], rtol=1e-4, atol=1e-4 * float(a[ok].abs().max()) if bool(ok.any()) else 0.0), name

@@ -439,7 +439,8 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_fp32_kernel(const __grid_cons
     B200FA_WAIT(pv_full, (n - 1) & 1, 0xc21);
     tc_fence_after();
     add_part<kD / 64>(o, tm + Cfg::kTmemO + half * (kD / 2), sc);
-    if (!all_finite(o)) *not_finite = 1;
+    // the row sum too: where dropout drops a key whose probability is NaN, only that knows of it
+    if (!all_finite(o) || !(l < INFINITY)) *not_finite = 1;
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xc30);
     if (*not_finite) {
