@@ -206,3 +206,34 @@ def test_fp32_values_that_are_not_finite_under_masks_and_dropout(which, value, H
         ok = a.isfinite()
         assert bool(b[ok].isfinite().all()), name
         assert torch.allclose(a[ok], b[ok], rtol=1e-4, atol=1e-4 * float(a[ok].abs().max()) if bool(ok.any()) else 0.0), name
+
+
+def fastest_ms(call, reps=7):
+    times = []
+    for _ in range(reps):
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        call()
+        end.record()
+        end.synchronize()
+        times.append(start.elapsed_time(end))
+    return min(times[2:])
+
+
+def test_fp32_rows_past_the_end_do_not_count_as_not_finite():
+    """Scores around -100, a length that fits no tile: the zero rows past the last key have probabilities of exp(100), which
+    must not send their thread block to compute its rows again."""
+    g = torch.Generator().manual_seed(5)
+    q, k, v, dout = (torch.randn(1, 8, 1000, 64, generator=g).cuda() for _ in range(4))
+    ms = []
+    for shift in (0.0, 3.6):
+        qs, ks = q * 0.1 + shift, k * 0.1 - shift
+        out, lse = raw.flash_fwd(qs, ks, v, causal=0)
+        if shift:
+            assert float(lse.max()) < -90.0
+        ref = raw.flash_bwd(dout, qs, ks, v, out, lse, causal=0, simt=True)
+        for a, b in zip(ref, raw.flash_bwd(dout, qs, ks, v, out, lse, causal=0)):
+            # five roundings of 2^-24 of a score of 100: 3e-5 of its dS; times keys of 3.6 whose sum cancels to their spread of 0.1
+            assert float((a - b).norm() / a.norm()) < 1e-3
+        ms.append(fastest_ms(lambda: raw.flash_bwd(dout, qs, ks, v, out, lse, causal=0)))
+    assert ms[1] < 2.0 * ms[0], ms

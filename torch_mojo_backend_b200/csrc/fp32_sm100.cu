@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_fp32_kernel(const __grid_cons
     tc_fence_after();
     add_part<kD / 64>(o, tm + Cfg::kTmemO + half * (kD / 2), sc);
     // the row sum too: where dropout drops a key whose probability is NaN, only that knows of it
-    if (!all_finite(o) || !(l < INFINITY)) *not_finite = 1;
+    if (q_row < p.Sq && (!all_finite(o) || !(l < INFINITY))) *not_finite = 1;
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xc30);
     if (*not_finite) {
@@ -706,7 +706,7 @@ __device__ __forceinline__ void dq_block(const BwdParams& p, int block, uint8_t*
       tc_fence_after();
       add_part<kD / 64>(dq, tm + Cfg::kTmemDQ + half * (kD / 2), 1.f);
     }
-    if (!all_finite(dq)) *not_finite = 1;
+    if (q_row < p.S && !all_finite(dq)) *not_finite = 1;
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xd30);
     if (*not_finite) {
@@ -1002,7 +1002,8 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
       add_part<kD / 64>(dv, tm + Cfg::kTmemDV + half * (kD / 2), 1.f);
       add_part<kD / 64>(dk, tm + Cfg::kTmemDK + half * (kD / 2), 1.f);
     }
-    if (!all_finite(dk) || !all_finite(dv)) *not_finite = 1;
+    // (rows past the end are zeros and not masked: with a logsumexp below -88 their probabilities overflow)
+    if (n0 + r < p.Sk && (!all_finite(dk) || !all_finite(dv))) *not_finite = 1;
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xe30);
     if (*not_finite) {
