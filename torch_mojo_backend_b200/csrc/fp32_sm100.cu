@@ -21,7 +21,7 @@
 // the A operand in tensor memory, 48 from shared memory), against ~14000 cycles of fp32 FMAs as measured.
 //
 // A product with an infinity cannot be split (inf * 0 is NaN): a CTA one of whose results is not finite computes its
-// rows again with scalar fp32 code before it leaves, so that infinities spread as through fp32 products.
+// rows again with fp32 FMAs before it leaves, so that infinities spread as through fp32 products (fma_rows below).
 #include <algorithm>
 #include <mutex>
 
@@ -214,15 +214,94 @@ __device__ __forceinline__ void issue_dim(uint32_t d, uint32_t a, uint32_t b_lo,
   }
 }
 
-// sum over a warp
-__device__ __forceinline__ float warp_sum(float v) {
+// The FMA forms (fma_rows_*), for CTAs whose results are not finite, by the math warps: a row is four neighbouring lanes,
+// which deal the 16-byte pieces of the head dimension among them; a lane has pieces of two rows 64 apart, so that what it
+// reads from shared memory, which bounds this, serves both.  The other sequence comes in tiles of 64 rows, in two
+// buffers where the ring was.  B200, us, a NaN in V of every head, FMA kernels / these (with the tensor-core pass ahead
+// of them) / a warp a row without staging: B4 H12 S1024 D64 causal forward 187 / 488 / 6349, backward 605 / 1076 / 12260;
+// B2 Hq16 Hkv4 S1024 D128 forward 512 / 1083 / 10377; B1 H4 S4096 D64 causal (128 CTAs against 512) 264 / 1158 / 17704.
+constexpr int kLaneRows = 2;
+// all math warps, with a bounded wait
+struct RowSync {
+  uint64_t* bar;
+  volatile uint32_t* abort_flag;
+  uint32_t* status;
+  long long budget;
+  uint32_t phase = 0;
+  __device__ __forceinline__ bool operator()() {
+    mbar_arrive_warp(bar);
+    const bool ok = mbar_wait_warp(bar, phase, abort_flag, status, 0xf00, budget);
+    phase ^= 1;
+    return ok;
+  }
+};
+// rows s0 + [0, 64) of a tensor to [row][kD]; zeros past the end
+template <int kD>
+__device__ __forceinline__ void stage_rows(float* dst, const View4& t, int b, int h, int s0, int rows) {
 #pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int it = 0; it < kBN * kD / 4 / 256; ++it) {
+    const int idx = static_cast<int>(threadIdx.x) + it * 256, r = idx / (kD / 4), c = idx % (kD / 4);
+    const bool inside = s0 + r < rows;
+    cp_async16(dst + r * kD + c * 4, row_ptr(t, b, h, inside ? s0 + r : 0) + c * 4, inside);
+  }
 }
-// dropout: is element (row, col) of head `bh` kept
-__device__ __forceinline__ bool kept(const DropoutParams& d, int bh, int row, int col) {
-  return (dropout_bits16(d, bh, row, col >> 4) >> (col & 15)) & 1u;
+// this lane's pieces of a row
+template <int kD>
+__device__ __forceinline__ void load_part(float2 (&x)[kD / 8], const float* row, int part) {
+#pragma unroll
+  for (int i = 0; i < kD / 16; ++i) {
+    const float4 v = reinterpret_cast<const float4*>(row)[4 * i + part];
+    x[2 * i] = make_float2(v.x, v.y);
+    x[2 * i + 1] = make_float2(v.z, v.w);
+  }
+}
+template <int kD>
+__device__ __forceinline__ void store_part(float* row, int part, const float2 (&x)[kD / 8], float mul) {
+#pragma unroll
+  for (int i = 0; i < kD / 16; ++i)
+    reinterpret_cast<float4*>(row)[4 * i + part] =
+        make_float4(x[2 * i].x * mul, x[2 * i].y * mul, x[2 * i + 1].x * mul, x[2 * i + 1].y * mul);
+}
+// the products of a lane's rows with a streamed one, whole in all four lanes
+template <int kD>
+__device__ __forceinline__ void dot_parts(float (&s)[kLaneRows], const float2 (&x)[kLaneRows][kD / 8], const float* row, int part) {
+  float2 a[kLaneRows], b[kLaneRows];
+#pragma unroll
+  for (int j = 0; j < kLaneRows; ++j) a[j] = b[j] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < kD / 16; ++i) {
+    const float4 v = reinterpret_cast<const float4*>(row)[4 * i + part];
+#pragma unroll
+    for (int j = 0; j < kLaneRows; ++j) {
+      a[j] = __ffma2_rn(x[j][2 * i], make_float2(v.x, v.y), a[j]);
+      b[j] = __ffma2_rn(x[j][2 * i + 1], make_float2(v.z, v.w), b[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kLaneRows; ++j) {
+    s[j] = (a[j].x + a[j].y) + (b[j].x + b[j].y);
+    s[j] += __shfl_xor_sync(0xffffffffu, s[j], 1);
+    s[j] += __shfl_xor_sync(0xffffffffu, s[j], 2);
+  }
+}
+// acc[j] += w[j] * the streamed row, for the rows that see it (`all`: every one).  A row that does not is left out: zero
+// times what is not finite is not zero.
+template <int kD>
+__device__ __forceinline__ void add_parts(float2 (&acc)[kLaneRows][kD / 8], const float (&w)[kLaneRows], bool all, const bool (&sees)[kLaneRows],
+                                          const float* row, int part) {
+#pragma unroll
+  for (int i = 0; i < kD / 16; ++i) {
+    const float4 v = reinterpret_cast<const float4*>(row)[4 * i + part];
+#pragma unroll
+    for (int j = 0; j < kLaneRows; ++j) {
+      const float2 w2 = make_float2(w[j], w[j]);
+      const float2 lo = __ffma2_rn(w2, make_float2(v.x, v.y), acc[j][2 * i]), hi = __ffma2_rn(w2, make_float2(v.z, v.w), acc[j][2 * i + 1]);
+      if (all || sees[j]) {
+        acc[j][2 * i] = lo;
+        acc[j][2 * i + 1] = hi;
+      }
+    }
+  }
 }
 
 // Block index -> (row tile, head), the longest causal rows first over all heads
@@ -243,49 +322,95 @@ struct FwdF32Cfg {
   static constexpr int kSlots = kD == 64 ? 8 : 4;
   static constexpr int kOffX = kSlots * Tile::kBytes;         // [parity][half][row] maxima
   static constexpr int kOffBars = kOffX + 2 * 2 * kBM * 4;
-  static constexpr int kNumBars = 2 * kSlots + 10;
+  static constexpr int kNumBars = 2 * kSlots + 11;
   static constexpr int kSmemBytes = kOffBars + kNumBars * 8 + 16;
   static constexpr int kTmemQ = 0, kTmemS = 192, kTmemP = 256, kTmemO = 384;
 };
 
-// rows [m0, m0 + 128) of the output, one warp a row, in scalar fp32
 template <int kD, bool kDropout>
-__device__ __forceinline__ void fwd_rows_scalar(const FwdParams& p, int b, int h, int hk, int m0, int warp, int lane) {
-  constexpr int kE = kD / 32;
-#pragma unroll 1
-  for (int r = warp; r < kBM && m0 + r < p.Sq; r += kMathWarps) {
-    const int q_row = m0 + r;
-    float q[kE], o[kE], m = -INFINITY, l = 0.f;
+__device__ __forceinline__ bool fma_rows_fwd(const FwdParams& p, int b, int h, int hk, int m0, int warp, int lane, uint8_t* smem, RowSync sync) {
+  constexpr int kKeys = kD == 64 ? 4 : 2, kTile = kBN * kD;   // keys a step
+  float* buf = reinterpret_cast<float*>(smem);   // [tile & 1][K, V][64][kD]
+  const int part = lane & 3, bh = b * p.Hq + h;
+  int q_row[kLaneRows], last[kLaneRows];
 #pragma unroll
-    for (int e = 0; e < kE; ++e) {
-      q[e] = row_ptr(p.q, b, h, q_row)[lane + 32 * e];
-      o[e] = 0.f;
-    }
-    const int last = p.causal ? min(q_row + p.causal_off, p.Sk - 1) : p.Sk - 1;
-#pragma unroll 1
-    for (int k = 0; k <= last; ++k) {
-      const float* kr = row_ptr(p.k, b, hk, k);
-      const float* vr = row_ptr(p.v, b, hk, k);
-      float s = 0.f;
-#pragma unroll
-      for (int e = 0; e < kE; ++e) s = fmaf(q[e], kr[lane + 32 * e], s);
-      s = warp_sum(s);
-      float m_new = fmaxf(m, s);
-      if (m_new == -INFINITY) m_new = 0.f;
-      const float corr = exp2f((m - m_new) * p.scale_log2);
-      float pr = exp2f((s - m_new) * p.scale_log2);
-      l = l * corr + pr;
-      if (kDropout && !kept(p.drop, b * p.Hq + h, q_row, k)) pr = 0.f;
-#pragma unroll
-      for (int e = 0; e < kE; ++e) o[e] = fmaf(pr, vr[lane + 32 * e], o[e] * corr);
-      m = m_new;
-    }
-    const float inv = l > 0.f ? (kDropout ? p.drop.inv_keep : 1.f) / l : 0.f;
-    float* dst = const_cast<float*>(row_ptr(p.out, b, h, q_row));
-#pragma unroll
-    for (int e = 0; e < kE; ++e) dst[lane + 32 * e] = o[e] * inv;
-    if (lane == 0) p.lse[(static_cast<int64_t>(b) * p.Hq + h) * p.Sq + q_row] = l > 0.f ? m * p.scale + logf(l) : -INFINITY;
+  for (int j = 0; j < kLaneRows; ++j) {
+    q_row[j] = min(m0 + j * 64 + warp * 8 + (lane >> 2), p.Sq - 1);   // (rows past the end do the last one's work)
+    last[j] = p.causal ? min(q_row[j] + p.causal_off, p.Sk - 1) : p.Sk - 1;
   }
+  const int warp_first = __reduce_min_sync(0xffffffffu, last[0]), warp_last = __reduce_max_sync(0xffffffffu, last[1]);
+  const int n_end = p.causal ? min(p.Sk, min(m0 + kBM, p.Sq) + p.causal_off) : p.Sk;
+  const int tiles = (max(n_end, 0) + kBN - 1) / kBN;
+  auto stage = [&](int t) {
+    stage_rows<kD>(buf + (t & 1) * 2 * kTile, p.k, b, hk, t * kBN, p.Sk);
+    stage_rows<kD>(buf + (t & 1) * 2 * kTile + kTile, p.v, b, hk, t * kBN, p.Sk);
+    cp_commit();
+  };
+  float2 q[kLaneRows][kD / 8], o[kLaneRows][kD / 8];
+  float m[kLaneRows], l[kLaneRows];
+#pragma unroll
+  for (int j = 0; j < kLaneRows; ++j) {
+    load_part<kD>(q[j], row_ptr(p.q, b, h, q_row[j]), part);
+#pragma unroll
+    for (int i = 0; i < kD / 8; ++i) o[j][i] = make_float2(0.f, 0.f);
+    m[j] = -INFINITY;
+    l[j] = 0.f;
+  }
+  if (tiles > 0) stage(0);
+#pragma unroll 1
+  for (int t = 0; t < tiles; ++t) {
+    cp_wait<0>();
+    if (!sync()) return false;   // the tile is here, and everyone is done with the one before
+    if (t + 1 < tiles) stage(t + 1);
+    const float* kt = buf + (t & 1) * 2 * kTile;
+    uint32_t keep[kLaneRows];
+#pragma unroll 1
+    for (int c = 0; c < kBN && t * kBN + c <= warp_last; c += kKeys) {
+      const int k = t * kBN + c;
+      if (kDropout && c % 16 == 0) {
+#pragma unroll
+        for (int j = 0; j < kLaneRows; ++j) keep[j] = dropout_bits16(p.drop, bh, q_row[j], k >> 4);
+      }
+      const bool all_see = k + kKeys - 1 <= warp_first;
+      float s[kKeys][kLaneRows];
+#pragma unroll
+      for (int u = 0; u < kKeys; ++u) dot_parts<kD>(s[u], q, kt + (c + u) * kD, part);
+#pragma unroll
+      for (int j = 0; j < kLaneRows; ++j) {
+        float m_new = m[j];
+#pragma unroll
+        for (int u = 0; u < kKeys; ++u) {
+          if (!all_see && k + u > last[j]) s[u][j] = -INFINITY;
+          m_new = fmaxf(m_new, s[u][j]);
+        }
+        if (m_new == -INFINITY) m_new = 0.f;
+        const float corr = exp2f((m[j] - m_new) * p.scale_log2);
+        m[j] = m_new;
+        l[j] *= corr;
+#pragma unroll
+        for (int i = 0; i < kD / 8; ++i) o[j][i] = __fmul2_rn(o[j][i], make_float2(corr, corr));
+#pragma unroll
+        for (int u = 0; u < kKeys; ++u) {
+          s[u][j] = exp2f((s[u][j] - m_new) * p.scale_log2);
+          l[j] += s[u][j];
+          if (kDropout && !((keep[j] >> ((c + u) & 15)) & 1u)) s[u][j] = 0.f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kKeys; ++u) {
+        const bool sees[kLaneRows] = {k + u <= last[0], k + u <= last[1]};
+        add_parts<kD>(o, s[u], all_see, sees, kt + kTile + (c + u) * kD, part);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kLaneRows; ++j) {
+    if (m0 + j * 64 + warp * 8 + (lane >> 2) >= p.Sq) continue;
+    const float inv = l[j] > 0.f ? (kDropout ? p.drop.inv_keep : 1.f) / l[j] : 0.f;
+    store_part<kD>(const_cast<float*>(row_ptr(p.out, b, h, q_row[j])), part, o[j], inv);
+    if (part == 0) p.lse[static_cast<int64_t>(bh) * p.Sq + q_row[j]] = l[j] > 0.f ? m[j] * p.scale + logf(l[j]) : -INFINITY;
+  }
+  return true;
 }
 
 template <int kD, bool kDropout>
@@ -304,6 +429,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_fp32_kernel(const __grid_cons
   uint64_t* pv_full = p_full + 1;            // P V ready, P planes consumed
   uint64_t* xchg = pv_full + 1;              // [4] the two warps of a row have written their half's maximum
   uint64_t* done = xchg + 4;                 // every math warp knows whether its results are finite (8)
+  uint64_t* rows_done = done + 1;            // RowSync's (8)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* not_finite = tmem_slot + 2;
@@ -338,6 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_fp32_kernel(const __grid_cons
     mbar_init(pv_full, 1);
     for (int i = 0; i < 4; ++i) mbar_init(&xchg[i], 2);
     mbar_init(done, kMathWarps);
+    mbar_init(rows_done, kMathWarps);
     *abort_flag = 0;
     *not_finite = 0;
     fence_mbar_init();
@@ -444,7 +571,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_fp32_kernel(const __grid_cons
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xc30);
     if (*not_finite) {
-      fwd_rows_scalar<kD, kDropout>(p, b, h, hk, m0, warp, lane);
+      if (!fma_rows_fwd<kD, kDropout>(p, b, h, hk, m0, warp, lane, smem, RowSync{rows_done, abort_flag, p.status, p.wait_budget})) goto teardown;
     } else if (q_row < p.Sq) {
       const float inv = l > 0.f ? (kDropout ? p.drop.inv_keep : 1.f) / l : 0.f;
       float4* dst = reinterpret_cast<float4*>(const_cast<float*>(row_ptr(p.out, b, h, q_row)) + half * (kD / 2));
@@ -536,49 +663,81 @@ struct DqF32Cfg {
   using Tile = TileCfg<kD>;
   static constexpr int kSlots = 8;
   static constexpr int kOffBars = kSlots * Tile::kBytes;
-  static constexpr int kNumBars = 2 * kSlots + 6;
+  static constexpr int kNumBars = 2 * kSlots + 7;
   static constexpr int kSmemBytes = kOffBars + kNumBars * 8 + 16;
   static constexpr int kTmemQ = 0, kTmemDO = 96, kTmemS = 192, kTmemDP = 256, kTmemDS = 320, kTmemDQ = 448;
 };
 
 template <int kD, bool kDropout>
-__device__ __forceinline__ void dq_rows_scalar(const BwdParams& p, int b, int h, int hk, int m0, int warp, int lane) {
-  constexpr int kE = kD / 32;
-#pragma unroll 1
-  for (int r = warp; r < kBM && m0 + r < p.S; r += kMathWarps) {
-    const int q_row = m0 + r;
-    float q[kE], g[kE], dq[kE];
+__device__ __forceinline__ bool fma_rows_dq(const BwdParams& p, int b, int h, int hk, int m0, int warp, int lane, uint8_t* smem, RowSync sync) {
+  constexpr int kKeys = 2, kTile = kBN * kD;
+  float* buf = reinterpret_cast<float*>(smem);   // [tile & 1][K, V][64][kD]
+  const int part = lane & 3, bh = b * p.Hq + h;
+  int q_row[kLaneRows], last[kLaneRows];
 #pragma unroll
-    for (int e = 0; e < kE; ++e) {
-      q[e] = row_ptr(p.q, b, h, q_row)[lane + 32 * e];
-      g[e] = row_ptr(p.dout, b, h, q_row)[lane + 32 * e];
-      dq[e] = 0.f;
-    }
-    const int64_t bh = static_cast<int64_t>(b) * p.Hq + h;
-    const float lse = p.lse[bh * p.S + q_row], dps = __ldcg(p.dpsum + bh * p.Spad + q_row);
-    const float l2 = lse != -INFINITY ? lse * kLog2e : INFINITY;
-    const int last = p.causal ? min(q_row + p.causal_off, p.Sk - 1) : p.Sk - 1;
-#pragma unroll 1
-    for (int k = 0; k <= last; ++k) {
-      const float* kr = row_ptr(p.k, b, hk, k);
-      const float* vr = row_ptr(p.v, b, hk, k);
-      float s = 0.f, dp = 0.f;
-#pragma unroll
-      for (int e = 0; e < kE; ++e) {
-        s = fmaf(q[e], kr[lane + 32 * e], s);
-        dp = fmaf(g[e], vr[lane + 32 * e], dp);
-      }
-      s = warp_sum(s);
-      dp = warp_sum(dp);
-      if (kDropout) dp *= kept(p.drop, static_cast<int>(bh), q_row, k) ? p.drop.inv_keep : 0.f;
-      const float ds = exp2f(s * p.scale_log2 - l2) * (dp - dps);
-#pragma unroll
-      for (int e = 0; e < kE; ++e) dq[e] = fmaf(ds, kr[lane + 32 * e], dq[e]);
-    }
-    float* dst = const_cast<float*>(row_ptr(p.dq, b, h, q_row));
-#pragma unroll
-    for (int e = 0; e < kE; ++e) dst[lane + 32 * e] = dq[e] * p.scale;
+  for (int j = 0; j < kLaneRows; ++j) {
+    q_row[j] = min(m0 + j * 64 + warp * 8 + (lane >> 2), p.S - 1);   // (rows past the end do the last one's work)
+    last[j] = p.causal ? min(q_row[j] + p.causal_off, p.Sk - 1) : p.Sk - 1;
   }
+  const int warp_first = __reduce_min_sync(0xffffffffu, last[0]), warp_last = __reduce_max_sync(0xffffffffu, last[1]);
+  const int n_end = p.causal ? min(p.Sk, min(m0 + kBM, p.S) + p.causal_off) : p.Sk;
+  const int tiles = (max(n_end, 0) + kBN - 1) / kBN;
+  auto stage = [&](int t) {
+    stage_rows<kD>(buf + (t & 1) * 2 * kTile, p.k, b, hk, t * kBN, p.Sk);
+    stage_rows<kD>(buf + (t & 1) * 2 * kTile + kTile, p.v, b, hk, t * kBN, p.Sk);
+    cp_commit();
+  };
+  float2 q[kLaneRows][kD / 8], g[kLaneRows][kD / 8], dq[kLaneRows][kD / 8];
+  float l2[kLaneRows], dps[kLaneRows];
+#pragma unroll
+  for (int j = 0; j < kLaneRows; ++j) {
+    load_part<kD>(q[j], row_ptr(p.q, b, h, q_row[j]), part);
+    load_part<kD>(g[j], row_ptr(p.dout, b, h, q_row[j]), part);
+#pragma unroll
+    for (int i = 0; i < kD / 8; ++i) dq[j][i] = make_float2(0.f, 0.f);
+    const float lse = p.lse[static_cast<int64_t>(bh) * p.S + q_row[j]];
+    l2[j] = lse != -INFINITY ? lse * kLog2e : INFINITY;
+    dps[j] = __ldcg(p.dpsum + static_cast<int64_t>(bh) * p.Spad + q_row[j]);
+  }
+  if (tiles > 0) stage(0);
+#pragma unroll 1
+  for (int t = 0; t < tiles; ++t) {
+    cp_wait<0>();
+    if (!sync()) return false;   // the tile is here, and everyone is done with the one before
+    if (t + 1 < tiles) stage(t + 1);
+    const float* kt = buf + (t & 1) * 2 * kTile;
+    uint32_t keep[kLaneRows];
+#pragma unroll 1
+    for (int c = 0; c < kBN && t * kBN + c <= warp_last; c += kKeys) {
+      const int k = t * kBN + c;
+      if (kDropout && c % 16 == 0) {
+#pragma unroll
+        for (int j = 0; j < kLaneRows; ++j) keep[j] = dropout_bits16(p.drop, bh, q_row[j], k >> 4);
+      }
+      const bool all_see = k + kKeys - 1 <= warp_first;
+      float s[kKeys][kLaneRows], dp[kKeys][kLaneRows];
+#pragma unroll
+      for (int u = 0; u < kKeys; ++u) {
+        dot_parts<kD>(s[u], q, kt + (c + u) * kD, part);
+        dot_parts<kD>(dp[u], g, kt + kTile + (c + u) * kD, part);
+#pragma unroll
+        for (int j = 0; j < kLaneRows; ++j) {
+          if (kDropout) dp[u][j] *= (keep[j] >> ((c + u) & 15)) & 1u ? p.drop.inv_keep : 0.f;
+          s[u][j] = exp2f(s[u][j] * p.scale_log2 - l2[j]) * (dp[u][j] - dps[j]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kKeys; ++u) {
+        const bool sees[kLaneRows] = {k + u <= last[0], k + u <= last[1]};
+        add_parts<kD>(dq, s[u], all_see, sees, kt + (c + u) * kD, part);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kLaneRows; ++j) {
+    if (m0 + j * 64 + warp * 8 + (lane >> 2) < p.S) store_part<kD>(const_cast<float*>(row_ptr(p.dq, b, h, q_row[j])), part, dq[j], p.scale);
+  }
+  return true;
 }
 
 template <int kD, bool kDropout>
@@ -594,6 +753,7 @@ __device__ __forceinline__ void dq_block(const BwdParams& p, int block, uint8_t*
   uint64_t* ds_full = s_free + 1;            // dS planes written, the last tile's dS K read (8)
   uint64_t* dq_full = ds_full + 1;           // dS K ready, dS planes consumed
   uint64_t* done = dq_full + 1;              // (8)
+  uint64_t* rows_done = done + 1;            // RowSync's (8)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* not_finite = tmem_slot + 2;
@@ -620,6 +780,7 @@ __device__ __forceinline__ void dq_block(const BwdParams& p, int block, uint8_t*
     mbar_init(ds_full, kMathWarps);
     mbar_init(dq_full, 1);
     mbar_init(done, kMathWarps);
+    mbar_init(rows_done, kMathWarps);
     *abort_flag = 0;
     *not_finite = 0;
     fence_mbar_init();
@@ -710,7 +871,7 @@ __device__ __forceinline__ void dq_block(const BwdParams& p, int block, uint8_t*
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xd30);
     if (*not_finite) {
-      dq_rows_scalar<kD, kDropout>(p, b, h, hk, m0, warp, lane);
+      if (!fma_rows_dq<kD, kDropout>(p, b, h, hk, m0, warp, lane, smem, RowSync{rows_done, abort_flag, p.status, p.wait_budget})) goto teardown;
     } else if (q_row < p.S) {
       float4* dst = reinterpret_cast<float4*>(const_cast<float*>(row_ptr(p.dq, b, h, q_row)) + half * (kD / 2));
 #pragma unroll
@@ -796,59 +957,87 @@ struct DkdvF32Cfg {
   static constexpr int kStats = 4;                               // tiles whose statistics are kept
   static constexpr int kOffStat = kOffStream + kSlots * Tile::kBytes;   // [tile & 3][lse2 | dpsum][64], both negated
   static constexpr int kOffBars = kOffStat + kStats * 2 * kBN * 4;
-  static constexpr int kNumBars = 2 * kSlots + 6;
+  static constexpr int kNumBars = 2 * kSlots + 7;
   static constexpr int kSmemBytes = kOffBars + kNumBars * 8 + 16;
   static constexpr int kTmemS = 0, kTmemDP = 64, kTmemP = 128, kTmemDS = 224, kTmemDV = 320, kTmemDK = 384;
 };
 
 template <int kD, bool kDropout>
-__device__ __forceinline__ void dkdv_rows_scalar(const BwdParams& p, int b, int hk, int n0, int warp, int lane) {
-  constexpr int kE = kD / 32;
-  const int group = p.Hq / p.Hkv;
-#pragma unroll 1
-  for (int r = warp; r < kBM && n0 + r < p.Sk; r += kMathWarps) {
-    const int key = n0 + r;
-    float k[kE], v[kE], dk[kE], dv[kE];
+__device__ __forceinline__ bool fma_rows_dkdv(const BwdParams& p, int b, int hk, int n0, int warp, int lane, uint8_t* smem, RowSync sync) {
+  constexpr int kTile = kBN * kD;
+  float* buf = reinterpret_cast<float*>(smem);   // [tile & 1][Q, dO][64][kD]
+  const int part = lane & 3, group = p.Hq / p.Hkv;
+  int key[kLaneRows], first[kLaneRows];   // first query row that sees the key
 #pragma unroll
-    for (int e = 0; e < kE; ++e) {
-      k[e] = row_ptr(p.k, b, hk, key)[lane + 32 * e];
-      v[e] = row_ptr(p.v, b, hk, key)[lane + 32 * e];
-      dk[e] = dv[e] = 0.f;
-    }
-#pragma unroll 1
-    for (int h = hk * group; h < (hk + 1) * group; ++h) {
-      const int64_t bh = static_cast<int64_t>(b) * p.Hq + h;
-#pragma unroll 1
-      for (int q_row = p.causal ? max(0, key - p.causal_off) : 0; q_row < p.S; ++q_row) {
-        const float* qr = row_ptr(p.q, b, h, q_row);
-        const float* gr = row_ptr(p.dout, b, h, q_row);
-        float s = 0.f, dp = 0.f;
+  for (int j = 0; j < kLaneRows; ++j) {
+    key[j] = min(n0 + j * 64 + warp * 8 + (lane >> 2), p.Sk - 1);
+    first[j] = p.causal ? max(0, key[j] - p.causal_off) : 0;
+  }
+  const int warp_first = __reduce_min_sync(0xffffffffu, first[0]), warp_last = __reduce_max_sync(0xffffffffu, first[1]);
+  const int m_begin = p.causal ? max(0, n0 - p.causal_off) / kBN * kBN : 0;
+  const int per_head = max(0, (p.S - m_begin + kBN - 1) / kBN), tiles = group * per_head;
+  auto stage = [&](int t) {
+    const int h = hk * group + t / per_head, q0 = m_begin + t % per_head * kBN;
+    stage_rows<kD>(buf + (t & 1) * 2 * kTile, p.q, b, h, q0, p.S);
+    stage_rows<kD>(buf + (t & 1) * 2 * kTile + kTile, p.dout, b, h, q0, p.S);
+    cp_commit();
+  };
+  float2 k[kLaneRows][kD / 8], v[kLaneRows][kD / 8], dk[kLaneRows][kD / 8], dv[kLaneRows][kD / 8];
 #pragma unroll
-        for (int e = 0; e < kE; ++e) {
-          s = fmaf(k[e], qr[lane + 32 * e], s);
-          dp = fmaf(v[e], gr[lane + 32 * e], dp);
+  for (int j = 0; j < kLaneRows; ++j) {
+    load_part<kD>(k[j], row_ptr(p.k, b, hk, key[j]), part);
+    load_part<kD>(v[j], row_ptr(p.v, b, hk, key[j]), part);
+#pragma unroll
+    for (int i = 0; i < kD / 8; ++i) dk[j][i] = dv[j][i] = make_float2(0.f, 0.f);
+  }
+  if (tiles > 0) stage(0);
+#pragma unroll 1
+  for (int t = 0; t < tiles; ++t) {
+    cp_wait<0>();
+    if (!sync()) return false;
+    if (t + 1 < tiles) stage(t + 1);
+    const float* qt = buf + (t & 1) * 2 * kTile;
+    const int bh = b * p.Hq + hk * group + t / per_head, q0 = m_begin + t % per_head * kBN;
+#pragma unroll 1
+    for (int c0 = 0; c0 < kBN && q0 + c0 < p.S; c0 += 32) {
+      // lane L has the statistics of query row L of these 32, and its keep bits against the 16 keys that hold this warp's
+      const int mine = min(q0 + c0 + lane, p.S - 1);
+      const float lse = p.lse[static_cast<int64_t>(bh) * p.S + mine], my_dps = __ldcg(p.dpsum + static_cast<int64_t>(bh) * p.Spad + mine);
+      const float my_l2 = lse != -INFINITY ? lse * kLog2e : INFINITY;
+      uint32_t my_keep[kLaneRows];
+      if constexpr (kDropout) {
+#pragma unroll
+        for (int j = 0; j < kLaneRows; ++j) my_keep[j] = dropout_bits16(p.drop, bh, mine, (n0 + j * 64 + warp * 8) >> 4);
+      }
+#pragma unroll 1
+      for (int u = max(0, warp_first - q0 - c0); u < min(32, p.S - q0 - c0); ++u) {
+        const float l2 = __shfl_sync(0xffffffffu, my_l2, u), dps = __shfl_sync(0xffffffffu, my_dps, u);
+        const float* qr = qt + (c0 + u) * kD;
+        float s[kLaneRows], dp[kLaneRows];
+        dot_parts<kD>(s, k, qr, part);
+        dot_parts<kD>(dp, v, qr + kTile, part);
+#pragma unroll
+        for (int j = 0; j < kLaneRows; ++j) {
+          const float pv = exp2f(s[j] * p.scale_log2 - l2);
+          float dm = 1.f;
+          if constexpr (kDropout) dm = (__shfl_sync(0xffffffffu, my_keep[j], u) >> (key[j] & 15)) & 1u ? p.drop.inv_keep : 0.f;
+          s[j] = pv * dm;
+          dp[j] = pv * (dp[j] * dm - dps);
         }
-        s = warp_sum(s);
-        dp = warp_sum(dp);
-        const float lse = p.lse[bh * p.S + q_row], dps = __ldcg(p.dpsum + bh * p.Spad + q_row);
-        const float pv = exp2f(s * p.scale_log2 - (lse != -INFINITY ? lse * kLog2e : INFINITY));
-        const float dm = !kDropout ? 1.f : kept(p.drop, static_cast<int>(bh), q_row, key) ? p.drop.inv_keep : 0.f;
-        const float ds = pv * (dp * dm - dps);
-#pragma unroll
-        for (int e = 0; e < kE; ++e) {
-          dv[e] = fmaf(pv * dm, gr[lane + 32 * e], dv[e]);
-          dk[e] = fmaf(ds, qr[lane + 32 * e], dk[e]);
-        }
+        const int q_row = q0 + c0 + u;
+        const bool sees[kLaneRows] = {q_row >= first[0], q_row >= first[1]};
+        add_parts<kD>(dv, s, q_row >= warp_last, sees, qr + kTile, part);
+        add_parts<kD>(dk, dp, q_row >= warp_last, sees, qr, part);
       }
     }
-    float* dst_k = const_cast<float*>(row_ptr(p.dk, b, hk, key));
-    float* dst_v = const_cast<float*>(row_ptr(p.dv, b, hk, key));
-#pragma unroll
-    for (int e = 0; e < kE; ++e) {
-      dst_k[lane + 32 * e] = dk[e] * p.scale;
-      dst_v[lane + 32 * e] = dv[e];
-    }
   }
+#pragma unroll
+  for (int j = 0; j < kLaneRows; ++j) {
+    if (n0 + j * 64 + warp * 8 + (lane >> 2) >= p.Sk) continue;
+    store_part<kD>(const_cast<float*>(row_ptr(p.dk, b, hk, key[j])), part, dk[j], p.scale);
+    store_part<kD>(const_cast<float*>(row_ptr(p.dv, b, hk, key[j])), part, dv[j], 1.f);
+  }
+  return true;
 }
 
 template <int kD, bool kDropout>
@@ -865,6 +1054,7 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
   uint64_t* ds_full = s_free + 1;            // P^T and dS^T planes written, the last tile's products read (8)
   uint64_t* acc_full = ds_full + 1;          // P^T dO and dS^T Q ready, the planes consumed
   uint64_t* done = acc_full + 1;             // (8)
+  uint64_t* rows_done = done + 1;            // RowSync's (8)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* not_finite = tmem_slot + 2;
@@ -889,6 +1079,7 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
     mbar_init(ds_full, kMathWarps);
     mbar_init(acc_full, 1);
     mbar_init(done, kMathWarps);
+    mbar_init(rows_done, kMathWarps);
     *abort_flag = 0;
     *not_finite = 0;
     fence_mbar_init();
@@ -1007,7 +1198,7 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xe30);
     if (*not_finite) {
-      dkdv_rows_scalar<kD, kDropout>(p, b, hk, n0, warp, lane);
+      if (!fma_rows_dkdv<kD, kDropout>(p, b, hk, n0, warp, lane, smem, RowSync{rows_done, abort_flag, p.status, p.wait_budget})) goto teardown;
     } else if (n0 + r < p.Sk) {
       float4* dst_k = reinterpret_cast<float4*>(const_cast<float*>(row_ptr(p.dk, b, hk, n0 + r)) + half * (kD / 2));
       float4* dst_v = reinterpret_cast<float4*>(const_cast<float*>(row_ptr(p.dv, b, hk, n0 + r)) + half * (kD / 2));

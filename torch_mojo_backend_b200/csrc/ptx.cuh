@@ -279,6 +279,18 @@ __device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
 }
 
 // ---------------------------------------------------------------------------------------
+// 16-byte asynchronous copies, per thread
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool inside) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  const int n = inside ? 16 : 0;   // the rest of the 16 bytes is filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// ---------------------------------------------------------------------------------------
 // tcgen05.ld / st, shape 32x32b: thread t of warp w touches TMEM lane 32*(w%4)+t and
 // N consecutive 32-bit columns starting at the column field of `taddr`.
 // ---------------------------------------------------------------------------------------

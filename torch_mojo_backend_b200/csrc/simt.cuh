@@ -35,6 +35,7 @@
 
 #include "common.cuh"
 #include "philox.cuh"
+#include "ptx.cuh"
 
 namespace b200fa {
 namespace {
@@ -85,15 +86,6 @@ __device__ __forceinline__ void store4(__half* p, float a, float b, float c, flo
   const __half2 lo = __floats2half2_rn(a, b), hi = __floats2half2_rn(c, d);
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
-
-__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool inside) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-  const int n = inside ? 16 : 0;   // the rest of the 16 bytes is filled with zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // The shape of a block: TM rows per thread, TY threads down the rows.
 template <int kTM, int kTY>
