@@ -252,3 +252,18 @@ def test_fp32_values_that_are_not_finite_cost_a_few_times_the_fma_kernels(B, Hq,
         fwd.append(fastest_ms(lambda: raw.flash_fwd(q, k, v, causal=mode, simt=simt)))
         bwd.append(fastest_ms(lambda: raw.flash_bwd(dout, q, k, v, out, lse, causal=mode, simt=simt)))
     assert fwd[1] < 5.0 * fwd[0] and bwd[1] < 5.0 * bwd[0], (fwd, bwd)
+
+
+@pytest.mark.parametrize("bits", [0x7f800001, 0x7fbfffff, 0x7fffffff, 0xff800001])
+@pytest.mark.parametrize("Sk", [100, 200])
+def test_fp32_a_nan_is_one_whatever_its_payload(bits, Sk):
+    """A query whose NaN has its payload below the bits of the first part, against keys all of whose parts are positive."""
+    g = torch.Generator().manual_seed(4)
+    q, k, v = (torch.randn(1, 2, s, 64, generator=g).cuda() for s in (130, Sk, Sk))
+    k[..., 5] = 1 + 2.0 ** -9 + 2.0 ** -18
+    q.view(torch.int32)[0, 1, 7, 5] = bits - (1 << 32) if bits >> 31 else bits
+    out, lse = raw.flash_fwd(q, k, v, causal=0)
+    nan = torch.zeros(2, 130, dtype=torch.bool)
+    nan[1, 7] = True
+    assert torch.equal(out.isnan().all(-1)[0].cpu(), nan) and torch.equal(out.isnan().any(-1)[0].cpu(), nan)
+    assert torch.equal(~lse.isfinite()[0].cpu(), nan)

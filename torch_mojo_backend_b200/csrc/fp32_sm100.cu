@@ -74,7 +74,7 @@ __device__ __forceinline__ void split2(float x0, float x1, uint32_t& h, uint32_t
   float2 t = __ffma2_rn(make_float2(__uint_as_float(v0 & 0xffff0000u), __uint_as_float(v1 & 0xffff0000u)), one, r);
   if (lift != 0.f) {
     t = __ffma2_rn(make_float2(x0, x1), make_float2(lift, lift), t);
-    l = __byte_perm(__float_as_uint(t.x) + 0x8000u, __float_as_uint(t.y) + 0x8000u, 0x7632);
+    l = pack2<true>(t.x, t.y);   // (by the conversion: a NaN stays one, whose payload may be in bits that h does not have)
   } else {
     l = __byte_perm(__float_as_uint(t.x), __float_as_uint(t.y), 0x7632);   // (eight bits are left: exact)
   }
