@@ -229,3 +229,14 @@ def test_valid_call_without_gpu_reports_cuda_error_not_success():
 def test_struct_layout_matches_header():
     assert ctypes.sizeof(_lib.Tensor4) == 8 + 32 + 32
     assert _lib.Tensor4.shape.offset == 8 and _lib.Tensor4.stride.offset == 40
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,splits", [
+    (10, 16, 4, 3, 7936, 128, 7),     # 12 rows: 7 splits take 175 us, 3 take 187
+    (8, 10, 1, 1, 7588, 64, 17),      # 10 rows: 17 splits take 37 us, 12 take 47
+])
+def test_split_count_of_fp32_calls_of_many_rows(B, Hq, Hkv, Sq, Sk, D, splits):
+    """The fp32 kernel is bound by its instructions there: a part-filled wave does not make its CTAs faster.  (The workspace
+    has room for the larger of the 16-bit and the fp32 count; the 16-bit one is smaller in both.)"""
+    row_bytes = B * Hq * Sq * (D + 2) * 4
+    assert _lib.fwd_splitkv_workspace_bytes(B, Hq, Hkv, Sq, Sk, D) // row_bytes == splits

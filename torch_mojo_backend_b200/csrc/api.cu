@@ -346,18 +346,25 @@ int bwd_impl(const b200fa_tensor4* q, const b200fa_tensor4* k, const b200fa_tens
 // and D = 128: prologue, merge of the warps); a split costs 2 KB more, and a merge through the workspace, where the
 // splits do not form a cluster, some 3 us (clearing the counters, the fences, the partials' way through L2): 64 KB of
 // keys while HBM is idle, half that when it is not.  A wave
-// that is not full gives each of its CTAs more of HBM, until about 0.85 of the CTAs that fit saturate it.
+// that is not full gives each of its CTAs more of HBM, until about 0.85 of the CTAs that fit saturate it; the fp32 kernel's
+// instructions, not HBM, bound it at many rows, where a CTA gains less by idle neighbours (0.9, 0.95), and above 8 rows, of
+// which each warp has half, a key takes so long that what is fixed is worth fewer of them.
 // Clusters do not cross a GPC: what fits at once is counted as seven of 18 SMs and one of 13 (the launcher asks the device;
 // a wrong guess here costs time, not results).
-// Over 1179 random calls (1-900 KV heads, 512-131072 keys, 1-16 rows, all types) the choice takes 2.6 % more time than each
-// call's best count, in 85 of them over 10 % more; a rule that does not count the merge 5.7 %, in 237.
-// B200, us, such a rule / this: B1 Hq32 Hkv8 Sk4250 D128 bf16 15.4 / 12.5 (17 / 16 splits), B8 Hq16 Hkv4 Sq4 Sk7233
-// 33 / 28 (9 / 8), B2 Hq32 Hkv8 Sq4 Sk7698 25 / 21.5 (18 / 12).
+// Measured with every count forced, one graph of calls over caches larger than L2: 6260 random calls (1-1024 KV heads,
+// 512-131072 keys, 1-16 rows, both head dims, 16 and 32 bits) that the constants were not chosen by.  The choice takes 1.2 %
+// more time than each call's best count, in 180 of them over 10 % more; a rule that does not count the merge 4.4 %, in 915;
+// the constants of the 16-bit kernel for the fp32 one above 8 rows 2.8 % there, against 0.9 %.
+// B200, us, a rule without the merge / this: B1 Hq32 Hkv8 Sk4250 D128 bf16 15.4 / 12.5 (17 / 16 splits), B8 Hq16 Hkv4 Sq4
+// Sk7233 33 / 28 (9 / 8), B2 Hq32 Hkv8 Sq4 Sk7698 25 / 21.5 (18 / 12); fp32 with the 16-bit constants / this: B10 Hq16 Hkv4
+// Sq3 Sk7936 D128 187 / 175 (3 / 7), 8 KV heads of 10 rows, Sk7588 D64 47 / 37 (12 / 17).
 // `kv_heads`: batch * KV heads, of the whole problem if the call computes a piece of one.
 int splitkv_splits(int64_t kv_heads, int64_t rows, int64_t Sk, int64_t D, bool fp32, int* split_len) {
   const int64_t per_sm = fp32 ? (rows <= 4 ? 2 : 1) : D == 64 ? (rows <= 8 ? 4 : 3) : (rows <= 8 ? 3 : 2);
   const int64_t slots = per_sm * 148;
-  const double unit = 256.0 / (D * (fp32 ? 4 : 2)), fixed = 192 * unit;   // in keys; unit: 256 bytes of them
+  const double saturated = !fp32 ? 0.85 : rows > 8 ? 0.95 : rows > (D == 64 ? 2 : 4) ? 0.9 : 0.85;
+  const double unit = 256.0 / (D * (fp32 ? 4 : 2)) * (fp32 && rows > 8 ? 0.7 : 1.0);   // in keys; 256 bytes of them
+  const double fixed = 192 * unit;
   int64_t max_n = (Sk + 255) / 256;
   if (max_n > 64) max_n = 64;
   if (max_n < 1) max_n = 1;
@@ -369,7 +376,7 @@ int splitkv_splits(int64_t kv_heads, int64_t rows, int64_t Sk, int64_t D, bool f
     const int64_t full = kv_heads * n / slots, rest = kv_heads * n % slots;
     const int64_t clusters = n <= 2 ? slots / 2 : 7 * (18 * per_sm / n) + 13 * per_sm / n;
     double cost = full * (len + fixed) + 8 * unit * n;
-    if (rest > 0) cost += len * std::max(0.85, static_cast<double>(rest) / slots) + fixed;
+    if (rest > 0) cost += len * std::max(saturated, static_cast<double>(rest) / slots) + fixed;
     if (n > 1 && (n > kSplitkvCluster || kv_heads > clusters))
       cost += 256 * unit * (1.0 - 0.5 * std::min(1.0, static_cast<double>(kv_heads * n) / slots));
     if (best_cost < 0.0 || cost < best_cost) {
