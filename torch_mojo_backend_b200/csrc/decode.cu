@@ -157,8 +157,23 @@ __device__ __forceinline__ void finish_split(const SplitKvParams& p, int b, int 
 template <typename T, int kD>
 __device__ __forceinline__ void finish_in_cluster(const SplitKvParams& p, int b, int hk, int rows, int tid, int nthreads,
                                                   const float* o, int row_tile, int tile_stride, const float2* ml) {
-  cluster_sync();
   const int group = p.Hq / p.Hkv;
+  if (p.nsplit == 1) {   // nothing to merge: the same arithmetic with one weight, which is 1
+    __syncthreads();
+#pragma unroll 4
+    for (int idx = tid; idx < rows * (kD / 2); idx += nthreads) {
+      const int rr = idx / (kD / 2), d = idx % (kD / 2) * 2;
+      const float2 v = ml[rr], x = *reinterpret_cast<const float2*>(o + ((rr / row_tile) * tile_stride + rr % row_tile) * (kD + 2) + d);
+      const float inv = v.y > 0.f ? 1.f / v.y : 0.f;
+      const int h = hk * group + rr / p.Sq, qi = rr % p.Sq;
+      T* dst = reinterpret_cast<T*>(p.out.ptr) + (int64_t)b * p.out.sb + (int64_t)h * p.out.sh + (int64_t)qi * p.out.ss + d;
+      dst[0] = st_f32<T>(x.x * inv);
+      dst[1] = st_f32<T>(x.y * inv);
+      if (d == 0) p.lse[((int64_t)b * p.Hq + h) * p.Sq + qi] = v.y > 0.f ? v.x * 0.6931471805599453f + logf(v.y) : -INFINITY;
+    }
+    return;
+  }
+  cluster_sync();
   for (int idx = static_cast<int>(blockIdx.x) * nthreads + tid; idx < rows * (kD / 2); idx += p.nsplit * nthreads) {
     const int rr = idx / (kD / 2), d = idx % (kD / 2) * 2;
     const uint32_t a_ml = smem_u32(ml + rr);
