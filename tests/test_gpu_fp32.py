@@ -1,6 +1,7 @@
 """The fp32 kernels at the edges of their tiles, on the GPU: rows and columns around 32, 64 and
-128, both block shapes (problems of fewer than TALL_BLOCKS 64-row blocks take the short one), grouped heads, both causal
-alignments, dropout, and views of a fused projection, against the same attention in float64."""
+128, grouped heads, both causal alignments, dropout, and views of a fused projection, against the same attention in float64.
+Every case runs the FMA kernels (`simt`), in both block shapes (problems of fewer than TALL_BLOCKS 64-row blocks take the
+short one), and what the library picks: the tensor-core kernels, but for backwards and forwards over few keys at D = 128."""
 
 import numpy as np
 import pytest
@@ -21,12 +22,12 @@ CASES = [
     (1, 3, 1, 129, 63, 128, 2, 0.0),       # the first query rows see no key
     (2, 4, 2, 96, 200, 64, 1, 0.25),
     (1, 2, 2, 130, 70, 128, 0, 0.5),
-    (19, 8, 8, 130, 129, 64, 1, 0.0),      # 456 tall blocks each way
+    (19, 8, 8, 130, 129, 64, 1, 0.0),      # 456 tall blocks each way in the FMA kernels
     (19, 8, 4, 193, 321, 64, 2, 0.2),
     (25, 6, 6, 65, 66, 128, 1, 0.0),
     (13, 12, 6, 60, 130, 128, 0, 0.3),
 ]
-# the tall shape in all three kernels
+# the tall shape in all three FMA kernels
 TALL = [
     (38, 6, 6, 65, 66, 128, 1, 0.0),
     (20, 12, 6, 130, 200, 128, 2, 0.3),
@@ -35,14 +36,16 @@ TALL = [
 ]
 
 
+@pytest.mark.parametrize("simt", [False, True])
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,mode,p", TALL)
-def test_fp32_tall_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p):
+def test_fp32_tall_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p, simt):
     assert min(B * Hq * -(-Sq // 64), B * Hkv * -(-Sk // 64)) >= TALL_BLOCKS
-    test_fp32_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p)
+    test_fp32_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p, simt)
 
 
+@pytest.mark.parametrize("simt", [False, True])
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,mode,p", CASES)
-def test_fp32_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p):
+def test_fp32_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p, simt):
     g = torch.Generator().manual_seed(Sq * 1000 + Sk)
     scale = D ** -0.5
     # q is a view into a wider row, as a fused projection gives it
@@ -52,8 +55,8 @@ def test_fp32_tile_edges(B, Hq, Hkv, Sq, Sk, D, mode, p):
     dropout = (p, 11, 5) if p else None
     qc = torch.empty(B, Sq, Hq, 2 * D, device="cuda")[..., :D].transpose(1, 2).copy_(q)
     kc, vc = k.cuda(), v.cuda()
-    out, lse = raw.flash_fwd(qc, kc, vc, causal=mode, scale=scale, dropout=dropout)
-    dq, dk, dv = raw.flash_bwd(dout.cuda(), qc, kc, vc, out, lse, causal=mode, scale=scale, dropout=dropout)
+    out, lse = raw.flash_fwd(qc, kc, vc, causal=mode, scale=scale, dropout=dropout, simt=simt)
+    dq, dk, dv = raw.flash_bwd(dout.cuda(), qc, kc, vc, out, lse, causal=mode, scale=scale, dropout=dropout, simt=simt)
     torch.cuda.synchronize()
     keep, inv = keep_mask(B, Hq, Sq, Sk, p, 11, 5)
     ref = reference(q.numpy(), k.numpy(), v.numpy(), dout.numpy(), mode, scale, keep, inv)
@@ -92,7 +95,7 @@ def reference(q, k, v, do, mode, scale, keep, inv):
             "dv": fold(np.swapaxes(pd, -1, -2) @ do)}
 
 
-# keys of more than 96: the tensor-core forward; D = 64: the tensor-core backward at any length
+# the tensor-core kernels: forwards at D = 64 and, over more than a few keys, at D = 128; backwards at D = 64
 SPLIT = [
     # B, Hq, Hkv, Sq, Sk, D, causal mode, dropout
     (1, 2, 2, 1, 97, 64, 0, 0.0),
@@ -102,15 +105,20 @@ SPLIT = [
     (1, 3, 3, 257, 257, 64, 1, 0.2),
     (3, 2, 2, 64, 640, 64, 1, 0.0),        # more key tiles than ring slots, and keys that nobody sees
     (1, 2, 2, 1, 2, 64, 0, 0.0),
+    (3, 4, 2, 33, 5, 64, 0, 0.2),
+    (1, 2, 1, 200, 64, 64, 2, 0.0),
     (1, 2, 1, 128, 129, 128, 2, 0.0),
     (2, 4, 4, 65, 320, 128, 0, 0.25),
     (1, 2, 2, 193, 193, 128, 1, 0.0),
 ]
 
 
-def errors(B, Hq, Hkv, Sq, Sk, D, mode, p, simt):
+def errors(B, Hq, Hkv, Sq, Sk, D, mode, p, simt, values=None):
+    """2-norm errors relative to float64.  `values`: what q and k are made of, from normal values."""
     g = torch.Generator().manual_seed(Sq * 1000 + Sk)
     q, k, v, dout = (torch.randn(B, h, s, D, generator=g) for h, s in ((Hq, Sq), (Hkv, Sk), (Hkv, Sk), (Hq, Sq)))
+    if values:
+        q, k = values(q), values(k)
     dropout = (p, 11, 5) if p else None
     qc, kc, vc = q.cuda(), k.cuda(), v.cuda()
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
@@ -137,11 +145,55 @@ def test_fp32_on_the_tensor_cores(B, Hq, Hkv, Sq, Sk, D, mode, p):
         assert err < bound, f"{name}: relative error {err:.2e}"
 
 
-@pytest.mark.parametrize("S,D", [(512, 64), (512, 128)])
-def test_fp32_tensor_core_forms_lose_no_precision(S, D):
-    fma, split = (errors(1, 4, 2, S, S, D, 1, 0.0, simt) for simt in (True, False))
-    for name in fma:   # (lse is at the rounding of its own value in both)
-        assert split[name] < 1.1 * fma[name], f"{name}: {split[name]:.2e} against {fma[name]:.2e}"
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S,std", [(200, 1.0), (512, 0.5), (512, 1.0), (1000, 0.577), (2048, 1.0)])
+def test_fp32_tensor_core_forms_lose_no_precision(S, std, D):
+    """Against the FMA kernels, both relative to float64, over the spreads that attention meets.  The logsumexp is at the rounding
+    of its own value in both (measured 0.96 to 1.07 of theirs), the rest 0.18 to 0.86; the D = 128 backward is the same one."""
+    fma, split = (errors(1, 4, 2, S, S, D, 1, 0.0, simt, lambda x: x * std) for simt in (True, False))
+    for name in fma:
+        bound = 1.1 if name == "lse" or (D == 128 and name != "out") else 1.0
+        assert split[name] < bound * fma[name], f"{name}: {split[name]:.2e} against {fma[name]:.2e}"
+
+
+def one_large_channel(x):
+    x[..., 3] = x[..., 3].abs() + 20
+    return x * 0.5
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("values", [one_large_channel, lambda x: x * 0.3 + 2, lambda x: x.mul(1.5).round()],
+                         ids=["one large channel", "large mean", "whole numbers"])
+def test_fp32_tensor_core_scores_that_do_not_look_random(values, D):
+    """What the correction of the scores' operand does not fit: scores whose terms are all large, or exact.  Everything but the
+    logsumexp is still nearer to float64 than the FMA kernels leave it; that is within an ulp of its value (2^-23), where they
+    leave it half of one."""
+    fma, split = (errors(1, 4, 2, 512, 512, D, 1, 0.0, simt, values) for simt in (True, False))
+    assert split.pop("lse") < 2.0 ** -23
+    for name in split:
+        if D == 64 or name == "out":   # (the gradients of two calls in a row at D = 128 are of two kinds: see below)
+            assert split[name] < fma[name], f"{name}: {split[name]:.2e} against {fma[name]:.2e}"
+
+
+@pytest.mark.parametrize("values", [one_large_channel, lambda x: x * 0.3 + 2], ids=["one large channel", "large mean"])
+@pytest.mark.parametrize("Sq,Sk,D", [(256, 256, 128), (300, 90, 128), (512, 512, 64), (64, 64, 64), (300, 90, 64), (300, 97, 64)])
+def test_fp32_training_takes_forward_and_backward_of_one_kind(Sq, Sk, D, values):
+    """Keys that share a large component: gradients are no further from float64 than those of the FMA kernels for both
+    (measured 0.57 to 1.0 of them; 1.4 to 8 with one kind for the forward and the other for the backward)."""
+    import torch_mojo_backend_b200 as tmb
+
+    tmb.register_mojo_devices()
+    fma = errors(1, 4, 2, Sq, Sk, D, 0, 0.0, True, values)
+    g = torch.Generator().manual_seed(Sq * 1000 + Sk)
+    q, k, v, dout = (torch.randn(1, h, s, D, generator=g) for h, s in ((4, Sq), (2, Sk), (2, Sk), (4, Sq)))
+    q, k = values(q), values(k)
+    ref = reference(q.numpy(), k.numpy(), v.numpy(), dout.numpy(), 0, D ** -0.5, *keep_mask(1, 4, Sq, Sk, 0.0, 11, 5))
+    leaves = [tmb.from_cuda(t.cuda()).requires_grad_() for t in (q, k, v)]
+    out = torch.nn.functional.scaled_dot_product_attention(*leaves, enable_gqa=True)
+    grads = torch.autograd.grad(out, leaves, tmb.from_cuda(dout.cuda()))
+    for name, got in zip(("dq", "dk", "dv"), grads):
+        err = np.linalg.norm(tmb.to_cuda(got).double().cpu().numpy() - ref[name]) / np.linalg.norm(ref[name])
+        assert err < 1.05 * fma[name], f"{name}: {err:.2e} against {fma[name]:.2e}"
 
 
 @pytest.mark.parametrize("which,value", [("v", float("inf")), ("k", float("-inf")), ("k", float("nan")), ("q", float("inf")),

@@ -418,3 +418,28 @@ def test_a_call_that_nobody_differentiates_reaches_the_bridge_as_the_operator_do
     assert not alone(q, k, v) and type(sdpa()[0].grad_fn).__name__ == "ScaledDotProductFlashAttentionBackward0"
     with torch.no_grad():
         assert alone(q, k, v)
+
+
+def test_the_fp32_forward_of_a_training_call_is_of_the_backwards_kind(host_backed_mojo, monkeypatch):
+    """Head dimension 128 in fp32: FMA arithmetic in the backward, so in the forward too where a backward follows."""
+    from torch_mojo_backend_b200 import _lib
+
+    seen = []
+    plain = _lib.fwd
+    monkeypatch.setattr(_lib, "fwd", lambda *args, simt=False, whole_heads=0, **kw: (seen.append(simt), plain(*args, **kw))[1])
+    sdpa = torch.nn.functional.scaled_dot_product_attention
+    flash = torch.ops.aten._scaled_dot_product_flash_attention
+    for dtype, D in ((torch.float32, 128), (torch.float32, 64), (torch.bfloat16, 128)):
+        q, k, v = (mojo((2, 4, 130, D), dtype) for _ in range(3))
+        sdpa(q, k, v)
+        flash(q, k, v, 0.0, False)
+        with flash_ops.piece_of(8, True):
+            flash(q, k, v, 0.0, False)
+        k.requires_grad_()
+        sdpa(q, k, v)
+        with torch.no_grad():
+            sdpa(q, k, v)
+            flash(q, k, v, 0.0, False)
+        exact = dtype == torch.float32 and D == 128
+        assert seen == [False, False, exact, exact, False, False]
+        seen.clear()

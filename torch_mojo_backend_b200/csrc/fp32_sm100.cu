@@ -1410,13 +1410,15 @@ cudaError_t launch_bwd(const BwdParams& p, cudaStream_t stream) {
   return launch_early(k2, dim3(static_cast<unsigned>(q_blocks)), kThreads, DqF32Cfg<kD>::kSmemBytes, stream, true, p);
 }
 
-// Few keys: the fp32 FMA kernels have less to set up and smaller tiles.
-// B200, us, FMA kernels against these (D = 64): 64 keys 5.2-11 / 6.4-14 whatever the batch, 89 keys 8.3 / 9.1, 92 keys
-// B2 Hq12 Sq1061 9.5 / 16.3, 111 keys 7.7 / 7.5, 135 keys B8 Hq16 23.7 / 19.8, 196 and more 1.1-3.8 times as fast.  At
-// D = 128 the FMA kernels lose as soon as they run in waves: 98 keys B16 Hq24 73.6 / 41.7, B1 Hq32 Sq86 12.0 / 13.6.
+// Few keys at D = 128: the fp32 FMA kernels have less to set up and smaller tiles, and lose as soon as they run in waves.
+// B200, us, FMA kernels against these: B1 Hq32 Sq86 12.0 / 13.6, 98 keys B16 Hq24 73.6 / 41.7.
+// At D = 64 they would save 1-3 us of 6-14 below 96 keys while they fit at once (B2 Hq12 Sq1061 Sk92 9.5 against 16.3; in
+// waves they lose, B16 H8 Sq1000 Sk77 121 / 66), but the backward there is on the tensor cores at any length, and a forward
+// and a backward whose scores have different errors give gradients up to eight times further from float64 than two of one
+// kind, where keys share a large component.
 bool few_keys(const FwdParams& p) {
   const int64_t keys = p.causal ? std::min<int64_t>(p.Sk, static_cast<int64_t>(p.Sq) + p.causal_off) : p.Sk;   // that anyone sees
-  return p.D == 64 ? keys <= 96 : keys <= 128 && p.whole_heads * ((p.Sq + 31) / 32) <= 148;
+  return p.D == 128 && keys <= 128 && p.whole_heads * ((p.Sq + 31) / 32) <= 148;
 }
 
 }  // namespace

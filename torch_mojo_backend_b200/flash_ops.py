@@ -195,25 +195,35 @@ _piece = threading.local()
 
 
 @contextlib.contextmanager
-def piece_of(whole_heads: int):
+def piece_of(whole_heads: int, backward: bool = False):
     """Forwards of this thread inside the block compute pieces of a problem of `whole_heads` (batch *
-    query heads) and give the bits that one call over the whole would."""
-    before = getattr(_piece, "heads", 0)
-    _piece.heads = int(whole_heads)
+    query heads) and give the bits that one call over the whole would; `backward`: their results go into the
+    backward operator, although no tensor of theirs asks for a gradient."""
+    before = getattr(_piece, "heads", 0), getattr(_piece, "backward", False)
+    _piece.heads, _piece.backward = int(whole_heads), backward
     try:
         yield
     finally:
-        _piece.heads = before
+        _piece.heads, _piece.backward = before
+
+
+def _backward_follows(*tensors) -> bool:
+    return getattr(_piece, "backward", False) or (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))
 
 
 def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is_causal: bool,
-                  scale: float | None, dropout_p: float = 0.0, philox=(0, 0)):
+                  scale: float | None, dropout_p: float = 0.0, philox=(0, 0), for_backward: bool = False):
     """Allocate ``out`` (same dtype as q) and ``lse`` (fp32, (B,Hq,Sq)), enqueue the forward
     kernel, return ``(out, lse, q_used, k_used, v_used)`` like
     ``fast_fa4_16bit_d64_causal_forward`` (aten_fast.py:7151-7285).  A decode-shaped call (all
     query rows of a GQA group fit one split-KV thread block, long key sequence, no dropout) goes
     to the split-KV kernels, the counterpart of the reference's decode path
-    (aten_fast.py:9171-9203)."""
+    (aten_fast.py:9171-9203).
+
+    ``for_backward``: the fp32 backward at head dimension 128 is FMA arithmetic, and so is the forward
+    whose results it takes.  Its gradients lean on score errors that are the same in both: with an ``out`` of the
+    tensor-core forward, nearer to the truth as it is, they come out up to ten times further from it where keys
+    share a large component."""
     batch, heads_q, seq, head_dim = q._shape
     heads_kv, seq_k = k._shape[1], k._shape[2]
     index = q._device_index
@@ -237,6 +247,8 @@ def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is
         return out, lse, q_used, k_used, v_used
     _log("fwd B=%d Hq=%d Hkv=%d Sq=%d Sk=%d D=%d causal=%s p=%s", batch, heads_q, heads_kv, seq, seq_k, head_dim, is_causal,
          dropout_p)
+    if for_backward and head_dim == 128 and code == _lib.F32:
+        piece["simt"] = True
     rc = _lib.fwd(_t4(q_used), _t4(k_used), _t4(v_used), _t4(out), lse._ptr, code, bool(is_causal), float(scale),
                   _stream_for(index), index, _status_ptr(index), dropout=_dropout_arg(dropout_p, philox), **piece)
     _check(rc, "b200fa_fwd")
@@ -244,7 +256,7 @@ def flash_forward(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, is
 
 
 def forward_with_its_own_mask(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMojoTensor, dropout_p: float,
-                              is_causal: bool, scale: float | None):
+                              is_causal: bool, scale: float | None, for_backward: bool = False):
     """``(out, lse, (seed, offset))`` of inputs that ``flash_inputs`` has accepted; the Philox state the dropout mask
     is drawn from is reserved here."""
     CALL_COUNTERS["aten::_scaled_dot_product_flash_attention"] += 1
@@ -254,7 +266,7 @@ def forward_with_its_own_mask(q: TorchMojoTensor, k: TorchMojoTensor, v: TorchMo
         if q._holder.is_cuda and torch.cuda.is_current_stream_capturing():
             raise RuntimeError("mojo attention with dropout cannot be captured: every replay would draw the same mask")
         philox = device_module._reserve_philox_state(q._device_index, q._shape[0] * q._shape[1])
-    out, lse, _, _, _ = flash_forward(q, k, v, is_causal, scale, dropout_p, philox)
+    out, lse, _, _, _ = flash_forward(q, k, v, is_causal, scale, dropout_p, philox, for_backward)
     return out, lse, philox
 
 
@@ -281,7 +293,8 @@ def scaled_dot_product_flash_attention(query, key, value, dropout_p=0.0, is_caus
         )
     q, k, v = inputs
     index = q._device_index
-    out, lse, (seed, offset) = forward_with_its_own_mask(q, k, v, dropout_p, is_causal, scale)
+    out, lse, (seed, offset) = forward_with_its_own_mask(q, k, v, dropout_p, is_causal, scale,
+                                                         _backward_follows(query, key, value))
     rng_state = TorchMojoTensor._alloc((2,), torch.uint64, index)
     if float(dropout_p):
         # the pair as two signed 64-bit patterns (uint64 fills are not universally supported), by two fills: a copy from
@@ -371,6 +384,6 @@ def scaled_dot_product_flash_attention_backward(grad_out, query, key, value, out
               and l._dtype == torch.float32 and tuple(l._shape) == (batch, heads_q, seq))
     if not usable:
         CALL_COUNTERS["backward_recomputed_forward"] += 1
-        o, l, _, _, _ = flash_forward(q, k, v, bool(is_causal), float(scale), dropout_p, philox)
+        o, l, _, _, _ = flash_forward(q, k, v, bool(is_causal), float(scale), dropout_p, philox, for_backward=True)
     CALL_COUNTERS["aten::_scaled_dot_product_flash_attention_backward"] += 1
     return flash_backward(g, q, k, v, o, l, bool(is_causal), float(scale), dropout_p, philox)

@@ -112,7 +112,7 @@ class HostAttentionPipeline:
                 uploaded.record(s_in)
             with torch.cuda.stream(s_run):
                 s_run.wait_event(uploaded)
-                with flash_ops.piece_of(q.shape[0] * q.shape[1]):
+                with flash_ops.piece_of(q.shape[0] * q.shape[1], backward):
                     fwd = flash_fwd(dev_in[0], dev_in[1], dev_in[2], 0.0, is_causal, False, scale=scale)
                 o, lse = fwd[0], fwd[1]
                 g = ()

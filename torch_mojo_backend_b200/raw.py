@@ -45,7 +45,9 @@ def flash_fwd(q, k, v, *, causal, scale: float | None = None, out=None, lse=None
     ``out`` defaults to a new contiguous (B, Hq, Sq, D) tensor; pass a pre-allocated (possibly
     strided) tensor to choose the storage layout.  ``lse`` is fp32 (B, Hq, Sq).  ``causal`` is a
     bool (True: diagonal from the top-left corner) or one of ``_lib.CAUSAL_*``; ``dropout`` is
-    None or ``(p, philox_seed, philox_offset)``.  A call that computes a piece of a larger problem
+    None or ``(p, philox_seed, philox_offset)``; ``simt`` takes the exact-fp32 FMA kernels, which an fp32
+    forward at head dimension 128 should whose results go into ``flash_bwd`` (that one is FMA arithmetic there, and
+    its gradients lean on both having the same errors in the scores).  A call that computes a piece of a larger problem
     (some batch entries or whole groups of heads, one rank's shard) has the bits of one call over the
     whole if it is told the whole's batch * query heads in ``whole_heads``.
     """
