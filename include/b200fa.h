@@ -78,7 +78,14 @@ typedef struct b200fa_tensor4 {
  *   key/value head h / (Hq / Hkv));  D in {64, 128};  any Sq, Sk, masked or not (the reference's
  *   gate needs Sq == Sk, aten_fast.py:7029-7030); `causal` is one of B200FA_CAUSAL_*.
  *   dtype  : B200FA_BF16 / B200FA_F16 run the tcgen05 tensor-core kernel,
- *            B200FA_F32 runs an exact-fp32 SIMT kernel.
+ *            B200FA_F32 runs a tcgen05 kernel on three bf16 parts of every value (six of the nine
+ *            partial products, sums of a row in fp32): with normal values `out` is within 4e-7 of
+ *            float64 (2-norm) up to 4096 keys, nearer than fp32 FMAs come, `lse` within an ulp;
+ *            at D = 128 over up to 128 keys that fit the GPU at once, an FMA kernel.
+ *            b200fa_fwd_simt and `exact_fp32` keep FMA arithmetic.
+ * The fp32 backward is of the tcgen05 kind at D = 64 and of the FMA kind at D = 128.  Its gradients
+ * lean on the forward having the same errors in the scores, so at D = 128 call b200fa_fwd_simt (or
+ * pass `exact_fp32`) for a forward whose out and lse go into b200fa_bwd.
  * Replaces flash_attention_fwd_<dtype>_d<D>_causal{,_strided_qkv,_bhsd}
  * (torch_mojo_backend/eager_flash_attention/fa4_ops.mojo:61-102, 428-449, 666-744).
  */
@@ -224,7 +231,7 @@ int b200fa_fwd_splits(int64_t batch, int64_t heads_q, int64_t seqlen_q, int64_t 
                       int dtype, int causal, int64_t whole_heads);
 
 /*
- * Same contracts as b200fa_fwd / b200fa_bwd, but always run the exact-fp32 SIMT kernels
+ * Same contracts as b200fa_fwd / b200fa_bwd, but always run the SIMT kernels of fp32 FMAs
  * whatever the storage type (16-bit inputs are widened to fp32 on load).  They exist so the
  * tensor-core kernels can be cross-checked on the device at sizes where a CPU comparison
  * would take minutes; they have no counterpart in the reference.

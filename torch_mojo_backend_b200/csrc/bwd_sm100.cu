@@ -65,9 +65,8 @@ __device__ __forceinline__ float2 exp2_mufu2(float2 x) { return make_float2(ex2_
 // ------------------------------------------------------------------------------------------
 // dK / dV kernel.  One CTA = one 128-row K/V tile of one (batch, kv head); it walks every
 // query tile at or below the causal diagonal for every query head of the GQA group.
-// TMEM columns: [0,128) S^T; [128,256) dP^T, overwritten by 16-bit dS^T (the A operand of the
-// dK MMA); then the dV and dK accumulators.  16-bit P^T goes through shared memory instead, so
-// S^T of the next step can be issued while the exponentials of this step are still running.
+// TMEM columns: two work buffers of 128, in turn: S^T of a step, over which 16-bit P^T and dS^T go (the A operands of the
+// dV and dK MMAs); then the dV and dK accumulators; dP^T at D = 64 in a third buffer, at D = 128 in the other step's.
 // ------------------------------------------------------------------------------------------
 template <int kD, bool kBf16, bool kCausal, bool kDropout>
 __global__ void __launch_bounds__(kDkdvThreads, 1)

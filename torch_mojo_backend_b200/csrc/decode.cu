@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, kNT == 1 ? 3 : 2) splitkv_part
 // cross a GPC, so the last ones of a full wave would wait for a second: 57 heads of 7 splits, D = 128, 31 us through the
 // workspace, 37 as clusters).  B200, us, whole call, through the workspace / as clusters: B4 Hq32 Hkv8 Sk1000 D128 bf16
 // (4 splits) 14.4 / 9.9, B2 Hq4 Hkv2 Sq2 Sk1364 D64 (6) 10.4 / 5.6, B20 Hq16 Hkv8 Sq2 Sk5672 D64 (3) 46.5 / 40.4,
-// B8 Hq32 Hkv8 Sk32768 D128 (6) 168 / 162, B16 Hq32 Hkv8 Sq4 Sk16384 D128 (2) 183 / 178.
+// B8 Hq32 Hkv8 Sk32768 D128 (6) 168 / 162; nothing at B16 Hq32 Hkv8 Sq4 Sk16384 D128 (2; 183 / 182).
 template <typename Kernel>
 cudaError_t launch_splits(Kernel kern, int threads, bool cluster, const SplitKvParams& p, cudaStream_t stream, int* resident) {
   cudaLaunchAttribute attr;

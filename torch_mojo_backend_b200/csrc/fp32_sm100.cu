@@ -7,8 +7,10 @@
 // of |x x'| and zero on average.  tcgen05 truncates its accumulator after every 16 terms, always towards zero, so a
 // long running sum would drift: the products are therefore issued smallest first, a tile product
 // starts from zero, and the sum over the tiles of a row (O, dQ, dK, dV) is kept in registers and added to
-// with rounding to nearest.  The relative errors against float64, at launch_fwd_fp32, are smaller than those
-// of the fp32 FMA kernels of simt.cuh.
+// with rounding to nearest.  A single product is up to 2.0e-7 of itself off, where an FMA rounds to 6e-8; the long sums,
+// which decide, are nearer to float64 than those of the fp32 FMA kernels (simt.cuh): at launch_fwd_fp32.
+// Probabilities below 2^-126 of a row's largest are zero (ex2.approx.ftz).
+// (The first part rounded to nearest too leaves out a quarter as much: errors 1-3 % smaller, kernels 1-13 % slower.)
 //
 // Same math and masks as simt.cuh (reference: torch_mojo_backend/eager_flash_attention/
 // fa4_fwd_kernel.mojo:650-861, fa4_bwd_kernel.mojo:1-44, 810-980).  A CTA owns 128 resident rows and
@@ -17,8 +19,10 @@
 //   warps 8-11  converters: fp32 rows from global memory, split into three swizzled bf16 tiles in a
 //               ring slot of shared memory
 //   warp  12    issues the MMAs
-// The bound is the tensor pipe: a 128x64 product over 64 elements is 24 MMAs of 128x64x16 (32 cycles each with
-// the A operand in tensor memory, 48 from shared memory), against ~14000 cycles of fp32 FMAs as measured.
+// A 128x64 product over 64 elements is 24 MMAs of 128x64x16 (32 cycles each with the A operand in tensor memory, 48
+// from shared memory), against ~14000 cycles of fp32 FMAs as measured.  No unit is the bound: the tensor pipe is busy 39 %
+// (forward), 57 % (dK/dV) and 52 % (dQ) of the active cycles at B4 H12 S1024 D64, issue slots 36-45 %.  One CTA fits an SM, and
+// what it waits for is its own chain of products, exponentials, splits and arrivals, two to three tiles deep.
 //
 // A product with an infinity cannot be split (inf * 0 is NaN): a CTA one of whose results is not finite computes its
 // rows again with fp32 FMAs before it leaves, so that infinities spread as through fp32 products (fma_rows below).
@@ -59,6 +63,8 @@ __device__ __forceinline__ int plane_of(uint32_t planes, int t) { return (planes
 // 6.9e-8 of them at D = 64 (four steps of full size) and 1.15e-7 at D = 128 (eight), measured as the slope of the
 // error of lse over the mean score.  The resident operand of the scores is raised by as much, in its smallest plane
 // (one ulp of it is too coarse); without that lse is 10 to 100 % further from float64 than the fp32 FMA kernels leave it.
+// It fits scores whose 16-term steps look alike.  Where one channel outweighs the others or all terms are large, lse is 1.1 to
+// 3.0 times as far from float64 as the FMA kernels leave it, still within an ulp (9e-8 of its value); out is nearer even so.
 template <int kD>
 constexpr float kLift = kD == 64 ? 6.9e-8f : 1.15e-7f;
 
@@ -1425,9 +1431,10 @@ bool few_keys(const FwdParams& p) {
 
 // Relative errors (2-norm, the worst of out / dQ / dK / dV, these kernels against the fp32 FMA ones): B4 H12 S1024 D64
 // causal 3.5e-7 / 7.8e-7, B1 Hq4 Hkv2 S4096 D64 causal 3.8e-7 / 1.9e-6, Sq64 Sk16384 D64 5.8e-7 / 2.3e-6; out alone at
-// D = 128: S777 2.6e-7 / 5.6e-7, Sq130 Sk8192 2.7e-7 / 1.7e-6.
-// Times (us, B200): B4 H12 S1024 D64 causal forward 163 -> 56.5, backward 563 -> 153; B2 Hq16 Hkv4 S1024 D128 forward
-// 488 -> 118; B2 H4 S256 D64 causal 12.8 -> 12.5 and 41 -> 21.8.
+// D = 128: S777 2.6e-7 / 5.6e-7, Sq130 Sk8192 2.7e-7 / 1.7e-6.  Over normal values of spread 0.5 to 1 and 128 to 4096 keys,
+// in terms of the FMA kernels' error: out 0.18-0.55, dQ 0.41-0.86, dK 0.30-0.81, dV 0.27-0.71, lse 0.96-1.07 (1.00 on average).
+// Times (us, B200): B4 H12 S1024 D64 causal forward 163 -> 56, backward 563 -> 155; B2 Hq16 Hkv4 S1024 D128 unmasked forward
+// 488 -> 130; B2 H4 S256 D64 causal 12.8 -> 12.8 and 41 -> 22.4.
 cudaError_t launch_fwd_fp32(const FwdParams& p, cudaStream_t stream, int* launches) {
   if (few_keys(p)) return launch_fwd_simt(p, kF32, stream, launches);
   const bool drop = p.drop.threshold != 0;
@@ -1437,6 +1444,10 @@ cudaError_t launch_fwd_fp32(const FwdParams& p, cudaStream_t stream, int* launch
   return e;
 }
 
+// At any length.  B200, us, FMA kernels against these: one to 64 heads 14-16 / 10-13 at 16 to 64 rows and keys, 73 / 34 at Sq96
+// Sk1024; 256 heads 97 / 55 at 128 rows and keys; 1024 heads 137 / 135 at 64.  The FMA kernels are faster only for up to 32 rows
+// and keys of 75 to 443 heads (296 heads: 22 / 33), where a second wave of 128-row blocks costs more than the blocks do;
+// a rule on heads would give a piece of a batch other bits than the whole, and the call's host side takes 200 us.
 cudaError_t launch_bwd_fp32(const BwdParams& p, cudaStream_t stream, int* launches) {
   const cudaError_t e = p.drop.threshold != 0 ? launch_bwd<64, true>(p, stream) : launch_bwd<64, false>(p, stream);
   if (e == cudaSuccess && launches) *launches += 3;
