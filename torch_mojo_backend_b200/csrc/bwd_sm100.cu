@@ -470,6 +470,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 teardown:
   tc_fence_before();
   __syncthreads();
+  settle_if_aborted(abort_flag);
   if (warp == 16) {
     __syncwarp();
     tc_fence_after();
@@ -814,6 +815,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ 
 teardown:
   tc_fence_before();
   __syncthreads();
+  settle_if_aborted(abort_flag);
   if (warp == 8) {
     __syncwarp();
     tc_fence_after();

@@ -653,6 +653,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_fp32_kernel(const __grid_cons
 teardown:
   tc_fence_before();
   __syncthreads();
+  settle_if_aborted(abort_flag);
   if (warp == kMmaWarp) {
     __syncwarp();
     tc_fence_after();
@@ -942,6 +943,7 @@ __device__ __forceinline__ void dq_block(const BwdParams& p, int block, uint8_t*
 teardown:
   tc_fence_before();
   __syncthreads();
+  settle_if_aborted(abort_flag);
   if (warp == kMmaWarp) {
     __syncwarp();
     tc_fence_after();
@@ -1298,6 +1300,7 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
 teardown:
   tc_fence_before();
   __syncthreads();
+  settle_if_aborted(abort_flag);
   if (warp == kMmaWarp) {
     __syncwarp();
     tc_fence_after();

@@ -681,6 +681,7 @@ teardown:
   if (!kSplit && warp == Cfg::kEpiWarp0 && lane == 0) tma_store_wait_read();
   tc_fence_before();
   __syncthreads();
+  if (!kSplit || !*skip_flag) settle_if_aborted(abort_flag);   // (a skipped block has issued nothing)
   if (warp == Cfg::kMmaWarp0) {
     __syncwarp();
     tc_fence_after();

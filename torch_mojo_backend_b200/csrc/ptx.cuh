@@ -107,6 +107,17 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 // This thread's warp, in a form the compiler knows to be the same for the whole warp.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
 
+// In a block's teardown, when nothing new is issued: where a wait has run out, copies and MMAs of the block may still be on
+// their way to or from the shared memory it is about to give back.  They take microseconds; it stays for a tenth of a
+// millisecond more.
+__device__ __forceinline__ void settle_if_aborted(const volatile uint32_t* abort_flag) {
+  if (*abort_flag) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 200000) {
+    }
+  }
+}
+
 // True when an earlier CTA of this launch (or an earlier launch sharing the status word) has
 // already reported a failed wait: later CTAs then leave at once instead of each spending its
 // own budget on a protocol that is known to be broken.
