@@ -293,7 +293,7 @@ def test_fp32_rows_past_the_end_do_not_count_as_not_finite():
 
 @pytest.mark.parametrize("B,Hq,Hkv,S,D,mode", [(4, 12, 12, 1024, 64, 1), (2, 16, 4, 1024, 128, 0)])
 def test_fp32_values_that_are_not_finite_cost_a_few_times_the_fma_kernels(B, Hq, Hkv, S, D, mode):
-    """Measured 1.8 to 2.6 times; one row at a time it was 20 to 65 times."""
+    """Measured 2.1 to 2.6 times; one row at a time it was 20 to 65 times."""
     g = torch.Generator().manual_seed(2)
     q, k, v, dout = (torch.randn(B, h, S, D, generator=g).cuda() for h in (Hq, Hkv, Hkv, Hq))
     v[:, :, 0, 0] = float("nan")

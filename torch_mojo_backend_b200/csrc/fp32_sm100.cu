@@ -224,8 +224,10 @@ __device__ __forceinline__ void issue_dim(uint32_t d, uint32_t a, uint32_t b_lo,
 // which deal the 16-byte pieces of the head dimension among them; a lane has pieces of two rows 64 apart, so that what it
 // reads from shared memory, which bounds this, serves both.  The other sequence comes in tiles of 64 rows, in two
 // buffers where the ring was.  B200, us, a NaN in V of every head, FMA kernels / these (with the tensor-core pass ahead
-// of them) / a warp a row without staging: B4 H12 S1024 D64 causal forward 187 / 488 / 6349, backward 605 / 1076 / 12260;
+// of them) / a warp a row without staging: B4 H12 S1024 D64 causal forward 187 / 488 / 6349, backward 605 / 1338 / 12260;
 // B2 Hq16 Hkv4 S1024 D128 forward 512 / 1083 / 10377; B1 H4 S4096 D64 causal (128 CTAs against 512) 264 / 1158 / 17704.
+// The backward's are functions that are called, with nothing handed over but the block: inlined, two rows a lane in dK/dV
+// too, they cost calls of finite values 2-3 % (B4 H12 S1024 155.5 against 154; the forward's costs nothing inlined).
 constexpr int kLaneRows = 2;
 // all math warps, with a bounded wait
 struct RowSync {
@@ -241,6 +243,12 @@ struct RowSync {
     return ok;
   }
 };
+// (its barrier is the last one of every kernel here)
+template <class Cfg>
+__device__ __forceinline__ RowSync row_sync(uint8_t* smem, uint32_t* status, long long budget) {
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBars);
+  return RowSync{bars + Cfg::kNumBars - 1, reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars) + 1, status, budget};
+}
 // rows s0 + [0, 64) of a tensor to [row][kD]; zeros past the end
 template <int kD>
 __device__ __forceinline__ void stage_rows(float* dst, const View4& t, int b, int h, int s0, int rows) {
@@ -269,22 +277,22 @@ __device__ __forceinline__ void store_part(float* row, int part, const float2 (&
         make_float4(x[2 * i].x * mul, x[2 * i].y * mul, x[2 * i + 1].x * mul, x[2 * i + 1].y * mul);
 }
 // the products of a lane's rows with a streamed one, whole in all four lanes
-template <int kD>
-__device__ __forceinline__ void dot_parts(float (&s)[kLaneRows], const float2 (&x)[kLaneRows][kD / 8], const float* row, int part) {
-  float2 a[kLaneRows], b[kLaneRows];
+template <int kD, int kN>
+__device__ __forceinline__ void dot_parts(float (&s)[kN], const float2 (&x)[kN][kD / 8], const float* row, int part) {
+  float2 a[kN], b[kN];
 #pragma unroll
-  for (int j = 0; j < kLaneRows; ++j) a[j] = b[j] = make_float2(0.f, 0.f);
+  for (int j = 0; j < kN; ++j) a[j] = b[j] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < kD / 16; ++i) {
     const float4 v = reinterpret_cast<const float4*>(row)[4 * i + part];
 #pragma unroll
-    for (int j = 0; j < kLaneRows; ++j) {
+    for (int j = 0; j < kN; ++j) {
       a[j] = __ffma2_rn(x[j][2 * i], make_float2(v.x, v.y), a[j]);
       b[j] = __ffma2_rn(x[j][2 * i + 1], make_float2(v.z, v.w), b[j]);
     }
   }
 #pragma unroll
-  for (int j = 0; j < kLaneRows; ++j) {
+  for (int j = 0; j < kN; ++j) {
     s[j] = (a[j].x + a[j].y) + (b[j].x + b[j].y);
     s[j] += __shfl_xor_sync(0xffffffffu, s[j], 1);
     s[j] += __shfl_xor_sync(0xffffffffu, s[j], 2);
@@ -292,14 +300,14 @@ __device__ __forceinline__ void dot_parts(float (&s)[kLaneRows], const float2 (&
 }
 // acc[j] += w[j] * the streamed row, for the rows that see it (`all`: every one).  A row that does not is left out: zero
 // times what is not finite is not zero.
-template <int kD>
-__device__ __forceinline__ void add_parts(float2 (&acc)[kLaneRows][kD / 8], const float (&w)[kLaneRows], bool all, const bool (&sees)[kLaneRows],
+template <int kD, int kN>
+__device__ __forceinline__ void add_parts(float2 (&acc)[kN][kD / 8], const float (&w)[kN], bool all, const bool (&sees)[kN],
                                           const float* row, int part) {
 #pragma unroll
   for (int i = 0; i < kD / 16; ++i) {
     const float4 v = reinterpret_cast<const float4*>(row)[4 * i + part];
 #pragma unroll
-    for (int j = 0; j < kLaneRows; ++j) {
+    for (int j = 0; j < kN; ++j) {
       const float2 w2 = make_float2(w[j], w[j]);
       const float2 lo = __ffma2_rn(w2, make_float2(v.x, v.y), acc[j][2 * i]), hi = __ffma2_rn(w2, make_float2(v.z, v.w), acc[j][2 * i + 1]);
       if (all || sees[j]) {
@@ -676,10 +684,15 @@ struct DqF32Cfg {
 };
 
 template <int kD, bool kDropout>
-__device__ __forceinline__ bool fma_rows_dq(const BwdParams& p, int b, int h, int hk, int m0, int warp, int lane, uint8_t* smem, RowSync sync) {
+__device__ __noinline__ bool fma_rows_dq(const BwdParams& p, int block, uint8_t* smem) {
+  RowSync sync = row_sync<DqF32Cfg<kD>>(smem, p.status, p.wait_budget);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int tile, bh;
+  tile_and_head(block, (p.S + kBM - 1) / kBM, p.B * p.Hq, p.causal, &tile, &bh);
+  const int m0 = tile * kBM, b = bh / p.Hq, h = bh - b * p.Hq, hk = h / (p.Hq / p.Hkv);
   constexpr int kKeys = 2, kTile = kBN * kD;
   float* buf = reinterpret_cast<float*>(smem);   // [tile & 1][K, V][64][kD]
-  const int part = lane & 3, bh = b * p.Hq + h;
+  const int part = lane & 3;
   int q_row[kLaneRows], last[kLaneRows];
 #pragma unroll
   for (int j = 0; j < kLaneRows; ++j) {
@@ -878,7 +891,7 @@ __device__ __forceinline__ void dq_block(const BwdParams& p, int block, uint8_t*
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xd30);
     if (*not_finite) {
-      if (!fma_rows_dq<kD, kDropout>(p, b, h, hk, m0, warp, lane, smem, RowSync{rows_done, abort_flag, p.status, p.wait_budget})) goto teardown;
+      if (!fma_rows_dq<kD, kDropout>(p, block, smem)) goto teardown;
     } else if (q_row < p.S) {
       float4* dst = reinterpret_cast<float4*>(const_cast<float*>(row_ptr(p.dq, b, h, q_row)) + half * (kD / 2));
 #pragma unroll
@@ -971,79 +984,88 @@ struct DkdvF32Cfg {
 };
 
 template <int kD, bool kDropout>
-__device__ __forceinline__ bool fma_rows_dkdv(const BwdParams& p, int b, int hk, int n0, int warp, int lane, uint8_t* smem, RowSync sync) {
-  constexpr int kTile = kBN * kD;
+__device__ __noinline__ bool fma_rows_dkdv(const BwdParams& p, int block, uint8_t* smem) {
+  RowSync sync = row_sync<DkdvF32Cfg<kD>>(smem, p.status, p.wait_budget);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int tile, bhk;
+  tile_and_head(block, (p.Sk + kBM - 1) / kBM, p.B * p.Hkv, false, &tile, &bhk);
+  const int n0 = tile * kBM, b = bhk / p.Hkv, hk = bhk - b * p.Hkv;
+  constexpr int kN = 1, kTile = kBN * kD;   // (two rows a lane do not fit: 128 registers of operands and sums)
   float* buf = reinterpret_cast<float*>(smem);   // [tile & 1][Q, dO][64][kD]
   const int part = lane & 3, group = p.Hq / p.Hkv;
-  int key[kLaneRows], first[kLaneRows];   // first query row that sees the key
-#pragma unroll
-  for (int j = 0; j < kLaneRows; ++j) {
-    key[j] = min(n0 + j * 64 + warp * 8 + (lane >> 2), p.Sk - 1);
-    first[j] = p.causal ? max(0, key[j] - p.causal_off) : 0;
-  }
-  const int warp_first = __reduce_min_sync(0xffffffffu, first[0]), warp_last = __reduce_max_sync(0xffffffffu, first[1]);
-  const int m_begin = p.causal ? max(0, n0 - p.causal_off) / kBN * kBN : 0;
-  const int per_head = max(0, (p.S - m_begin + kBN - 1) / kBN), tiles = group * per_head;
-  auto stage = [&](int t) {
-    const int h = hk * group + t / per_head, q0 = m_begin + t % per_head * kBN;
-    stage_rows<kD>(buf + (t & 1) * 2 * kTile, p.q, b, h, q0, p.S);
-    stage_rows<kD>(buf + (t & 1) * 2 * kTile + kTile, p.dout, b, h, q0, p.S);
-    cp_commit();
-  };
-  float2 k[kLaneRows][kD / 8], v[kLaneRows][kD / 8], dk[kLaneRows][kD / 8], dv[kLaneRows][kD / 8];
-#pragma unroll
-  for (int j = 0; j < kLaneRows; ++j) {
-    load_part<kD>(k[j], row_ptr(p.k, b, hk, key[j]), part);
-    load_part<kD>(v[j], row_ptr(p.v, b, hk, key[j]), part);
-#pragma unroll
-    for (int i = 0; i < kD / 8; ++i) dk[j][i] = dv[j][i] = make_float2(0.f, 0.f);
-  }
-  if (tiles > 0) stage(0);
 #pragma unroll 1
-  for (int t = 0; t < tiles; ++t) {
-    cp_wait<0>();
-    if (!sync()) return false;
-    if (t + 1 < tiles) stage(t + 1);
-    const float* qt = buf + (t & 1) * 2 * kTile;
-    const int bh = b * p.Hq + hk * group + t / per_head, q0 = m_begin + t % per_head * kBN;
-#pragma unroll 1
-    for (int c0 = 0; c0 < kBN && q0 + c0 < p.S; c0 += 32) {
-      // lane L has the statistics of query row L of these 32, and its keep bits against the 16 keys that hold this warp's
-      const int mine = min(q0 + c0 + lane, p.S - 1);
-      const float lse = p.lse[static_cast<int64_t>(bh) * p.S + mine], my_dps = __ldcg(p.dpsum + static_cast<int64_t>(bh) * p.Spad + mine);
-      const float my_l2 = lse != -INFINITY ? lse * kLog2e : INFINITY;
-      uint32_t my_keep[kLaneRows];
-      if constexpr (kDropout) {
+  for (int row0 = n0; row0 < min(n0 + kBM, p.Sk); row0 += 64) {
+    int key[kN], first[kN];   // first query row that sees the key
 #pragma unroll
-        for (int j = 0; j < kLaneRows; ++j) my_keep[j] = dropout_bits16(p.drop, bh, mine, (n0 + j * 64 + warp * 8) >> 4);
-      }
-#pragma unroll 1
-      for (int u = max(0, warp_first - q0 - c0); u < min(32, p.S - q0 - c0); ++u) {
-        const float l2 = __shfl_sync(0xffffffffu, my_l2, u), dps = __shfl_sync(0xffffffffu, my_dps, u);
-        const float* qr = qt + (c0 + u) * kD;
-        float s[kLaneRows], dp[kLaneRows];
-        dot_parts<kD>(s, k, qr, part);
-        dot_parts<kD>(dp, v, qr + kTile, part);
+    for (int j = 0; j < kN; ++j) {
+      key[j] = min(row0 + j * 64 + warp * 8 + (lane >> 2), p.Sk - 1);
+      first[j] = p.causal ? max(0, key[j] - p.causal_off) : 0;
+    }
+    const int warp_first = __reduce_min_sync(0xffffffffu, first[0]), warp_last = __reduce_max_sync(0xffffffffu, first[kN - 1]);
+    const int m_begin = p.causal ? max(0, row0 - p.causal_off) / kBN * kBN : 0;
+    const int per_head = max(0, (p.S - m_begin + kBN - 1) / kBN), tiles = group * per_head;
+    auto stage = [&](int t) {
+      const int h = hk * group + t / per_head, q0 = m_begin + t % per_head * kBN;
+      stage_rows<kD>(buf + (t & 1) * 2 * kTile, p.q, b, h, q0, p.S);
+      stage_rows<kD>(buf + (t & 1) * 2 * kTile + kTile, p.dout, b, h, q0, p.S);
+      cp_commit();
+    };
+    float2 k[kN][kD / 8], v[kN][kD / 8], dk[kN][kD / 8], dv[kN][kD / 8];
 #pragma unroll
-        for (int j = 0; j < kLaneRows; ++j) {
-          const float pv = exp2f(s[j] * p.scale_log2 - l2);
-          float dm = 1.f;
-          if constexpr (kDropout) dm = (__shfl_sync(0xffffffffu, my_keep[j], u) >> (key[j] & 15)) & 1u ? p.drop.inv_keep : 0.f;
-          s[j] = pv * dm;
-          dp[j] = pv * (dp[j] * dm - dps);
+    for (int j = 0; j < kN; ++j) {
+      load_part<kD>(k[j], row_ptr(p.k, b, hk, key[j]), part);
+      load_part<kD>(v[j], row_ptr(p.v, b, hk, key[j]), part);
+#pragma unroll
+      for (int i = 0; i < kD / 8; ++i) dk[j][i] = dv[j][i] = make_float2(0.f, 0.f);
+    }
+    if (tiles > 0) stage(0);
+#pragma unroll 1
+    for (int t = 0; t < tiles; ++t) {
+      cp_wait<0>();
+      if (!sync()) return false;
+      if (t + 1 < tiles) stage(t + 1);
+      const float* qt = buf + (t & 1) * 2 * kTile;
+      const int bh = b * p.Hq + hk * group + t / per_head, q0 = m_begin + t % per_head * kBN;
+#pragma unroll 1
+      for (int c0 = 0; c0 < kBN && q0 + c0 < p.S; c0 += 32) {
+        // lane L has the statistics of query row L of these 32, and its keep bits against the 16 keys that hold this warp's
+        const int mine = min(q0 + c0 + lane, p.S - 1);
+        const float lse = p.lse[static_cast<int64_t>(bh) * p.S + mine], my_dps = __ldcg(p.dpsum + static_cast<int64_t>(bh) * p.Spad + mine);
+        const float my_l2 = lse != -INFINITY ? lse * kLog2e : INFINITY;
+        uint32_t my_keep[kN];
+        if constexpr (kDropout) {
+#pragma unroll
+          for (int j = 0; j < kN; ++j) my_keep[j] = dropout_bits16(p.drop, bh, mine, (row0 + j * 64 + warp * 8) >> 4);
         }
-        const int q_row = q0 + c0 + u;
-        const bool sees[kLaneRows] = {q_row >= first[0], q_row >= first[1]};
-        add_parts<kD>(dv, s, q_row >= warp_last, sees, qr + kTile, part);
-        add_parts<kD>(dk, dp, q_row >= warp_last, sees, qr, part);
+#pragma unroll 1
+        for (int u = max(0, warp_first - q0 - c0); u < min(32, p.S - q0 - c0); ++u) {
+          const float l2 = __shfl_sync(0xffffffffu, my_l2, u), dps = __shfl_sync(0xffffffffu, my_dps, u);
+          const float* qr = qt + (c0 + u) * kD;
+          float s[kN], dp[kN];
+          dot_parts<kD>(s, k, qr, part);
+          dot_parts<kD>(dp, v, qr + kTile, part);
+#pragma unroll
+          for (int j = 0; j < kN; ++j) {
+            const float pv = exp2f(s[j] * p.scale_log2 - l2);
+            float dm = 1.f;
+            if constexpr (kDropout) dm = (__shfl_sync(0xffffffffu, my_keep[j], u) >> (key[j] & 15)) & 1u ? p.drop.inv_keep : 0.f;
+            s[j] = pv * dm;
+            dp[j] = pv * (dp[j] * dm - dps);
+          }
+          const int q_row = q0 + c0 + u;
+          const bool sees[kN] = {q_row >= first[0]};
+          add_parts<kD>(dv, s, q_row >= warp_last, sees, qr + kTile, part);
+          add_parts<kD>(dk, dp, q_row >= warp_last, sees, qr, part);
+        }
       }
     }
-  }
 #pragma unroll
-  for (int j = 0; j < kLaneRows; ++j) {
-    if (n0 + j * 64 + warp * 8 + (lane >> 2) >= p.Sk) continue;
-    store_part<kD>(const_cast<float*>(row_ptr(p.dk, b, hk, key[j])), part, dk[j], p.scale);
-    store_part<kD>(const_cast<float*>(row_ptr(p.dv, b, hk, key[j])), part, dv[j], 1.f);
+    for (int j = 0; j < kN; ++j) {
+      if (row0 + j * 64 + warp * 8 + (lane >> 2) >= p.Sk) continue;
+      store_part<kD>(const_cast<float*>(row_ptr(p.dk, b, hk, key[j])), part, dk[j], p.scale);
+      store_part<kD>(const_cast<float*>(row_ptr(p.dv, b, hk, key[j])), part, dv[j], 1.f);
+    }
+    if (!sync()) return false;   // the next pass writes the buffers
   }
   return true;
 }
@@ -1206,7 +1228,7 @@ __device__ __forceinline__ void dkdv_block(const BwdParams& p, int block, uint8_
     mbar_arrive_warp(done);
     B200FA_WAIT(done, 0, 0xe30);
     if (*not_finite) {
-      if (!fma_rows_dkdv<kD, kDropout>(p, b, hk, n0, warp, lane, smem, RowSync{rows_done, abort_flag, p.status, p.wait_budget})) goto teardown;
+      if (!fma_rows_dkdv<kD, kDropout>(p, block, smem)) goto teardown;
     } else if (n0 + r < p.Sk) {
       float4* dst_k = reinterpret_cast<float4*>(const_cast<float*>(row_ptr(p.dk, b, hk, n0 + r)) + half * (kD / 2));
       float4* dst_v = reinterpret_cast<float4*>(const_cast<float*>(row_ptr(p.dv, b, hk, n0 + r)) + half * (kD / 2));
