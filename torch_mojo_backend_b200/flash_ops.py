@@ -207,11 +207,7 @@ def piece_of(whole_heads: int, backward: bool = False):
         _piece.heads, _piece.backward = before
 
 
-def _fma_backward_follows(q: TorchMojoTensor, *arguments) -> bool:
-    """The results go into the fp32 backward of FMA arithmetic (head dimension 128).  `q`: the payload of the first of
-    the call's `arguments`."""
-    if q._dtype is not torch.float32 or q._shape[3] != 128:
-        return False
+def _backward_follows(*arguments) -> bool:
     return getattr(_piece, "backward", False) or (torch.is_grad_enabled() and any(t.requires_grad for t in arguments))
 
 
@@ -297,8 +293,9 @@ def scaled_dot_product_flash_attention(query, key, value, dropout_p=0.0, is_caus
         )
     q, k, v = inputs
     index = q._device_index
-    out, lse, (seed, offset) = forward_with_its_own_mask(q, k, v, dropout_p, is_causal, scale,
-                                                         _fma_backward_follows(q, query, key, value))
+    # (asked of the calls alone that it makes a difference to)
+    fma_backward = q._shape[3] == 128 and q._dtype is torch.float32 and _backward_follows(query, key, value)
+    out, lse, (seed, offset) = forward_with_its_own_mask(q, k, v, dropout_p, is_causal, scale, fma_backward)
     rng_state = TorchMojoTensor._alloc((2,), torch.uint64, index)
     if float(dropout_p):
         # the pair as two signed 64-bit patterns (uint64 fills are not universally supported), by two fills: a copy from
