@@ -1,7 +1,7 @@
 // Exact-fp32 SIMT attention kernels (forward and backward).
 //
-// These serve fp32 tensors where fp32_sm100.cu does not: the backward at head dimension 128, and forwards over few
-// keys.  All products and sums are fp32 FMAs; the softmax
+// These serve fp32 tensors where fp32_sm100.cu does not, at head dimension 128: the backward, the forward ahead of it, and
+// forwards over few keys.  All products and sums are fp32 FMAs; the softmax
 // uses exp2f on scale*log2(e)-scaled scores, the same formulation as the tensor-core path
 // (reference math: torch_mojo_backend/eager_flash_attention/fa4_fwd_kernel.mojo:650-861 and
 // fa4_bwd_kernel.mojo:1-44, 810-980).  They are templated on the storage type so the same
